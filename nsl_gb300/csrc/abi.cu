@@ -171,10 +171,10 @@ int apply_one(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *in, doubl
     if (fm->kind == NSLG_FM_DIAG) {  // e = sgn delta K (M) or sgn delta* K (M^dagger): CUDA-core kernel
         const int dmode = mode == MODE_M ? MODE_DIAG_M : MODE_DIAG_MDAG;
         if constexpr (std::is_same_v<T, double>)
-            return fm_apply_simt<double>(dmode, in, out, fm->phase, e->re, e->is_real ? nullptr : e->im, Nt, Nx,
+            return fm_apply_simt<double>(dmode, in, out, fm->phase, e->reT, e->imT, Nt, Nx,
                                          rows, st);
         else if constexpr (std::is_same_v<T, float>)
-            return fm_apply_simt<float>(dmode, in, out, fm->phase32, e->re32, e->is_real ? nullptr : e->im32, Nt, Nx,
+            return fm_apply_simt<float>(dmode, in, out, fm->phase32, e->re32T, e->im32T, Nt, Nx,
                                         rows, st);
         else
             NSLG_REQUIRE(false, NSLG_ERR_UNSUPPORTED,
@@ -190,19 +190,19 @@ int apply_one(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *in, doubl
             NSLG_TRY(ws_get(fm, "oz_digits", (size_t)oz_digits() * 2 * rows * oz_ld(Nx) * 2, &dg));
             return fm_apply_oz(mode, in, out, fm->phase, *P, dg, rexp, Nt, Nx, rows, fm->tc_err, st);
         }
-        return fm_apply_simt<double>(mode, in, out, fm->phase, e->re, e->is_real ? nullptr : e->im, Nt, Nx, rows, st);
+        return fm_apply_simt<double>(mode, in, out, fm->phase, e->reT, e->imT, Nt, Nx, rows, st);
     } else if constexpr (std::is_same_v<T, TF32x3>) {
         if (e->is_real) {
             TcPlanes *P;
             NSLG_TRY(tc_planes(fm, e, &P));
             return fm_apply_tc(mode, in, out, fm->phase, *P, Nt, Nx, rows, fm->tc_err, st);
         }
-        return fm_apply_simt<float>(mode, in, out, fm->phase32, e->re32, e->im32, Nt, Nx, rows, st);
+        return fm_apply_simt<float>(mode, in, out, fm->phase32, e->re32T, e->im32T, Nt, Nx, rows, st);
     } else if constexpr (std::is_same_v<T, float>) {
-        return fm_apply_simt<float>(mode, in, out, fm->phase32, e->re32, e->is_real ? nullptr : e->im32, Nt, Nx,
+        return fm_apply_simt<float>(mode, in, out, fm->phase32, e->re32T, e->im32T, Nt, Nx,
                                     rows, st);
     } else {
-        return fm_apply_simt<double>(mode, in, out, fm->phase, e->re, e->is_real ? nullptr : e->im, Nt, Nx, rows,
+        return fm_apply_simt<double>(mode, in, out, fm->phase, e->reT, e->imT, Nt, Nx, rows,
                                      st, mask, sys_rows);
     }
 }
@@ -370,17 +370,11 @@ NSLG_API int nslg_fm_destroy(nslg_fm *fm) {
     drop_graphs(fm);
     for (auto &kv : fm->lin) {
         cudaFree(kv.second.full);
-        cudaFree(kv.second.re);
-        cudaFree(kv.second.im);
-        cudaFree(kv.second.re32);
-        cudaFree(kv.second.im32);
+        free_planes(kv.second);
     }
     for (auto &kv : fm->memo) {
         cudaFree(kv.second.full);
-        cudaFree(kv.second.re);
-        cudaFree(kv.second.im);
-        cudaFree(kv.second.re32);
-        cudaFree(kv.second.im32);
+        free_planes(kv.second);
         if (kv.second.tc) {
             cudaFree(kv.second.tc->hi);
             cudaFree(kv.second.tc->lo);

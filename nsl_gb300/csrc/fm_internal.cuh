@@ -43,8 +43,10 @@ struct ExpEntry {
     double2 *full = nullptr;  // complex (Nx, Nx) row-major
     double *re = nullptr;     // real plane, FP64
     double *im = nullptr;     // imaginary plane, FP64 (null when exp(d K) is exactly real)
-    float *re32 = nullptr;    // FP32 copies for the mixed-precision inner operator
-    float *im32 = nullptr;
+    // transposed planes (reT[y Nx + x] = E[x, y]) of the CUDA-core operators, FP64 and FP32; the imaginary ones are null
+    // when exp(d K) is exactly real
+    double *reT = nullptr, *imT = nullptr;
+    float *re32T = nullptr, *im32T = nullptr;
     bool is_real = true;
     TcPlanes *tc = nullptr;   // built on first tensor-core use
     OzPlanes *oz = nullptr;   // built on first split-BF16 use
@@ -140,9 +142,11 @@ int get_lin(nslg_fm *fm, double2 d, int one_minus, const ExpEntry **out);
 // The matrix of one operator factor for the handle's discretisation: exp(d K) or d K.
 int get_factor(nslg_fm *fm, double2 d, const ExpEntry **out);
 int install_exp(nslg_fm *fm, double2 d, const double2 *E_dev);
+void free_planes(ExpEntry &e);  // every plane of an entry but `full`
 
 // ----- kernels (launchers) ---------------------------------------------------------------------------------------
-// Fused M / Mdag application on FP64 vectors with the product in T (double: FP64 drop-in; float: FP32 operator).
+// Fused M / Mdag application on FP64 vectors with the product in T (double: FP64 drop-in; float: FP32 operator);
+// Ere, Eim: the transposed planes (ExpEntry::reT ...).
 // With sys_mask only tiles holding rows of systems s (sys_rows consecutive rows each) with sys_mask[s] != 0 compute.
 template <typename T>
 int fm_apply_simt(int mode, const double2 *psi, double2 *out, const cplx_t<T> *phase, const T *Ere, const T *Eim,

@@ -188,17 +188,27 @@ __global__ void k_scale(double2 *out, const double2 *in, double2 s, int64_t n) {
     if (i < n) out[i] = cmul(s, in[i]);
 }
 
-// Planes of exp(d K): re/im FP64 and FP32, plus a flag set when any imaginary part is nonzero.
-__global__ void k_split_planes(const double2 *E, double *re, double *im, float *re32, float *im32, int64_t n,
+// Planes of exp(d K): re/im FP64 row-major, re transposed in FP64 and FP32, plus a flag set when any imaginary part is
+// nonzero.
+__global__ void k_split_planes(const double2 *E, double *re, double *im, double *reT, float *re32T, int n,
                                int *nonreal) {
     const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+    if (i >= (int64_t)n * n) return;
     const double2 v = E[i];
+    const int64_t j = (i % n) * n + i / n;
     re[i] = v.x;
     im[i] = v.y;
-    re32[i] = (float)v.x;
-    im32[i] = (float)v.y;
+    reT[j] = v.x;
+    re32T[j] = (float)v.x;
     if (v.y != 0.0) atomicOr(nonreal, 1);
+}
+// the transposed imaginary planes of a complex entry
+__global__ void k_split_imag(const double2 *E, double *imT, float *im32T, int n) {
+    const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (int64_t)n * n) return;
+    const int64_t j = (i % n) * n + i / n;
+    imT[j] = E[i].y;
+    im32T[j] = (float)E[i].y;
 }
 
 // 1-norm (max column sum of |K|) of a complex (n, n) matrix, one block.
@@ -376,24 +386,42 @@ int compute_phases(nslg_fm *fm) {
     return NSLG_OK;
 }
 
+void free_planes(ExpEntry &e) {
+    cudaFree(e.re);
+    cudaFree(e.im);
+    cudaFree(e.reT);
+    cudaFree(e.imT);
+    cudaFree(e.re32T);
+    cudaFree(e.im32T);
+    e.re = e.im = e.reT = e.imT = nullptr;
+    e.re32T = e.im32T = nullptr;
+}
+
 static int make_entry(nslg_fm *fm, double2 *full, nslg::ExpEntry *e) {
     const int64_t n = fm->Nx * fm->Nx;
     cudaStream_t st = fm->ctx->stream;
     e->full = full;
     NSLG_CUDA(cudaMalloc(&e->re, n * sizeof(double)));
     NSLG_CUDA(cudaMalloc(&e->im, n * sizeof(double)));
-    NSLG_CUDA(cudaMalloc(&e->re32, n * sizeof(float)));
-    NSLG_CUDA(cudaMalloc(&e->im32, n * sizeof(float)));
+    NSLG_CUDA(cudaMalloc(&e->reT, n * sizeof(double)));
+    NSLG_CUDA(cudaMalloc(&e->re32T, n * sizeof(float)));
     int *flag;
     NSLG_TRY(ws_get(fm, "exp_flag", 1, &flag));
     NSLG_CUDA(cudaMemsetAsync(flag, 0, sizeof(int), st));
-    k_split_planes<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(full, e->re, e->im, e->re32, e->im32, n, flag);
+    k_split_planes<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(full, e->re, e->im, e->reT, e->re32T, (int)fm->Nx, flag);
     note_launch(st);
     NSLG_CUDA(cudaGetLastError());
     int h = 0;
     NSLG_CUDA(cudaMemcpyAsync(&h, flag, sizeof(int), cudaMemcpyDeviceToHost, st));
     NSLG_CUDA(cudaStreamSynchronize(st));
     e->is_real = (h == 0);
+    if (!e->is_real) {
+        NSLG_CUDA(cudaMalloc(&e->imT, n * sizeof(double)));
+        NSLG_CUDA(cudaMalloc(&e->im32T, n * sizeof(float)));
+        k_split_imag<<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(full, e->imT, e->im32T, (int)fm->Nx);
+        note_launch(st);
+        NSLG_CUDA(cudaGetLastError());
+    }
     return NSLG_OK;
 }
 
@@ -404,10 +432,7 @@ int install_exp(nslg_fm *fm, double2 d, const double2 *E_dev) {
     if (it != fm->memo.end()) {
         NSLG_CUDA(cudaMemcpyAsync(it->second.full, E_dev, n * sizeof(double2), cudaMemcpyDeviceToDevice,
                                   fm->ctx->stream));
-        cudaFree(it->second.re);
-        cudaFree(it->second.im);
-        cudaFree(it->second.re32);
-        cudaFree(it->second.im32);
+        free_planes(it->second);
         return make_entry(fm, it->second.full, &it->second);
     }
     double2 *full;

@@ -63,10 +63,10 @@ int apply_factor(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *in, do
     const int Nt = (int)fm->Nt, Nx = (int)fm->Nx;
     if (fm->kind == NSLG_FM_DIAG) mode = mode == MODE_M ? MODE_DIAG_M : MODE_DIAG_MDAG;
     if constexpr (sizeof(T) == 8)
-        return fm_apply_simt<double>(mode, in, out, fm->phase, e->re, e->is_real ? nullptr : e->im, Nt, Nx, rows,
+        return fm_apply_simt<double>(mode, in, out, fm->phase, e->reT, e->imT, Nt, Nx, rows,
                                      fm->ctx->stream);
     else
-        return fm_apply_simt<float>(mode, in, out, fm->phase32, e->re32, e->is_real ? nullptr : e->im32, Nt, Nx,
+        return fm_apply_simt<float>(mode, in, out, fm->phase32, e->re32T, e->im32T, Nt, Nx,
                                     rows, fm->ctx->stream);
 }
 

@@ -188,3 +188,31 @@ def test_split_bf16_digit_bound_refuses_delocalised_exp():
     with pytest.raises(RuntimeError, match="delocalised"):
         hfm.M(psi, precision="bf16split")
     hfm.M(psi, precision="fp64")
+
+
+@pytest.mark.parametrize("Nx", [1, 2, 31, 33, 64, 65, 127, 255, 256, 257, 320])
+@pytest.mark.parametrize("Nt,R", [(1, 1), (3, 2), (7, 5), (64, 6)])
+def test_cuda_core_operator_splits(Nx, Nt, R):
+    """The CUDA-core operators at the edges of their work split (whole rows up to 256 sites, runs of sites beyond; 1 to 8
+    rows per thread), with a real and a complex, non-symmetric exp(delta K), against the same formula in numpy. A sum of
+    Nx complex products in any order, its factors rounded once, is within 4 (Nx + 8) eps of the sum of their moduli."""
+    import nsl_gb300 as N
+
+    rng = np.random.default_rng(100 * Nx + Nt)
+    phi = rng.standard_normal((Nt, Nx)) + 0.3j * rng.standard_normal((Nt, Nx))
+    psi = rng.standard_normal((R, Nt, Nx)) + 1j * rng.standard_normal((R, Nt, Nx))
+    ph = np.exp(1j * phi)
+    sign = np.where(np.arange(Nt) == 0, -1.0, 1.0)[:, None]
+    for E in (rng.standard_normal((Nx, Nx)) + 0j, rng.standard_normal((Nx, Nx)) + 1j * rng.standard_normal((Nx, Nx))):
+        lat = N.Ring(Nx)
+        lat.set_exp_hopping_matrix(0.125, E)
+        fm = N.HubbardExp(lat, Nt, 0.125 * Nt)
+        fm.populate(phi)
+        wantM = psi - sign * np.roll((ph * psi) @ E.T, 1, 1)
+        sizeM = np.abs(psi) + np.roll(np.abs(ph * psi) @ np.abs(E).T, 1, 1)
+        wantD = psi - np.conj(ph) * np.roll(sign * (psi @ E.T), -1, 1)
+        sizeD = np.abs(psi) + np.abs(ph) * np.roll(np.abs(psi) @ np.abs(E).T, -1, 1)
+        for prec, eps in (("fp64", 2.0 ** -53), ("fp32", 2.0 ** -24)):
+            for op, want, size in (("M", wantM, sizeM), ("Mdagger", wantD, sizeD)):
+                err = np.abs(getattr(fm, op)(psi, precision=prec) - want)
+                assert np.all(err <= 4 * (Nx + 8) * eps * size), (prec, op, (err / size).max())
