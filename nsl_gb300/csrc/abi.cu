@@ -151,7 +151,7 @@ int prepare_apply(nslg_fm *fm, int op, int64_t nbatch, int precision) {
         void *dg;
         const int64_t rows = nbatch * fm->Nt;
         NSLG_TRY(ws_get(fm, "oz_rexp", (size_t)2 * rows, &rexp));
-        NSLG_TRY(ws_get(fm, "oz_digits", (size_t)oz_digits() * 2 * rows * oz_ld((int)fm->Nx) * 2, &dg));
+        NSLG_TRY(ws_get(fm, "oz_digits", oz_digit_bytes(rows, (int)fm->Nx), &dg));
     }
     if (op == NSLG_OP_MMDAGGER || op == NSLG_OP_MDAGGERM) {
         void *w;
@@ -187,7 +187,7 @@ int apply_one(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *in, doubl
             int *rexp;
             void *dg;
             NSLG_TRY(ws_get(fm, "oz_rexp", (size_t)2 * rows, &rexp));
-            NSLG_TRY(ws_get(fm, "oz_digits", (size_t)oz_digits() * 2 * rows * oz_ld(Nx) * 2, &dg));
+            NSLG_TRY(ws_get(fm, "oz_digits", oz_digit_bytes(rows, Nx), &dg));
             return fm_apply_oz(mode, in, out, fm->phase, *P, dg, rexp, Nt, Nx, rows, fm->tc_err, st);
         }
         return fm_apply_simt<double>(mode, in, out, fm->phase, e->reT, e->imT, Nt, Nx, rows, st);
@@ -383,6 +383,7 @@ NSLG_API int nslg_fm_destroy(nslg_fm *fm) {
         if (kv.second.oz) {
             cudaFree(kv.second.oz->planes);
             cudaFree(kv.second.oz->col_exp);
+            cudaFree(kv.second.oz->klist);
             delete kv.second.oz;
         }
     }

@@ -300,8 +300,8 @@ __global__ void __launch_bounds__(RT) k_cg_p_oz(const double2 *__restrict__ r, d
                                                 int rows_per_sys, const double *__restrict__ p_rr, int npart,
                                                 const CgState *__restrict__ st_in, CgState *__restrict__ st_out,
                                                 int64_t max_iter, int reliable, double update_frac,
-                                                int *__restrict__ go, __nv_bfloat16 *__restrict__ planes, int *__restrict__ rexp, int ld,
-                                                int64_t rows) {
+                                                int *__restrict__ go, __nv_bfloat16 *__restrict__ planes, int *__restrict__ rexp,
+                                                int ld) {
     constexpr int WPB = RT / 32;
     const int s = blockIdx.y, lane = threadIdx.x % 32, w = threadIdx.x / 32;
     const CgState S = st_in[s];
@@ -378,11 +378,11 @@ __global__ void __launch_bounds__(RT) k_cg_p_oz(const double2 *__restrict__ r, d
         rexp[2 * grow] = er;
         rexp[2 * grow + 1] = ei;
     }
-    const int64_t mreal = 2 * rows;
+    const int nkb = ld / OZ_KB;
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         const int y = 2 * (lane + 32 * k);
-        if (y < ld) write_digits2(planes, mreal, grow, ld, y, c[k], er, ei);
+        if (y < ld) write_digits2(planes, grow, nkb, y, c[k], er, ei);
     }
     for (int y = 2 * (lane + 32 * NP); y < ld; y += 64) {
         unsigned long long b[4] = {0ull, 0ull, 0ull, 0ull};
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__(RT) k_cg_p_oz(const double2 *__restrict__ r, d
                 b[2 * h] = (unsigned long long)__double_as_longlong(pv.x);
                 b[2 * h + 1] = (unsigned long long)__double_as_longlong(pv.y);
             }
-        write_digits2(planes, mreal, grow, ld, y, b, er, ei);
+        write_digits2(planes, grow, nkb, y, b, er, ei);
     }
 }
 
@@ -799,7 +799,7 @@ int cg_iteration_fused(CgRun &R, CgState *st_a, CgState *st_b, int j) {
         dim3 grid((unsigned)ceil_div(rps, RT / 32), (unsigned)R.P.nsys);
         k_cg_p_oz<<<grid, RT, 0, st>>>(R.v.r, R.v.p, R.v.x, R.alpha, Nx, rps, R.part_r, R.npart, st_a, st_b,
                                        R.max_iter, R.reliable, UPDATE_FRAC_FP64_CLASS, R.active,
-                                       static_cast<__nv_bfloat16 *>(R.oz_dg), R.oz_rexp, oz_ld(Nx), rows);
+                                       static_cast<__nv_bfloat16 *>(R.oz_dg), R.oz_rexp, oz_ld(Nx));
     } else {
         dim3 grid(R.P.nblk, (unsigned)R.P.nsys);
         k_cg_p<<<grid, RT, 0, st>>>(R.v.r, R.v.p, R.v.x, R.alpha, R.P.sy, R.P.nblk, R.part_r, R.npart, st_a, st_b,
@@ -1182,7 +1182,7 @@ int cg_run(CgRun &R, const double2 *b, const double2 *x0, double2 *x, double2 *x
             R.oz_second = op == NSLG_OP_MMDAGGER ? Pm : Pd;
             const int64_t rows = nbatch * fm->Nt;
             NSLG_TRY(ws_get(fm, "oz_rexp", (size_t)2 * rows, &R.oz_rexp));
-            NSLG_TRY(ws_get(fm, "oz_digits", (size_t)oz_digits() * 2 * rows * oz_ld((int)fm->Nx) * 2, &R.oz_dg));
+            NSLG_TRY(ws_get(fm, "oz_digits", oz_digit_bytes(rows, (int)fm->Nx), &R.oz_dg));
             R.npart = (int)npart;
             NSLG_TRY(ws_get(fm, "cg_partc", (size_t)(P.nsys * npart), &R.part_c));
             NSLG_TRY(ws_get(fm, "cg_partr", (size_t)(P.nsys * npart), &R.part_r));

@@ -26,16 +26,26 @@
 // launch with it reports NSLG_ERR_CUDA through the handle's tensor-core error flag, so its results are never used
 // silently.
 //
-// GB300's FP64 pipe (~2 operations per clock per SM) and, for N = 32 MMAs, the tensor core's shared-memory operand
-// reads (~44 cycles per M = 128, N = 32, K = 16 instruction measured on this part, 128 at N = 256) bound the work, so:
+// Zero digits. The same localisation leaves most of the digit planes of exp(delta K) empty: digit 0 reaches a site's
+// neighbours within two hops, digit 5 within about eleven. k_oz_planes records which digits of every 32-site x 16-site
+// block are present; k-blocks and digits without an entry are neither loaded nor multiplied (exact: they are zeros).
+// Products left: 237 of 378 per tile at honeycomb 12x12 (delta = 1/8), 388 of 1512 at 24x24 (delta = 12/128).
+//
+// What bounds the work, and what each measure gave (kernel time, M on 64 right-hand sides at 12x12, Nt = 64, and
+// M^dagger on 8 at 24x24, Nt = 128): 86 and 272 us with every digit product its own N = 32 MMA and 2-D tensor copies of
+// 32-byte rows. Skipping zero digits: 90 and 148 us, because the copy engine, about a cycle per 32-byte row, was the
+// limit at 12x12; digits stored in stage order, one contiguous bulk copy per k-block and operand: 73 and 108 us; one
+// MMA per operand digit over all its partners (N up to 192; the tensor core re-read the operand slice from shared memory
+// for every N = 32 MMA, 74 cycles each): 59 and 85 us. What is left is L2 traffic: ~5 TB/s of digits into the SMs.
+//
 //  * k_oz_digits: one warp per (r, t) row computes Y = phase o psi (M) or psi (M^dagger) once (kept in registers
 //    for rows of up to 32 * OZ_CACHE sites), the row's power-of-two scales (real and imaginary rows separately) from
 //    integer maxima of the FP64 bit patterns, and writes the S digit planes of the operand (BF16 pairs, rows padded
 //    to a multiple of 32 sites) with integer operations. FP64 work: the phase product only. (In the fused CG
 //    iteration on M M^dagger the operands come ready: the M^dagger epilogue forms phase o tmp and the CG update
 //    kernel writes the digits of the next search direction.)
-//  * k_fm_apply_oz: a persistent, warp-specialised TMA -> tcgen05 pipeline (see the kernel): 21 digit MMAs per
-//    16-site k-block into S = 6 TMEM accumulators, two accumulator sets so that the epilogue of one 128 x 32 tile
+//  * k_fm_apply_oz: a persistent, warp-specialised TMA -> tcgen05 pipeline (see the kernel): up to 21 digit products per
+//    16-site k-block (6 MMAs) into S = 6 TMEM accumulators, two accumulator sets so that the epilogue of one 128 x 32 tile
 //    overlaps the MMAs of the next; the epilogue recombines the integer-valued G_d in 64-bit integers (exact),
 //    builds the FP64 value from integer operations, then applies the time shift, boundary sign, conj(phase)
 //    (M^dagger) and psi -.
@@ -44,7 +54,6 @@
 // out = (Y o pro) E^T (o epi) of a complex matrix Y with a real matrix E, optionally column-scaled before (in the
 // digit pre-pass) or after (in the epilogue).
 
-#include <cudaTypedefs.h>
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -58,8 +67,8 @@ namespace nslg {
 
 namespace {
 
-constexpr int OZ_BM = 128;       // real GEMM rows per tile (64 complex rows)
-constexpr int OZ_BK = 16;        // sites per k-block: 32 bytes of BF16, one MMA K step
+constexpr int OZ_BM = OZ_TILE_A;       // real GEMM rows per tile (64 complex rows)
+constexpr int OZ_BK = OZ_KB;        // sites per k-block: 32 bytes of BF16, one MMA K step
 constexpr int OZ_NACC = OZ_S;    // one TMEM accumulator per order d < S
 constexpr int OZ_BN = 32;        // output sites per tile
 constexpr int OZ_ROWB = OZ_BK * 2;           // bytes per smem row
@@ -111,22 +120,14 @@ __host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
 }
 
 // D[tmem] (+)= A[smem] * B[smem]^T, kind::f16 (BF16 operands, FP32 accumulation), issued by one thread.
-// COLL selects the A collector buffer: 0 = none, 1 = fill (read A and keep it), 2 = use (A from the buffer),
-// 3 = lastuse (A from the buffer, then released): consecutive MMAs on the same A slice may reuse it (the instruction
-// rate measured on this part is the same with and without the collector, ~44 cycles per N = 32 MMA).
-template <int COLL>
+// (The A collector buffer does not change the instruction rate measured on this part, ~44 cycles per N = 32 MMA.)
 __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
-#define NSLG_MMA_F16(Q)                                                                         \
-    asm volatile("{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16" Q \
-                 " [%0], %1, %2, %3, p;\n}\n" ::"r"(d_tmem),                                   \
-                 "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                           \
-                 : "memory")
-    if constexpr (COLL == 1) NSLG_MMA_F16(".collector::a::fill");
-    else if constexpr (COLL == 2) NSLG_MMA_F16(".collector::a::use");
-    else if constexpr (COLL == 3) NSLG_MMA_F16(".collector::a::lastuse");
-    else NSLG_MMA_F16("");
-#undef NSLG_MMA_F16
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+            d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
 }
 
 // zint 2^e as an FP64 value (rounded to nearest, ties away from zero) from integer operations only: GB300 runs an
@@ -209,23 +210,23 @@ __global__ void __launch_bounds__(256, 2)
         ex[2 * grow] = er;
         ex[2 * grow + 1] = ei;
     }
-    const int64_t mreal = 2 * rows;
+    const int nkb = ld / OZ_BK;
 #pragma unroll
     for (int k = 0; k < NP; ++k) {
         const int y = 2 * (lane + 32 * k);
-        if (y < ld) write_digits2(planes, mreal, grow, ld, y, c[k], er, ei);
+        if (y < ld) write_digits2(planes, grow, nkb, y, c[k], er, ei);
     }
     for (int y = 2 * (lane + 32 * NP); y < ld; y += 64) {
         unsigned long long b[4];
         operand_pair<MODE>(psi, phase, grow, t, Nx, y, b);
-        write_digits2(planes, mreal, grow, ld, y, b, er, ei);
+        write_digits2(planes, grow, nkb, y, b, er, ei);
     }
 }
 
 // Persistent, warp-specialised split-BF16 kernel: one CTA per SM walks the (row block, site block) tiles
 // t = blockIdx.x, blockIdx.x + gridDim.x, ... (site blocks fastest, so the CTAs working at one time share the
 // operand rows of a few row blocks in L2). Warp 0 (one thread) streams the digit tiles of every k-block of every tile
-// through an OZP_STAGES-deep TMA ring; warp 1 (one thread) issues the 21 MMAs per k-block into one of two TMEM
+// through an OZP_STAGES-deep ring of bulk copies; warp 1 (one thread) issues a k-block's MMAs into one of two TMEM
 // accumulator sets (2 x 192 columns) and commits each finished tile to its set's `full` barrier; warps 2..9 (two
 // groups of four, one TMEM lane quarter each; group g takes sites [16 g, 16 g + 16) of the tile) recombine, finish
 // and store a tile while the MMAs of the next one run, then release its accumulator set. Every wait is bounded: a
@@ -235,7 +236,7 @@ template <int MODE, int EPI>
 __global__ void __launch_bounds__(OZP_THREADS, 1)
     k_fm_apply_oz(const double2 *__restrict__ psi, double2 *__restrict__ out, const double2 *__restrict__ phase,
                   const int *__restrict__ row_exp, const int *__restrict__ col_exp,
-                  const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int Nt,
+                  const int *__restrict__ klist, const uint8_t *__restrict__ dga, const uint8_t *__restrict__ dgb, int Nt,
                   int Nx, int64_t rows, int nkb, int *err, const OzEpi epi) {
     constexpr int BN = OZ_BN, STAGE = OZ_STAGE, NACC = OZ_NACC;
     extern __shared__ uint8_t smem_raw[];
@@ -249,7 +250,6 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
     volatile int *abort_flag = reinterpret_cast<volatile int *>(bar_done + 2);
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
-    const int64_t mreal = 2 * rows;
     const int nmt = (int)((rows + OZ_BM / 2 - 1) / (OZ_BM / 2));
     const int ntn = (Nx + BN - 1) / BN;
     const int ntiles = nmt * ntn;
@@ -275,8 +275,6 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
         tc::mbar_init(bar_done, 1);
         *abort_flag = 0;
         tc::fence_mbar_init();
-        tc::prefetch_tmap(&map_a);
-        tc::prefetch_tmap(&map_b);
         if (col_exp[Nx] != 0 && err) atomicExch(err, OZ_ERR_BOUND);  // exp(delta K) failed the digit-sum bound
     }
     if (warp == 1) tc::tmem_alloc(tmem_slot, OZP_TMEM_COLS);
@@ -284,16 +282,22 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
     __syncthreads();
     tc::tc_fence_after();
     const uint32_t tmem = *tmem_slot;
-    constexpr uint32_t idesc = idesc_bf16(OZ_BM, BN);
 
     if (warp == 0) {
         if (lane == 0) {  // TMA producer: S operand-digit tiles and S exp(delta K)-digit tiles per k-block
             int it = 0;
             for (int t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x) {
                 if (!live(t)) continue;
-                const int64_t mrow0 = (int64_t)(t / ntn) * OZ_BM;
-                const int n0 = (t % ntn) * BN;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const uint8_t *at = dga + (int64_t)(t / ntn) * nkb * (OZ_S * OZ_A_SLICE);
+                const uint8_t *bt = dgb + (int64_t)(t % ntn) * nkb * (OZ_S * OZ_B_SLICE);
+                const int *kl = klist + (int64_t)(t % ntn) * (nkb + 1);
+                const int nk = kl[0];
+                int next = kl[1];
+                for (int i = 1; i <= nk; ++i, ++it) {
+                    const int kb = next & 0xFFFF, mask = next >> 16;
+                    if (i < nk) next = kl[i + 1];
+                    // the present digits of exp(delta K) [b0, b1] and the operand digits that meet them
+                    const int b0 = __ffs(mask) - 1, nb = 32 - __clz(mask) - b0, na = OZ_S - b0;
                     const int s = it % OZP_STAGES;
                     if (it >= OZP_STAGES &&
                         (*abort_flag || !tc::mbar_wait(&bar_empty[s], ((it / OZP_STAGES) - 1) & 1, err, 21))) {
@@ -302,13 +306,10 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
                     }
                     uint8_t *a_base = smem + s * STAGE;
                     uint8_t *b_base = a_base + OZ_S * OZ_A_SLICE;
-                    tc::mbar_arrive_expect_tx(&bar_full[s], STAGE);
-#pragma unroll
-                    for (int l = 0; l < OZ_S; ++l) {
-                        tc::tma_load_2d(a_base + l * OZ_A_SLICE, &map_a, kb * OZ_BK, (int)(l * mreal + mrow0),
-                                        &bar_full[s]);
-                        tc::tma_load_2d(b_base + l * OZ_B_SLICE, &map_b, kb * OZ_BK, l * Nx + n0, &bar_full[s]);
-                    }
+                    tc::mbar_arrive_expect_tx(&bar_full[s], na * OZ_A_SLICE + nb * OZ_B_SLICE);
+                    tc::bulk_load(a_base, at + (int64_t)kb * (OZ_S * OZ_A_SLICE), na * OZ_A_SLICE, &bar_full[s]);
+                    tc::bulk_load(b_base + b0 * OZ_B_SLICE, bt + ((int64_t)kb * OZ_S + b0) * OZ_B_SLICE,
+                                  nb * OZ_B_SLICE, &bar_full[s]);
                 }
             }
             // the last copy into each stage has landed (at once in the normal case; bounded after an abort)
@@ -329,7 +330,12 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
                 tc::tc_fence_after();
                 const uint32_t dbase = tmem + (uint32_t)(buf * NACC * BN);
                 bool ok = true;
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const int *kl = klist + (int64_t)(t % ntn) * (nkb + 1);
+                const int nk = kl[0];
+                int next = kl[1];
+                for (int i = 1; i <= nk; ++i, ++it) {
+                    const int mask = next >> 16;
+                    if (i < nk) next = kl[i + 1];  // loaded while this k-block's data arrives
                     const int s = it % OZP_STAGES;
                     if (*abort_flag || !tc::mbar_wait(&bar_full[s], (it / OZP_STAGES) & 1, err, 22)) {
                         ok = false;
@@ -337,26 +343,21 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
                     }
                     // (no tcgen05 fence here: the stage's completed transaction count already makes the TMA writes
                     // visible to the MMAs; a fence per k-block costs ~250 cycles of this thread's issue stream)
-                    // ordered by the operand digit a, so that the A collector buffer serves the S - a products of
-                    // slice a; accumulator d = a + b starts (accumulate = 0) with its first product (0, d) of the
-                    // tile's first k-block. The issue rate of this one thread bounds the kernel (N = 32 MMAs take
-                    // ~17 tensor-pipe cycles each), so every descriptor is the stage's base descriptor plus a
-                    // compile-time offset (the address field is bits 0-13 of the descriptor, in 16-byte units).
+                    // One MMA per operand digit a: the digits b0 <= b <= min(b1, S - 1 - a) of exp(delta K) lie one
+                    // after the other in shared memory (32 rows each), and so do their accumulators d = a + b in
+                    // TMEM, so they are one B operand of N = 32 x (number of digits) and the operand slice is read
+                    // once. The tile's first k-block has every digit, so its a = 0 product (N = 192, accumulate =
+                    // 0) starts all accumulators. Descriptors are the stage's base descriptor plus an offset (the
+                    // address field is bits 0-13, in 16-byte units).
                     const uint64_t dst = dsm0 + (uint64_t)((s * STAGE) >> 4);
-                    const uint32_t acc0 = kb == 0 ? 0u : 1u;
+                    const int b0 = __ffs(mask) - 1, b1 = 31 - __clz(mask);
+                    const uint64_t db = dst + (uint64_t)((OZ_S * OZ_A_SLICE + b0 * OZ_B_SLICE) >> 4);
 #pragma unroll
                     for (int a = 0; a < OZ_S; ++a) {
-                        const uint64_t da = dst + (uint64_t)((a * OZ_A_SLICE) >> 4);
-#pragma unroll
-                        for (int b = 0; b < OZ_S - a; ++b) {
-                            const uint32_t dt = dbase + (uint32_t)((a + b) * BN);
-                            const uint64_t db = dst + (uint64_t)((OZ_S * OZ_A_SLICE + b * OZ_B_SLICE) >> 4);
-                            const uint32_t accum = a == 0 ? acc0 : 1u;
-                            if (OZ_S - a == 1) mma_bf16<0>(dt, da, db, idesc, accum);
-                            else if (b == 0) mma_bf16<1>(dt, da, db, idesc, accum);
-                            else if (b == OZ_S - a - 1) mma_bf16<3>(dt, da, db, idesc, accum);
-                            else mma_bf16<2>(dt, da, db, idesc, accum);
-                        }
+                        if (a >= OZ_S - b0) break;
+                        const int n = min(b1, OZ_S - 1 - a) - b0 + 1;
+                        mma_bf16(dbase + (uint32_t)((a + b0) * BN), dst + (uint64_t)((a * OZ_A_SLICE) >> 4), db,
+                                 idesc_bf16(OZ_BM, n * BN), (i == 1 && a == 0) ? 0u : 1u);
                     }
                     tc::mma_commit(&bar_empty[s]);
                 }
@@ -518,9 +519,9 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
 // ld BF16 (zero padded), the planes stacked along the row axis (S * Nx rows) for one 2-D tensor map. One block of
 // 256 threads per row x; it also evaluates the row's digit-sum bounds (256 sum_{l<=d} B_l(x), B_l(x) = sum_y |b_l|)
 // and sets col_exp[Nx] (zeroed before the launch) when an order d < OZ_EXACT reaches 2^24 or any order 2^30.
-__global__ void __launch_bounds__(256) k_oz_planes(const double2 *__restrict__ E, __nv_bfloat16 *planes, int *col_exp,
-                                                   int Nx, int ld) {
-    const int x = blockIdx.x;
+__global__ void __launch_bounds__(256) k_oz_planes(const double2 *__restrict__ E, char *planes, int *col_exp,
+                                                   int *klist, int Nx, int ld) {
+    const int x = blockIdx.x, nkb = ld / OZ_BK;
     unsigned long long m = 0ull;
     for (int y = threadIdx.x; y < Nx; y += blockDim.x) m = max(m, abs_bits(E[(int64_t)x * Nx + y].x));
     __shared__ unsigned long long red[256];
@@ -542,8 +543,12 @@ __global__ void __launch_bounds__(256) k_oz_planes(const double2 *__restrict__ E
         balanced_digits(scaled_int((unsigned long long)__double_as_longlong(v), e), a);
 #pragma unroll
         for (int l = 0; l < OZ_S; ++l) {
-            planes[((int64_t)l * Nx + x) * ld + y] = __float2bfloat16_rn(a[l]);
+            *reinterpret_cast<__nv_bfloat16 *>(planes + digit_offset<OZ_BN>(x, l, y, nkb)) = __float2bfloat16_rn(a[l]);
             B[l] += (int)fabsf(a[l]);
+            // (ld is a multiple of 32: the whole warp is here, half a warp covers one k-block)
+            const unsigned nz = __ballot_sync(0xffffffffu, a[l] != 0.f);
+            if (threadIdx.x % 16 == 0 && (nz >> (threadIdx.x % 32) & 0xFFFF))
+                atomicOr(&klist[(int64_t)(x / OZ_BN) * (nkb + 1) + 1 + y / OZ_BK], 1 << l);
         }
     }
     const int lane = threadIdx.x % 32, warp = threadIdx.x / 32;
@@ -567,31 +572,31 @@ __global__ void __launch_bounds__(256) k_oz_planes(const double2 *__restrict__ E
     }
 }
 
-PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
-    static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
-    if (!fn) {
-        cudaDriverEntryPointQueryResult q;
-        void *p = nullptr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+// Digit masks per k-block (k_oz_planes) -> the k-blocks each output tile works through: klist[tile (nkb + 1)] = count,
+// then k-block | mask << 16, the one with the most products first and with every digit (it starts all accumulators),
+// k-blocks without a digit left out. One thread per tile.
+__global__ void k_oz_klist(int *klist, int ntn, int nkb) {
+    const int nt = blockIdx.x * blockDim.x + threadIdx.x;
+    if (nt >= ntn) return;
+    int *kl = klist + (int64_t)nt * (nkb + 1);
+    int first = 0, most = -1;
+    for (int kb = 0; kb < nkb; ++kb) {
+        int products = 0;
+        for (int b = 0; b < OZ_S; ++b) products += (kl[1 + kb] >> b & 1) * (OZ_S - b);
+        if (products > most) {
+            most = products;
+            first = kb;
+        }
     }
-    return fn;
-}
-
-int make_map_bf16(CUtensorMap *map, const void *base, int64_t rows, int ld, int box_rows) {
-    auto fn = encode_fn();
-    NSLG_REQUIRE(fn != nullptr, NSLG_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-    const cuuint64_t dims[2] = {(cuuint64_t)ld, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t box[2] = {(cuuint32_t)OZ_BK, (cuuint32_t)box_rows};
-    const cuuint32_t estr[2] = {1, 1};
-    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void *>(base), dims, strides, box, estr,
-                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_32B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    NSLG_REQUIRE(r == CUDA_SUCCESS, NSLG_ERR_CUDA,
-                 "cuTensorMapEncodeTiled (bf16) failed (" + std::to_string((int)r) + ")");
-    return NSLG_OK;
+    kl[1 + first] = 0;
+    int n = 0;
+    for (int kb = 0; kb < nkb; ++kb) {  // compacts in place: n never passes kb
+        const int mask = kl[1 + kb];
+        if (mask) kl[1 + n++] = kb | mask << 16;
+    }
+    kl[1 + n] = n > 0 ? kl[1] : 0;
+    kl[1] = first | ((1 << OZ_S) - 1) << 16;
+    kl[0] = n + 1;
 }
 
 int set_smem_attr() {
@@ -629,7 +634,9 @@ unsigned oz_grid(int64_t rows, int Nx) {
 }  // namespace
 
 int oz_ld(int Nx) { return (int)ceil_div(Nx, OZ_LD_ALIGN) * OZ_LD_ALIGN; }
-int oz_digits() { return OZ_S; }
+size_t oz_digit_bytes(int64_t rows, int Nx) {
+    return (size_t)ceil_div(2 * rows, OZ_BM) * (oz_ld(Nx) / OZ_BK) * OZ_S * OZ_A_SLICE;
+}
 
 int oz_planes(nslg_fm *fm, const ExpEntry *e, OzPlanes **out) {
     auto *E = const_cast<ExpEntry *>(e);
@@ -639,22 +646,28 @@ int oz_planes(nslg_fm *fm, const ExpEntry *e, OzPlanes **out) {
         NSLG_REQUIRE(Nx <= 2048, NSLG_ERR_UNSUPPORTED, "split-BF16 operator supports Nx <= 2048");
         auto *P = new OzPlanes;
         P->ld = oz_ld(Nx);
-        const size_t n = (size_t)OZ_S * Nx * P->ld;
+        const int ntn = (int)ceil_div(Nx, OZ_BN), nkb = P->ld / OZ_BK;
+        const size_t nlist = (size_t)ntn * (nkb + 1);
+        const size_t bytes = (size_t)ntn * nkb * OZ_S * OZ_B_SLICE;  // rows padded to whole tiles, zero
         // col_exp[Nx] is the digit-sum bound flag
-        if (cudaMalloc(&P->planes, n * sizeof(__nv_bfloat16)) != cudaSuccess ||
-            cudaMalloc(&P->col_exp, (Nx + 1) * sizeof(int)) != cudaSuccess) {
+        if (cudaMalloc(&P->planes, bytes) != cudaSuccess ||
+            cudaMalloc(&P->col_exp, (Nx + 1) * sizeof(int)) != cudaSuccess ||
+            cudaMalloc(&P->klist, nlist * sizeof(int)) != cudaSuccess) {
             cudaGetLastError();
             cudaFree(P->planes);
+            cudaFree(P->col_exp);
             delete P;
             set_error("split-BF16 planes: device allocation failed");
             return NSLG_ERR_OOM;
         }
         NSLG_CUDA(cudaMemsetAsync(P->col_exp + Nx, 0, sizeof(int), fm->ctx->stream));
-        k_oz_planes<<<Nx, 256, 0, fm->ctx->stream>>>(E->full, static_cast<__nv_bfloat16 *>(P->planes), P->col_exp,
-                                                      Nx, P->ld);
-        note_launch(fm->ctx->stream);
+        NSLG_CUDA(cudaMemsetAsync(P->planes, 0, bytes, fm->ctx->stream));
+        NSLG_CUDA(cudaMemsetAsync(P->klist, 0, nlist * sizeof(int), fm->ctx->stream));
+        k_oz_planes<<<Nx, 256, 0, fm->ctx->stream>>>(E->full, static_cast<char *>(P->planes), P->col_exp,
+                                                      P->klist, Nx, P->ld);
+        k_oz_klist<<<1, 64, 0, fm->ctx->stream>>>(P->klist, ntn, nkb);  // ntn <= 64 (Nx <= 2048)
+        note_launch(fm->ctx->stream, 2);
         NSLG_CUDA(cudaGetLastError());
-        NSLG_TRY(make_map_bf16(&P->map, P->planes, (int64_t)OZ_S * Nx, P->ld, OZ_BN));
         NSLG_TRY(set_smem_attr());
         E->oz = P;
     }
@@ -667,14 +680,14 @@ namespace {
 
 template <int EPI>
 void launch_oz(int mode, dim3 grid, cudaStream_t st, const double2 *psi, double2 *out, const double2 *phase,
-               const int *rexp, const int *col_exp, const CUtensorMap &map_a, const CUtensorMap &map_b, int Nt, int Nx,
-               int64_t rows, int nkb, int *err, const OzEpi &epi) {
+               const int *rexp, const int *col_exp, const int *klist, const uint8_t *dga, const uint8_t *dgb,
+               int Nt, int Nx, int64_t rows, int nkb, int *err, const OzEpi &epi) {
     if (mode == MODE_M)
-        k_fm_apply_oz<MODE_M, EPI><<<grid, OZP_THREADS, OZP_SMEM, st>>>(psi, out, phase, rexp, col_exp, map_a, map_b,
+        k_fm_apply_oz<MODE_M, EPI><<<grid, OZP_THREADS, OZP_SMEM, st>>>(psi, out, phase, rexp, col_exp, klist, dga, dgb,
                                                                         Nt, Nx, rows, nkb, err, epi);
     else
-        k_fm_apply_oz<MODE_MDAG, EPI><<<grid, OZP_THREADS, OZP_SMEM, st>>>(psi, out, phase, rexp, col_exp, map_a,
-                                                                           map_b, Nt, Nx, rows, nkb, err, epi);
+        k_fm_apply_oz<MODE_MDAG, EPI><<<grid, OZP_THREADS, OZP_SMEM, st>>>(psi, out, phase, rexp, col_exp, klist, dga,
+                                                                           dgb, Nt, Nx, rows, nkb, err, epi);
 }
 
 }  // namespace
@@ -692,12 +705,11 @@ int oz_gemm(const double2 *Y, double2 *out, const double2 *pro_scale, const doub
     else k_oz_digits<MODE_MDAG><<<blocks, 256, 0, st>>>(Y, nullptr, 1, Nx, rows, P.ld, dg, rexp, nullptr, 1);
     note_launch(st);
     NSLG_CUDA(cudaGetLastError());
-    CUtensorMap map_a;
-    NSLG_TRY(make_map_bf16(&map_a, digits, (int64_t)OZ_S * 2 * rows, P.ld, OZ_BM));
+    const auto *dga = static_cast<const uint8_t *>(digits), *dgb = static_cast<const uint8_t *>(P.planes);
     const int nkb = P.ld / OZ_BK;
     const OzEpi plain;
     k_fm_apply_oz<MODE_OZ_GEMM, 0><<<oz_grid(rows, Nx), OZP_THREADS, OZP_SMEM, st>>>(
-        nullptr, out, epi_scale, rexp, P.col_exp, map_a, P.map, 1, Nx, rows, nkb, err, plain);
+        nullptr, out, epi_scale, rexp, P.col_exp, P.klist, dga, dgb, 1, Nx, rows, nkb, err, plain);
     note_launch(st);
     NSLG_CUDA(cudaGetLastError());
     return NSLG_OK;
@@ -724,16 +736,15 @@ int fm_apply_oz(int mode, const double2 *psi, double2 *out, const double2 *phase
         note_launch(st);
         NSLG_CUDA(cudaGetLastError());
     }
-    CUtensorMap map_a;
-    NSLG_TRY(make_map_bf16(&map_a, digits, (int64_t)OZ_S * 2 * rows, P.ld, OZ_BM));
+    const auto *dga = static_cast<const uint8_t *>(digits), *dgb = static_cast<const uint8_t *>(P.planes);
     const int nkb = P.ld / OZ_BK;
     const dim3 grid(oz_grid(rows, Nx));
     if (E.mode == 1)
-        launch_oz<1>(mode, grid, st, psi, out, phase, rexp, P.col_exp, map_a, P.map, Nt, Nx, rows, nkb, err, E);
+        launch_oz<1>(mode, grid, st, psi, out, phase, rexp, P.col_exp, P.klist, dga, dgb, Nt, Nx, rows, nkb, err, E);
     else if (E.mode == 2)
-        launch_oz<2>(mode, grid, st, psi, out, phase, rexp, P.col_exp, map_a, P.map, Nt, Nx, rows, nkb, err, E);
+        launch_oz<2>(mode, grid, st, psi, out, phase, rexp, P.col_exp, P.klist, dga, dgb, Nt, Nx, rows, nkb, err, E);
     else
-        launch_oz<0>(mode, grid, st, psi, out, phase, rexp, P.col_exp, map_a, P.map, Nt, Nx, rows, nkb, err, E);
+        launch_oz<0>(mode, grid, st, psi, out, phase, rexp, P.col_exp, P.klist, dga, dgb, Nt, Nx, rows, nkb, err, E);
     note_launch(st);
     NSLG_CUDA(cudaGetLastError());
     return NSLG_OK;

@@ -29,13 +29,13 @@ struct TcPlanes {
     CUtensorMap map_hi, map_lo;
 };
 
-// Split-BF16 digit planes of a real exp(d K) (S planes stacked along rows), per-row scale exponents and the TMA
-// descriptor (B operand of the exact-accumulation tensor-core operator).
+// Split-BF16 digit planes of a real exp(d K) (the B operand of the exact-accumulation tensor-core operator, in the layout
+// of oz_digits.cuh) and per-row scale exponents.
 struct OzPlanes {
-    void *planes = nullptr;  // BF16, (S * Nx, ld)
+    void *planes = nullptr;  // BF16
     int *col_exp = nullptr;  // (Nx)
+    int *klist = nullptr;    // per tile of output sites: the k-blocks with a nonzero digit and which digits (k_oz_klist)
     int ld = 0;
-    CUtensorMap map;
 };
 
 // exp(d K) memo entry (SpatialLattice::exp_hopping_matrix, lattice.tpp:52-58), kept in the layouts the kernels read.
@@ -231,7 +231,7 @@ int fm_apply_tc(int mode, const double2 *psi, double2 *out, const double2 *phase
                 int64_t rows, int *err, cudaStream_t st);
 int oz_planes(nslg_fm *fm, const ExpEntry *e, OzPlanes **out);
 int oz_ld(int Nx);   // digit-plane row length (Nx rounded up to the 32-site k-block)
-int oz_digits();     // digits per operand
+size_t oz_digit_bytes(int64_t rows, int Nx);  // workspace for the operand digits of `rows` complex rows
 // Epilogue extensions of the split-BF16 kernel for the CG on MM^dagger / M^dagger M (mode 0: plain application).
 // mode 1 (first factor): out is written and part[(2 row + c) * oz_ntiles(Nx) + n-tile] = sum of out^2 over the
 //   tile's sites, the curvature partial sums |M^dagger p|^2.
@@ -262,7 +262,7 @@ int oz_ntiles(int Nx);  // output-site tiles of the split-BF16 kernel (partial s
 // (rows, Nx), E the real matrix of the planes P; pro / epi may be null (no scale). digits / rexp as fm_apply_oz.
 int oz_gemm(const double2 *Y, double2 *out, const double2 *pro_scale, const double2 *epi_scale, const OzPlanes &P,
             void *digits, int *rexp, int Nx, int64_t rows, int *err, cudaStream_t st);
-// digits: workspace of oz_digits() * 2 * rows * oz_ld(Nx) BF16; rexp: 2 * rows ints (per-row scale exponents).
+// digits: workspace of oz_digit_bytes(rows, Nx); rexp: 2 * rows ints (per-row scale exponents).
 int fm_apply_oz(int mode, const double2 *psi, double2 *out, const double2 *phase, const OzPlanes &P, void *digits,
                 int *rexp, int Nt, int Nx, int64_t rows, int *err, cudaStream_t st, const OzEpi *epi = nullptr);
 

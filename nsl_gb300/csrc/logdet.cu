@@ -870,7 +870,7 @@ int grad_logdet_tc_many(nslg_fm *fm, int nmat, const ExpEntry *const *E, const d
     NSLG_TRY(ws_get(fm, "gr_S", (size_t)nmat * ms, &T));
     NSLG_TRY(ws_get(fm, "gr_P", (size_t)nmat * ms, &P));
     NSLG_TRY(ws_get(fm, "gr_G", (size_t)nmat * nn, &G));
-    const size_t dg_elems = (size_t)oz_digits() * 2 * n * oz_ld(n) * 2;  // digit planes of one product (bytes/2)
+    const size_t dg_elems = oz_digit_bytes(n, n);  // digits of one product's operand
     char *dg;
     int *rexp;
     NSLG_TRY(ws_get(fm, "fz_digits", dg_elems * nmat, &dg));

@@ -60,21 +60,36 @@ __device__ __forceinline__ int scale_exponent(unsigned long long maxbits) {
     return maxbits == 0 ? 0 : (int)(maxbits >> 52) - 1022;
 }
 
+// Digit planes in memory: the operand of the tensor-core kernel, already in the layout of its shared-memory stages, so
+// that a k-block's digits of a tile are one contiguous bulk copy (a 2-D tensor copy of 32-byte rows costs the copy engine
+// about a cycle per row, which bounded the kernel). GEMM rows are grouped by `tile` (128 for the operand, 32 for
+// exp(delta K)), sites by OZ_KB = 16: block (row / tile, site / 16, digit) holds tile rows of 32 bytes in the 32-byte
+// swizzle of the MMA descriptors (the 16-byte half of a row is exchanged in rows with bit 2 set).
+constexpr int OZ_KB = 16;       // sites per k-block
+constexpr int OZ_TILE_A = 128;  // GEMM rows (real and imaginary parts) per operand tile
+
+// Byte offset of (row, digit l, site y); nkb = k-blocks per row.
+template <int TILE> __host__ __device__ __forceinline__ int64_t digit_offset(int64_t row, int l, int y, int nkb) {
+    const int m = (int)(row % TILE);
+    return (((row / TILE) * nkb + y / OZ_KB) * OZ_S + l) * (TILE * 32) + m * 32 + (((y >> 3 & 1) ^ (m >> 2 & 1)) << 4) +
+           (y & 7) * 2;
+}
+
 // Digits of the complex operand values at sites y, y + 1 (y even) given by their FP64 bit patterns (integer work
 // only: scale, round, digits), written as BF16 pairs.
-__device__ __forceinline__ void write_digits2(__nv_bfloat16 *__restrict__ planes, int64_t mreal, int64_t grow,
-                                              int ld, int y, const unsigned long long (&b)[4], int er, int ei) {
+__device__ __forceinline__ void write_digits2(__nv_bfloat16 *__restrict__ planes, int64_t grow, int nkb, int y,
+                                              const unsigned long long (&b)[4], int er, int ei) {
     float a0[OZ_S], a1[OZ_S], i0[OZ_S], i1[OZ_S];
     balanced_digits(scaled_int(b[0], er), a0);
     balanced_digits(scaled_int(b[1], ei), i0);
     balanced_digits(scaled_int(b[2], er), a1);
     balanced_digits(scaled_int(b[3], ei), i1);
+    // the real and the imaginary row are neighbours in one tile and share the swizzle bit (bit 2 of an even row)
+    char *p = reinterpret_cast<char *>(planes) + digit_offset<OZ_TILE_A>(2 * grow, 0, y, nkb);
 #pragma unroll
     for (int l = 0; l < OZ_S; ++l) {
-        *reinterpret_cast<__nv_bfloat162 *>(planes + ((int64_t)l * mreal + 2 * grow) * ld + y) =
-            __floats2bfloat162_rn(a0[l], a1[l]);
-        *reinterpret_cast<__nv_bfloat162 *>(planes + ((int64_t)l * mreal + 2 * grow + 1) * ld + y) =
-            __floats2bfloat162_rn(i0[l], i1[l]);
+        *reinterpret_cast<__nv_bfloat162 *>(p + l * (OZ_TILE_A * 32)) = __floats2bfloat162_rn(a0[l], a1[l]);
+        *reinterpret_cast<__nv_bfloat162 *>(p + l * (OZ_TILE_A * 32) + 32) = __floats2bfloat162_rn(i0[l], i1[l]);
     }
 }
 

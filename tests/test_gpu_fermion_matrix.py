@@ -216,3 +216,46 @@ def test_cuda_core_operator_splits(Nx, Nt, R):
             for op, want, size in (("M", wantM, sizeM), ("Mdagger", wantD, sizeD)):
                 err = np.abs(getattr(fm, op)(psi, precision=prec) - want)
                 assert np.all(err <= 4 * (Nx + 8) * eps * size), (prec, op, (err / size).max())
+
+
+@pytest.mark.parametrize("Nx", [1, 16, 17, 32, 33, 63, 96, 145, 320])
+@pytest.mark.parametrize("kind", ["identity", "banded", "far", "zero_row", "dense"])
+def test_split_operator_skips_zero_digits(Nx, kind):
+    """The split-BF16 operator with exp(delta K) whose digit blocks are mostly empty: the identity, a narrow band, a band
+    plus entries in far k-blocks that only low digits represent, a zero row, and a dense one. Bound: operands rounded to
+    2^-53 of their row's maximum and the dropped orders, 32 Nx 2^-53 max|E| max|Y| per row. A matrix beyond the
+    digit-sum bound (the dense one at 320 sites) is refused."""
+    import nsl_gb300 as N
+    from test_split_digits import bounds_ok, digit_sum_bounds
+
+    Nt, R = 5, 3
+    rng = np.random.default_rng(Nx)
+    i, j = np.arange(Nx)[:, None], np.arange(Nx)[None, :]
+    E = np.eye(Nx)
+    if kind == "banded":
+        E = np.exp(-3.0 * np.abs(i - j)) * (np.abs(i - j) < 6)
+    elif kind == "far":
+        E = E + 2.0 ** -40 * (np.abs(i - j) > Nx // 2) + 2.0 ** -20 * (np.abs(i - j) == 3)
+    elif kind == "zero_row":
+        E[Nx // 2] = 0.0
+    elif kind == "dense":
+        E = rng.uniform(-1, 1, (Nx, Nx)) / Nx + E
+    lat = N.Ring(Nx)
+    lat.set_exp_hopping_matrix(0.125, E)
+    fm = N.HubbardExp(lat, Nt, 0.125 * Nt)
+    phi = rng.standard_normal((Nt, Nx)) + 0j
+    psi = (rng.standard_normal((R, Nt, Nx)) + 1j * rng.standard_normal((R, Nt, Nx))) * np.exp(rng.uniform(-9, 9, (R, Nt, 1)))
+    fm.populate(phi)
+    ph = np.exp(1j * phi)
+    sign = np.where(np.arange(Nt) == 0, -1.0, 1.0)[:, None]
+    if not bounds_ok(digit_sum_bounds(E)):
+        with pytest.raises(RuntimeError, match="delocalised"):
+            fm.M(psi, precision="bf16split")
+            fm.ctx.synchronize()
+        return
+    eps = 32 * Nx * 2.0 ** -53 * np.abs(E).max()
+    for op, want, row in (("M", psi - sign * np.roll((ph * psi) @ E.T, 1, 1), np.roll(np.abs(psi).max(2), 1, 1)),
+                          ("Mdagger", psi - np.conj(ph) * np.roll(sign * (psi @ E.T), -1, 1),
+                           np.roll(np.abs(psi).max(2), -1, 1))):
+        err = np.abs(getattr(fm, op)(psi, precision="bf16split") - want).max(2)
+        assert np.all(err <= eps * row + 2.0 ** -51 * np.abs(want).max(2)), (op, (err / row).max())
