@@ -160,6 +160,33 @@ template <typename T>
 int fm_apply_dev(nslg_fm *fm, int op, const double2 *psi, double2 *out, int64_t nbatch,
                  const int *sys_mask = nullptr, int64_t sys_rows = 1);
 
+// One batched complex FP64 product, row-major: C = alpha (A o kscale) B, rows scaled by rscale, (+ I) (+ C). Matrices of
+// a two-level batch (z1, z2) lie at z1 s + z2 s2 elements; the scales alike.
+struct ZProd {
+    int M, N, K;
+    double2 alpha{1, 0};
+    const double2 *A;
+    int64_t lda, sA, sA2 = 0;
+    const double2 *B;
+    int64_t ldb, sB, sB2 = 0;
+    double2 *C;
+    int64_t ldc, sC, sC2 = 0;
+    int batch2 = 1;
+    int real = 0;             // 1: A holds real numbers, 2: B does (imaginary parts zero: half the FMAs)
+    bool a_adjoint = false;   // A is given as its adjoint (K, M)
+    bool a_upper = false;     // A is upper triangular
+    bool upper = false;       // only the upper triangle of C is computed
+    bool add_identity = false, accumulate = false;
+    const double2 *kscale = nullptr;  // (K): column scale of A
+    int64_t sks = 0, sks2 = 0;
+    const double2 *rscale = nullptr;  // (M): row scale of the product
+    int64_t srs = 0, srs2 = 0;
+    ZProd(int M, int N, int K, const double2 *A, int64_t lda, int64_t sA, const double2 *B, int64_t ldb, int64_t sB,
+          double2 *C, int64_t ldc, int64_t sC)
+        : M(M), N(N), K(K), A(A), lda(lda), sA(sA), B(B), ldb(ldb), sB(sB), C(C), ldc(ldc), sC(sC) {}
+};
+int zprod(cudaStream_t st, const ZProd &p, int batch);
+
 // C[b] = alpha * A[b] @ B[b] (+ I if add_identity), complex FP64, row-major, batched with element strides.
 int zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2 *A, int64_t lda, int64_t sA,
           const double2 *B, int64_t ldb, int64_t sB, double2 *C, int64_t ldc, int64_t sC, int batch,
@@ -174,9 +201,9 @@ int compute_phases(nslg_fm *fm);
 int populate_dev(nslg_fm *fm, const double2 *phi, int species);  // phi: device buffer (Nt, Nx)
 // Batched FP64 gradient / log det over nmat matrices (logdet.cu): matrix g uses (g & emask) ? E1 : E0 and the
 // phase rows at ph + g * Nt * Nx; grad out (nmat, Nt, Nx) on the device, log det out[nmat] on the host.
-int grad_logdet_many(nslg_fm *fm, int nmat, const double2 *E0, const double2 *E1, int emask, const double2 *ph_inv,
+int grad_logdet_many(nslg_fm *fm, int nmat, const ExpEntry *E0, const ExpEntry *E1, int emask, const double2 *ph_inv,
                      double2 *out);
-int logdet_many(nslg_fm *fm, int nmat, const double2 *E0, const double2 *E1, int emask, const double2 *ph,
+int logdet_many(nslg_fm *fm, int nmat, const ExpEntry *E0, const ExpEntry *E1, int emask, const double2 *ph,
                 double2 *out);
 // Split-BF16 (tensor-core) gradient for nmat matrices with factors E[g] (real, Nx <= 2048); LU and solves batched.
 int grad_logdet_tc_many(nslg_fm *fm, int nmat, const ExpEntry *const *E, const double2 *ph_inv, double2 *out);

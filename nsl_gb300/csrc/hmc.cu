@@ -174,15 +174,15 @@ int populate_dev(nslg_fm *fm, const double2 *phi, int species) {
 namespace {
 
 // The time-slice factors of the gradient for both species: exp(-sgn delta K) (Exp) or 1 - sgn delta K (Diag).
-int grad_factors(nslg_fm *fm, const double2 **EP, const double2 **EH) {
+int grad_factors(nslg_fm *fm, const ExpEntry **EP, const ExpEntry **EH) {
     const ExpEntry *e[2];
     for (int s = 0; s < 2; ++s) {
         const int sgn = s == 0 ? 1 : -1;
         if (fm->kind == NSLG_FM_DIAG) NSLG_TRY(get_lin(fm, make_double2(sgn * fm->delta.x, sgn * fm->delta.y), 1, &e[s]));
         else NSLG_TRY(get_exp(fm, make_double2(-sgn * fm->delta.x, -sgn * fm->delta.y), &e[s]));
     }
-    *EP = e[0]->full;
-    *EH = e[1]->full;
+    *EP = e[0];
+    *EH = e[1];
     return NSLG_OK;
 }
 
@@ -212,7 +212,7 @@ int fermion_grads_many(nslg_fm *fm, const double2 *phi, int64_t nconf, double2 *
         }
         NSLG_TRY(grad_logdet_strat(fm, (int)(2 * nconf), Ep.data(), Ed.data(), ph, ph_inv, g2));
     } else {
-        const double2 *EP, *EH;
+        const ExpEntry *EP, *EH;
         NSLG_TRY(grad_factors(fm, &EP, &EH));
         NSLG_TRY(grad_logdet_many(fm, (int)(2 * nconf), EP, EH, 1, ph_inv, g2));
     }
@@ -254,20 +254,21 @@ int fermion_grads_tc_pair(nslg_fm *fm, const double2 *phi, double2 *g2) {
     return NSLG_OK;
 }
 
-// gP = grad log det M_P(phi), gH = grad log det M_H(phi); leaves fm populated with the hole species. When
+// gP = grad log det M_P(phi), gH = grad log det M_H(phi); leaves fm populated with the hole species (without `populate`,
+// where the species are computed as a pair, with what it was before). When
 // gH = gP + Nt * Nx both species are computed as a pair: in FP64 as one batch of two matrices, in split-BF16 with
 // the LU of the pair batched; otherwise one species after the other.
-int fermion_grads(nslg_fm *fm, const double2 *phi, double2 *gP, double2 *gH) {
+int fermion_grads(nslg_fm *fm, const double2 *phi, double2 *gP, double2 *gH, bool populate = true) {
     if (gH == gP + fm->Nt * fm->Nx) {
         // small lattices (Nx <= 32) take the FP64 pair whatever the force precision: their gradient is a few
         // latency-bound launches (scans, one Gauss-Jordan inverse) that tensor-core products would not shorten
         if (fm->force_precision == NSLG_PREC_FP64 || fm->Nx <= 32 || use_stratified_grad(fm)) {
             NSLG_TRY(fermion_grads_many(fm, phi, 1, gP));
-            return populate_dev(fm, phi, NSLG_HOLE);
+            return populate ? populate_dev(fm, phi, NSLG_HOLE) : (int)NSLG_OK;
         }
         if (fm->force_precision == NSLG_PREC_BF16_SPLIT) {
             const int rc = fermion_grads_tc_pair(fm, phi, gP);
-            if (rc == NSLG_OK) return populate_dev(fm, phi, NSLG_HOLE);
+            if (rc == NSLG_OK) return populate ? populate_dev(fm, phi, NSLG_HOLE) : (int)NSLG_OK;
             if (rc != NSLG_ERR_UNSUPPORTED) return rc;
         }
     }
@@ -397,7 +398,8 @@ int leapfrog_steps(nslg_fm *fm, double2 *q, double2 *p, double2 Ut, const double
         const double ck = (step == 0 || step == nmd) ? 0.5 * eps : eps;
         const double cd = (step == nmd) ? 0.0 : eps;
         if (nconf == 1) {
-            if (terms & 2) NSLG_TRY(fermion_grads(fm, q, gP, gH));
+            // the handle is left populated with the trajectory's last field only
+            if (terms & 2) NSLG_TRY(fermion_grads(fm, q, gP, gH, step == nmd));
             k_kick_drift<<<grid, 256, 0, st>>>(gP, gH, q, p, nullptr, uin, terms, real_force, ck, cd, n);
         } else {
             if (terms & 2) NSLG_TRY(fermion_grads_many(fm, q, nconf, gP));
@@ -596,7 +598,7 @@ int hubbard_eval_batch_dev(nslg_fm *fm, const double2 *phi, int64_t nconf, doubl
                 }
                 NSLG_TRY(logdet_strat(fm, (int)(2 * nconf), Ep.data(), Ed.data(), sg.data(), ph, ph_inv, ld.data()));
             } else {
-                NSLG_TRY(logdet_many(fm, (int)(2 * nconf), EP->full, EH->full, 1, ph, ld.data()));
+                NSLG_TRY(logdet_many(fm, (int)(2 * nconf), EP, EH, 1, ph, ld.data()));
             }
         } else {
             for (int64_t b = 0; b < nconf; ++b) {

@@ -2,9 +2,7 @@
 // exp(d K) of the hopping matrix (SpatialLattice::exp_hopping_matrix, lattice.tpp:52-58) and the phase factors of
 // HubbardExp::populate (hubbardExp.hpp:116-128).
 
-#include <cstdlib>
-#include <map>
-#include <mutex>
+#include <algorithm>
 #include <tuple>
 
 #include "fm_internal.cuh"
@@ -13,167 +11,161 @@ namespace nslg {
 
 namespace {
 
-constexpr int GK = 8;  // reduction depth per stage
+// C = alpha * (A o kscale) @ B (o rscale) (+ I) (+ C with accumulate), batched over blockIdx.z.
+//
+// GB300 runs FP64 at ~2 FMAs per clock per SM: a warp's DFMA occupies its scheduler for 64 cycles, so operand reads from
+// shared memory and L1 fit in its shadow and what matters is that no lane computes padding and that all 608 schedulers
+// have equal work. A thread owns one column of TM consecutive rows; a CTA's threads are the flattened (row group,
+// column) pairs of whole rows (N <= 256) or a run of columns of one row group; A is staged in shared memory, B is read
+// in place (consecutive lanes, consecutive columns). zsplit() picks the split. Every output sums over k in ascending
+// order whatever the split. Measured: the 32 products of 50 x 50 complex matrices of a chain step 58 -> 25 us (of it a factor of two from a real factor), 26 real-by-complex
+// products at n = 288 2.82 -> 2.07 ms (the rate of the FP64 pipe).
+// REAL: 1 = A holds real numbers (imaginary parts zero), 2 = B does; the product then skips the FMAs with the zero
+// imaginary parts (2 instead of 4 per term). TA: A is given as its adjoint (A[i, k] = conj(At[k lda + i])).
+constexpr int ZKC = 32;    // reduction depth per staged chunk
+constexpr int ZMAXT = 256;  // threads per CTA at most
 
-// C = alpha * A @ B (+ I) (+ C with accumulate), batched over blockIdx.z. A CTA owns a TB x TB tile of C; (TB/TI)^2 threads each own a
-// TI x TI block (rows ty + (TB/TI) i, cols tx + (TB/TI) j). GB300 runs FP64 at ~2 FMAs per clock per SM, so what
-// matters is that every SM gets work: large or batched products use 64-wide tiles, a single product of a few hundred
-// rows uses 16-wide tiles (324 CTAs for Nx = 288 instead of 25).
-// REAL: bit 0 = A holds real numbers (imaginary parts zero), bit 1 = B does; the product then skips the FMAs with
-// the zero imaginary parts (2 instead of 4 per term), which is what bounds these FP64 products.
-template <int TB, int TI, int REAL = 0>
-__global__ void __launch_bounds__((TB / TI) * (TB / TI))
-    k_zgemm(int M, int N, int K, double2 alpha, const double2 *__restrict__ A, int64_t lda, int64_t sA,
-            const double2 *__restrict__ B, int64_t ldb, int64_t sB, double2 *__restrict__ C, int64_t ldc, int64_t sC,
-            bool add_identity, bool accumulate, int batch2, int64_t sA2, int64_t sB2, int64_t sC2) {
-    constexpr int TD = TB / TI;  // threads per tile edge
-    constexpr int NT = TD * TD;
-    static_assert((TB * GK) % NT == 0, "tile loads");
-    __shared__ double2 As[GK][TB + 1];
-    __shared__ double2 Bs[GK][TB + 1];
-    const int tid = threadIdx.x, tx = tid % TD, ty = tid / TD;
-    const int m0 = blockIdx.x * TB, n0 = blockIdx.y * TB;
-    // two-level batch: z = z1 * batch2 + z2
-    const int z1 = blockIdx.z / batch2, z2 = blockIdx.z % batch2;
-    A += sA * z1 + sA2 * z2;
-    B += sB * z1 + sB2 * z2;
-    C += sC * z1 + sC2 * z2;
-
-    double2 acc[TI][TI];
+template <int REAL, bool TA, int TM>
+__global__ void __launch_bounds__(ZMAXT) k_zgemm(ZProd p, int G, int CW) {
+    extern __shared__ double2 As[];  // (G TM) x LS
+    const int LS = min(ZKC, p.K) + 1;
+    const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32, nwarps = blockDim.x / 32;
+    const int R = G * TM;
+    const int m0 = blockIdx.x * R;
+    const int z1 = blockIdx.z / p.batch2, z2 = blockIdx.z % p.batch2;
+    const double2 *A = p.A + p.sA * z1 + p.sA2 * z2;
+    const double2 *B = p.B + p.sB * z1 + p.sB2 * z2;
+    double2 *C = p.C + p.sC * z1 + p.sC2 * z2;
+    const double2 *ks = p.kscale ? p.kscale + p.sks * z1 + p.sks2 * z2 : nullptr;
+    const int g = tid / CW, c = tid - g * CW;
+    const int col = blockIdx.y * CW + c;
+    if (p.upper && min(p.N, (int)(blockIdx.y + 1) * CW) <= m0) return;  // every column of this CTA is left of its rows
+    const bool act = g < G && col < p.N && m0 + g * TM < p.M;
+    double2 acc[TM];
 #pragma unroll
-    for (int i = 0; i < TI; ++i)
-#pragma unroll
-        for (int j = 0; j < TI; ++j) acc[i][j] = make_double2(0, 0);
-
-    for (int k0 = 0; k0 < K; k0 += GK) {
-#pragma unroll
-        for (int l = 0; l < TB * GK / NT; ++l) {
-            const int idx = tid + NT * l;
-            // A tile TB x GK: thread -> (row = idx / GK, k = idx % GK)
-            const int ar = idx / GK, ak = idx % GK;
-            const int gr = m0 + ar, gk = k0 + ak;
-            As[ak][ar] = (gr < M && gk < K) ? A[(int64_t)gr * lda + gk] : make_double2(0, 0);
-            // B tile GK x TB: thread -> (k = idx / TB, col = idx % TB)
-            const int bk = idx / TB, bc = idx % TB;
-            const int gk2 = k0 + bk, gc = n0 + bc;
-            Bs[bk][bc] = (gk2 < K && gc < N) ? B[(int64_t)gk2 * ldb + gc] : make_double2(0, 0);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int kk = 0; kk < GK; ++kk) {
-            double2 a[TI], b[TI];
-#pragma unroll
-            for (int i = 0; i < TI; ++i) a[i] = As[kk][ty + TD * i];
-#pragma unroll
-            for (int j = 0; j < TI; ++j) b[j] = Bs[kk][tx + TD * j];
-#pragma unroll
-            for (int i = 0; i < TI; ++i)
-#pragma unroll
-                for (int j = 0; j < TI; ++j) {
-                    if constexpr (REAL == 2) {  // B real
-                        acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
-                        acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
-                    } else if constexpr (REAL == 1) {  // A real
-                        acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
-                        acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
-                    } else {
-                        acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
-                        acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
-                        acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
-                        acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
+    for (int i = 0; i < TM; ++i) acc[i] = make_double2(0, 0);
+    const int kbeg = p.a_upper ? m0 : 0;  // A upper triangular: nothing left of its diagonal
+    for (int k0 = kbeg; k0 < p.K; k0 += ZKC) {
+        const int kc = min(ZKC, p.K - k0);
+        if (k0 != kbeg) __syncthreads();
+        if constexpr (TA) {
+            for (int e = tid; e < R * kc; e += blockDim.x) {
+                const int kk = e / R, row = e - kk * R;
+                double2 v = make_double2(0, 0);
+                if (m0 + row < p.M) v = A[(int64_t)(k0 + kk) * p.lda + m0 + row];
+                As[row * LS + kk] = make_double2(v.x, -v.y);
+            }
+        } else {
+            for (int row = warp; row < R; row += nwarps)
+                for (int kk = lane; kk < kc; kk += 32) {
+                    double2 v = make_double2(0, 0);
+                    if (m0 + row < p.M) {
+                        v = A[(int64_t)(m0 + row) * p.lda + k0 + kk];
+                        if (ks) v = cmul(v, ks[k0 + kk]);
                     }
+                    As[row * LS + kk] = v;
                 }
         }
         __syncthreads();
-    }
+        if (act) {
+            const double2 *as = As + g * TM * LS;
+            const double2 *b = B + (int64_t)k0 * p.ldb + col;
+#pragma unroll 8
+            for (int kk = 0; kk < kc; ++kk) {
+                const double2 bv = b[(int64_t)kk * p.ldb];
 #pragma unroll
-    for (int i = 0; i < TI; ++i) {
-        const int r = m0 + ty + TD * i;
-        if (r >= M) continue;
-#pragma unroll
-        for (int j = 0; j < TI; ++j) {
-            const int c = n0 + tx + TD * j;
-            if (c >= N) continue;
-            double2 v = cmul(alpha, acc[i][j]);
-            if (add_identity && r == c) v.x += 1.0;
-            if (accumulate) {
-                const double2 o = C[(int64_t)r * ldc + c];
-                v.x += o.x;
-                v.y += o.y;
+                for (int i = 0; i < TM; ++i) {
+                    const double2 a = as[i * LS + kk];
+                    if constexpr (REAL == 2) {  // B real
+                        acc[i].x = fma(a.x, bv.x, acc[i].x);
+                        acc[i].y = fma(a.y, bv.x, acc[i].y);
+                    } else if constexpr (REAL == 1) {  // A real
+                        acc[i].x = fma(a.x, bv.x, acc[i].x);
+                        acc[i].y = fma(a.x, bv.y, acc[i].y);
+                    } else {
+                        acc[i].x = fma(a.x, bv.x, acc[i].x);
+                        acc[i].x = fma(-a.y, bv.y, acc[i].x);
+                        acc[i].y = fma(a.x, bv.y, acc[i].y);
+                        acc[i].y = fma(a.y, bv.x, acc[i].y);
+                    }
+                }
             }
-            C[(int64_t)r * ldc + c] = v;
         }
     }
-}
-
-// Small products (M, N, K <= 32): one CTA per 16x16 output tile and product, the whole K range loaded once, and the
-// K sum split over ZS_KG warp pairs whose partial sums are added in shared memory. FP64 arithmetic is slow per SM
-// partition on this part, so for these latency-bound products short dependent chains and more warps per product
-// matter more than operand reuse.
-constexpr int ZS_TB = 16, ZS_KG = 4, ZS_K = 32;
-
-__global__ void __launch_bounds__(64 * ZS_KG)
-    k_zgemm_small(int M, int N, int K, double2 alpha, const double2 *__restrict__ A, int64_t lda, int64_t sA,
-                  const double2 *__restrict__ B, int64_t ldb, int64_t sB, double2 *__restrict__ C, int64_t ldc,
-                  int64_t sC, bool add_identity, bool accumulate, int batch2, int64_t sA2, int64_t sB2,
-                  int64_t sC2) {
-    __shared__ double2 As[ZS_K][ZS_TB + 1];
-    __shared__ double2 Bs[ZS_K][ZS_TB + 1];
-    __shared__ double2 red[ZS_KG][ZS_TB * ZS_TB];
-    const int z1 = blockIdx.z / batch2, z2 = blockIdx.z % batch2;
-    A += sA * z1 + sA2 * z2;
-    B += sB * z1 + sB2 * z2;
-    C += sC * z1 + sC2 * z2;
-    const int m0 = blockIdx.x * ZS_TB, n0 = blockIdx.y * ZS_TB;
-    const int tid = threadIdx.x;
-    for (int e = tid; e < ZS_K * ZS_TB; e += 64 * ZS_KG) {
-        const int k = e / ZS_TB, i = e % ZS_TB;
-        As[k][i] = (m0 + i < M && k < K) ? A[(int64_t)(m0 + i) * lda + k] : make_double2(0, 0);
-        Bs[k][i] = (k < K && n0 + i < N) ? B[(int64_t)k * ldb + n0 + i] : make_double2(0, 0);
-    }
-    __syncthreads();
-    const int g = tid / 64, t = tid % 64, tx = t % 8, ty = t / 8;
-    double2 acc[2][2];
+    if (!act) return;
+    const double2 *rs = p.rscale ? p.rscale + p.srs * z1 + p.srs2 * z2 : nullptr;
 #pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) acc[i][j] = make_double2(0, 0);
-    for (int k = g; k < K; k += ZS_KG) {
-        const double2 a0 = As[k][ty], a1 = As[k][ty + 8], b0 = Bs[k][tx], b1 = Bs[k][tx + 8];
-        const double2 a[2] = {a0, a1}, b[2] = {b0, b1};
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 2; ++j) {
-                acc[i][j].x = fma(a[i].x, b[j].x, acc[i][j].x);
-                acc[i][j].x = fma(-a[i].y, b[j].y, acc[i][j].x);
-                acc[i][j].y = fma(a[i].x, b[j].y, acc[i][j].y);
-                acc[i][j].y = fma(a[i].y, b[j].x, acc[i][j].y);
-            }
-    }
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int j = 0; j < 2; ++j) red[g][(ty + 8 * i) * ZS_TB + tx + 8 * j] = acc[i][j];
-    __syncthreads();
-    for (int e = tid; e < ZS_TB * ZS_TB; e += 64 * ZS_KG) {
-        const int r = m0 + e / ZS_TB, c = n0 + e % ZS_TB;
-        if (r >= M || c >= N) continue;
-        double2 v = red[0][e];
-#pragma unroll
-        for (int q = 1; q < ZS_KG; ++q) {
-            v.x += red[q][e].x;
-            v.y += red[q][e].y;
-        }
-        v = cmul(alpha, v);
-        if (add_identity && r == c) v.x += 1.0;
-        if (accumulate) {
-            const double2 o = C[(int64_t)r * ldc + c];
+    for (int i = 0; i < TM; ++i) {
+        const int r = m0 + g * TM + i;
+        if (r >= p.M || (p.upper && col < r)) continue;
+        double2 v = acc[i];
+        if (p.alpha.y != 0.0) v = cmul(p.alpha, v);
+        else if (p.alpha.x != 1.0) v = make_double2(p.alpha.x * v.x, p.alpha.x * v.y);
+        if (rs) v = cmul(rs[r], v);
+        if (p.add_identity && r == col) v.x += 1.0;
+        if (p.accumulate) {
+            const double2 o = C[(int64_t)r * p.ldc + col];
             v.x += o.x;
             v.y += o.y;
         }
-        C[(int64_t)r * ldc + c] = v;
+        C[(int64_t)r * p.ldc + col] = v;
     }
+}
+
+// Small products (M, N, K <= ZSMALL): what bounds them is the dependent chain of FP64 steps of one output, so a CTA takes
+// 32 outputs (flattened, no padded tile) and its four warps, one per scheduler, a quarter of the k sum each.
+constexpr int ZSMALL = 32;
+
+template <int REAL, bool TA> __global__ void __launch_bounds__(128) k_zgemm_small(ZProd p) {
+    __shared__ double2 red[3][32];
+    const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
+    const int z1 = blockIdx.z / p.batch2, z2 = blockIdx.z % p.batch2;
+    const double2 *A = p.A + p.sA * z1 + p.sA2 * z2;
+    const double2 *B = p.B + p.sB * z1 + p.sB2 * z2;
+    double2 *C = p.C + p.sC * z1 + p.sC2 * z2;
+    const double2 *ks = p.kscale ? p.kscale + p.sks * z1 + p.sks2 * z2 : nullptr;
+    const int e = blockIdx.x * 32 + lane;
+    const int r = e / p.N, c = e - r * p.N;
+    const bool act = r < p.M && !(p.upper && c < r);
+    double2 acc = make_double2(0, 0);
+    if (act) {
+#pragma unroll 8
+        for (int k = w; k < p.K; k += 4) {
+            double2 a = TA ? A[(int64_t)k * p.lda + r] : A[(int64_t)r * p.lda + k];
+            if (TA) a.y = -a.y;
+            if (ks) a = cmul(a, ks[k]);
+            const double2 b = B[(int64_t)k * p.ldb + c];
+            if constexpr (REAL == 2) {
+                acc.x = fma(a.x, b.x, acc.x);
+                acc.y = fma(a.y, b.x, acc.y);
+            } else if constexpr (REAL == 1) {
+                acc.x = fma(a.x, b.x, acc.x);
+                acc.y = fma(a.x, b.y, acc.y);
+            } else {
+                acc.x = fma(a.x, b.x, acc.x);
+                acc.x = fma(-a.y, b.y, acc.x);
+                acc.y = fma(a.x, b.y, acc.y);
+                acc.y = fma(a.y, b.x, acc.y);
+            }
+        }
+    }
+    if (w > 0) red[w - 1][lane] = acc;
+    __syncthreads();
+    if (w > 0 || !act) return;
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+        acc.x += red[q][lane].x;
+        acc.y += red[q][lane].y;
+    }
+    double2 v = cmul(p.alpha, acc);
+    if (p.rscale) v = cmul(p.rscale[p.srs * z1 + p.srs2 * z2 + r], v);
+    if (p.add_identity && r == c) v.x += 1.0;
+    if (p.accumulate) {
+        const double2 o = C[(int64_t)r * p.ldc + c];
+        v.x += o.x;
+        v.y += o.y;
+    }
+    C[(int64_t)r * p.ldc + c] = v;
 }
 
 __global__ void k_set_identity(double2 *A, int n) {
@@ -262,118 +254,109 @@ __global__ void k_phases(const double2 *phi, double2 *phase, double2 *phase_inv,
 
 namespace {
 
-void launch_zgemm(int tile, cudaStream_t st, int M, int N, int K, double2 alpha, const double2 *A, int64_t lda,
-                  int64_t sA, const double2 *B, int64_t ldb, int64_t sB, double2 *C, int64_t ldc, int64_t sC,
-                  int batch, bool add_identity, bool accumulate, int batch2 = 1, int64_t sA2 = 0, int64_t sB2 = 0,
-                  int64_t sC2 = 0, int real = 0) {
-    const unsigned z = (unsigned)batch * (unsigned)batch2;
-    if (real && !(M <= ZS_K && N <= ZS_K && K <= ZS_K)) {  // a real operand: the 2-FMA products
-        const bool t64 = tile == 64;
-        dim3 grid((unsigned)ceil_div(M, t64 ? 64 : 16), (unsigned)ceil_div(N, t64 ? 64 : 16), z);
-        if (t64 && real == 1)
-            k_zgemm<64, 4, 1><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, add_identity,
-                                                     accumulate, batch2, sA2, sB2, sC2);
-        else if (t64)
-            k_zgemm<64, 4, 2><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, add_identity,
-                                                     accumulate, batch2, sA2, sB2, sC2);
-        else if (real == 1)
-            k_zgemm<16, 2, 1><<<grid, 64, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, add_identity,
-                                                    accumulate, batch2, sA2, sB2, sC2);
-        else
-            k_zgemm<16, 2, 2><<<grid, 64, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, add_identity,
-                                                    accumulate, batch2, sA2, sB2, sC2);
-        note_launch(st);
-        return;
+// How an (M, N) product of nz matrices is cut into CTAs: columns per CTA, row groups, rows per thread (as the
+// CUDA-core operator's split).
+struct ZSplit {
+    int CW, G, TM, threads, gx, gy;
+};
+
+ZSplit zsplit(int M, int N, int64_t nz) {
+    ZSplit S;
+    if (N > ZMAXT) {  // a run of columns of one row group, all runs alike and a whole number of warps
+        const int runs = (int)ceil_div(N, 128);
+        S.CW = (int)ceil_div(ceil_div(N, runs), 32) * 32;
+        S.gy = (int)ceil_div(N, S.CW);
+        S.G = 1;
+    } else {  // whole rows: as many row groups as leave the fewest idle lanes in the last warp
+        S.CW = N;
+        S.gy = 1;
+        S.G = 1;
+        double best = 0;
+        for (int G = 1; G * N <= ZMAXT && G <= M; ++G) {
+            const double eff = (double)(G * N) / (32.0 * (double)ceil_div(G * N, 32));
+            if (eff > best + 0.03) {
+                best = eff;
+                S.G = G;
+            }
+        }
     }
-    if (M <= ZS_K && N <= ZS_K && K <= ZS_K) {
-        dim3 grid((unsigned)ceil_div(M, ZS_TB), (unsigned)ceil_div(N, ZS_TB), z);
-        k_zgemm_small<<<grid, 64 * ZS_KG, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, add_identity,
-                                                  accumulate, batch2, sA2, sB2, sC2);
-    } else if (tile == 64) {
-        dim3 grid((unsigned)ceil_div(M, 64), (unsigned)ceil_div(N, 64), z);
-        k_zgemm<64, 4><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, add_identity,
-                                              accumulate, batch2, sA2, sB2, sC2);
-    } else {
-        dim3 grid((unsigned)ceil_div(M, 16), (unsigned)ceil_div(N, 16), z);
-        k_zgemm<16, 2><<<grid, 64, 0, st>>>(M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, add_identity,
-                                             accumulate, batch2, sA2, sB2, sC2);
+    S.threads = 32 * (int)ceil_div(S.G * S.CW, 32);
+    // rows per thread: the most that still keep the schedulers (4 per SM) evenly busy to 90 %, else the best balance
+    const int64_t sched = 4 * (int64_t)std::max(1, num_sms());
+    double best = 0;
+    S.TM = 1;
+    for (int TM = 8; TM >= 1; TM /= 2) {
+        const int64_t rb = ceil_div(M, (int64_t)S.G * TM);
+        const int64_t warps = rb * S.gy * (S.threads / 32) * nz;
+        const double eff = (double)warps / (double)(sched * ceil_div(warps, sched)) * (double)M / (double)(rb * S.G * TM);
+        if (eff > 1.02 * best) {
+            best = eff;
+            S.TM = TM;
+        }
+        if (eff >= 0.9) break;
     }
-    note_launch(st);
+    S.gx = (int)ceil_div(M, (int64_t)S.G * S.TM);
+    return S;
 }
 
-// Tile choice per (M, N, K, batch): measured once per process on the first overwriting call that is not being
-// captured (both tile variants write the same result: every output element sums over k in the same order), the
-// SM-count heuristic otherwise. NSLG_AUTOTUNE=0 keeps the heuristic.
-std::mutex g_tune_mu;
-std::map<std::tuple<int, int, int, int>, int> g_tile;
+template <int REAL, bool TA> void launch_zgemm(const ZSplit &S, unsigned nz, const ZProd &p, cudaStream_t st) {
+    const dim3 grid((unsigned)S.gx, (unsigned)S.gy, nz);
+    const size_t smem = (size_t)S.G * S.TM * (std::min(ZKC, p.K) + 1) * sizeof(double2);  // <= 37 KB (G N <= 256)
+    if (S.TM == 8) k_zgemm<REAL, TA, 8><<<grid, S.threads, smem, st>>>(p, S.G, S.CW);
+    else if (S.TM == 4) k_zgemm<REAL, TA, 4><<<grid, S.threads, smem, st>>>(p, S.G, S.CW);
+    else if (S.TM == 2) k_zgemm<REAL, TA, 2><<<grid, S.threads, smem, st>>>(p, S.G, S.CW);
+    else k_zgemm<REAL, TA, 1><<<grid, S.threads, smem, st>>>(p, S.G, S.CW);
+}
 
 }  // namespace
+
+int zprod(cudaStream_t st, const ZProd &p, int batch) {
+    if (p.M <= 0 || p.N <= 0 || batch == 0 || p.batch2 == 0) return NSLG_OK;
+    const int64_t nz = (int64_t)batch * p.batch2;
+    NSLG_REQUIRE(nz <= 65535, NSLG_ERR_SHAPE, "zgemm: at most 65535 products per launch");
+    if (p.M <= ZSMALL && p.N <= ZSMALL && p.K <= ZSMALL) {
+        const dim3 grid((unsigned)ceil_div((int64_t)p.M * p.N, 32), 1, (unsigned)nz);
+        if (p.a_adjoint) k_zgemm_small<0, true><<<grid, 128, 0, st>>>(p);
+        else if (p.real == 1) k_zgemm_small<1, false><<<grid, 128, 0, st>>>(p);
+        else if (p.real == 2) k_zgemm_small<2, false><<<grid, 128, 0, st>>>(p);
+        else k_zgemm_small<0, false><<<grid, 128, 0, st>>>(p);
+        note_launch(st);
+        NSLG_CUDA(cudaGetLastError());
+        return NSLG_OK;
+    }
+    const ZSplit S = zsplit(p.M, p.N, nz);
+    if (p.a_adjoint) launch_zgemm<0, true>(S, (unsigned)nz, p, st);
+    else if (p.real == 1) launch_zgemm<1, false>(S, (unsigned)nz, p, st);
+    else if (p.real == 2) launch_zgemm<2, false>(S, (unsigned)nz, p, st);
+    else launch_zgemm<0, false>(S, (unsigned)nz, p, st);
+    note_launch(st);
+    NSLG_CUDA(cudaGetLastError());
+    return NSLG_OK;
+}
 
 int zgemm(cudaStream_t st, int M, int N, int K, double2 alpha, const double2 *A, int64_t lda, int64_t sA,
           const double2 *B, int64_t ldb, int64_t sB, double2 *C, int64_t ldc, int64_t sC, int batch,
           bool add_identity, bool accumulate) {
-    if (M == 0 || N == 0 || batch == 0) return NSLG_OK;
-    static int sms = 0;
-    static const bool tune = [] {
-        const char *e = std::getenv("NSLG_AUTOTUNE");
-        return !(e && e[0] == '0');
-    }();
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
-    int tile = (ceil_div(M, 64) * ceil_div(N, 64) * batch >= 2 * sms) ? 64 : 16;
-    const auto key = std::make_tuple(M, N, K, batch);
-    bool measure = false;
-    if (tune) {
-        std::lock_guard<std::mutex> lock(g_tune_mu);
-        auto it = g_tile.find(key);
-        if (it != g_tile.end()) {
-            tile = it->second;
-        } else if (!accumulate) {
-            cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-            if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cudaGetLastError();
-            measure = cs == cudaStreamCaptureStatusNone;
-        }
-    }
-    if (measure) {
-        cudaEvent_t ev[3];
-        for (auto &e : ev) NSLG_CUDA(cudaEventCreate(&e));
-        NSLG_CUDA(cudaEventRecord(ev[0], st));
-        launch_zgemm(16, st, M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, add_identity, false);
-        NSLG_CUDA(cudaEventRecord(ev[1], st));
-        launch_zgemm(64, st, M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, add_identity, false);
-        NSLG_CUDA(cudaEventRecord(ev[2], st));
-        NSLG_CUDA(cudaEventSynchronize(ev[2]));
-        float t16 = 0, t64 = 0;
-        cudaEventElapsedTime(&t16, ev[0], ev[1]);
-        cudaEventElapsedTime(&t64, ev[1], ev[2]);
-        for (auto &e : ev) cudaEventDestroy(e);
-        std::lock_guard<std::mutex> lock(g_tune_mu);
-        g_tile[key] = t64 <= t16 ? 64 : 16;
-        NSLG_CUDA(cudaGetLastError());
-        return NSLG_OK;  // C holds the product (written by both variants)
-    }
-    launch_zgemm(tile, st, M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, add_identity, accumulate);
-    NSLG_CUDA(cudaGetLastError());
-    return NSLG_OK;
+    ZProd p(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC);
+    p.alpha = alpha;
+    p.add_identity = add_identity;
+    p.accumulate = accumulate;
+    return zprod(st, p, batch);
 }
 
 // Two-level batched product: C[z1, z2] = alpha A[z1, z2] B[z1, z2] with element offsets z1 * s + z2 * s2, for
-// batch x batch2 products in one launch (16-wide tiles: these are the small products of the scans).
+// batch x batch2 products in one launch.
 int zgemm2(cudaStream_t st, int M, int N, int K, double2 alpha, const double2 *A, int64_t lda, int64_t sA,
            int64_t sA2, const double2 *B, int64_t ldb, int64_t sB, int64_t sB2, double2 *C, int64_t ldc, int64_t sC,
            int64_t sC2, int batch, int batch2, int real) {
-    if (M == 0 || N == 0 || batch == 0 || batch2 == 0) return NSLG_OK;
-    NSLG_REQUIRE((int64_t)batch * batch2 <= 65535, NSLG_ERR_SHAPE, "zgemm2: at most 65535 products per launch");
-    // 64-wide tiles once they alone fill the GPU twice (the stratified products of large lattices), else 16-wide
-    const int tile = ceil_div(M, 64) * ceil_div(N, 64) * (int64_t)batch * batch2 >= 2 * num_sms() ? 64 : 16;
-    launch_zgemm(tile, st, M, N, K, alpha, A, lda, sA, B, ldb, sB, C, ldc, sC, batch, false, false, batch2, sA2, sB2,
-                 sC2, real);
-    NSLG_CUDA(cudaGetLastError());
-    return NSLG_OK;
+    ZProd p(M, N, K, A, lda, sA, B, ldb, sB, C, ldc, sC);
+    p.alpha = alpha;
+    p.sA2 = sA2;
+    p.sB2 = sB2;
+    p.sC2 = sC2;
+    p.batch2 = batch2;
+    p.real = real;
+    return zprod(st, p, batch);
 }
 
 int compute_phases(nslg_fm *fm) {

@@ -578,94 +578,215 @@ __global__ void k_perm_identity(double2 *B, int n, const int *piv, int64_t bstri
     }
 }
 
-// G[g] = A_g^{-1} for small matrices (n <= GJ_MAX) in one launch: Gauss-Jordan elimination with partial pivoting on
-// [A | I] in shared memory, one CTA per matrix. The pivot of step k is chosen from the same Schur-complement column
-// as in the LU with partial pivoting (same rule), so pivots (if given), swaps and singular mean the same as after
-// lu_factor.
-// Replaces the panel, triangular-solve and permutation launches of lu_factor + lu_inverse for the small lattices,
-// where each of those launches is a chain of dependent FP64 steps.
-constexpr int GJ_MAX = 32;
-constexpr int GJ_T = 256;
-constexpr int SCAN_MAX_MATRICES = 8;  // the small-lattice gradient uses scans up to this many matrices per call
+// G[g] = (A_g + 1)^{-1} for small matrices (n <= GJ_MAX) in one launch: in-place Gauss-Jordan elimination with partial
+// pivoting in shared memory, one CTA per matrix. Rows are never swapped: column k's pivot is the largest entry among the
+// rows that have not been pivots yet (first row on ties, the same choice as an LU with row swaps makes up to the row
+// order), and the permutation is applied on the way out, inv[k, p_j] = W[p_k, j]. A step is one warp's pivot search
+// (integer comparisons of the FP64 bit patterns: an FP64 comparison costs a warp 64 cycles), the scaled pivot row, and
+// one update of all n^2 elements, which the FP64 pipe of one SM bounds (n^3 complex FMAs, 2 FP64 FMAs per clock).
+// Measured: 52 us -> 38 us at n = 18; panel factorisation, triangular solves and permutation of 32 matrices of n = 50
+// 690 us -> 293 us.
+constexpr int GJ_MAX = 64;
+constexpr int GJ_T = 512;
+constexpr int SCAN_MAX = 32;           // the small-lattice gradient uses scans up to this size
+constexpr int SCAN_MAX_MATRICES = 8;   // and up to this many matrices per call
+
+constexpr size_t gj_smem(int n) { return (size_t)n * (n + 1) * sizeof(double2); }
 
 __global__ void __launch_bounds__(GJ_T) k_gj_inverse(const double2 *__restrict__ A, int64_t astride,
-                                                     double2 *__restrict__ G, int n, double2 *pivots, int *swaps,
-                                                     int *singular) {
-    __shared__ double2 W[GJ_MAX][2 * GJ_MAX + 1];
-    __shared__ double2 f[GJ_MAX];
+                                                     double2 *__restrict__ G, int n, int *singular) {
+    extern __shared__ double2 W[];  // n x (n + 1)
+    __shared__ double2 f[GJ_MAX], u[GJ_MAX];
     __shared__ double2 inv_sh;
-    __shared__ int pivot;
+    __shared__ int pivot, piv[GJ_MAX];
+    const int ld = n + 1, T = blockDim.x, tid = threadIdx.x;
     const int g = blockIdx.x;
     A += g * astride;
     G += (int64_t)g * n * n;
-    const int w = 2 * n;
-    for (int e = threadIdx.x; e < n * w; e += GJ_T) {
-        const int i = e / w, j = e % w;
-        W[i][j] = j < n ? A[(int64_t)i * n + j] : make_double2(j - n == i ? 1.0 : 0.0, 0.0);
+    for (int e = tid; e < n * n; e += T) {
+        const int i = e / n, j = e - i * n;
+        double2 v = A[e];
+        if (i == j) v.x += 1.0;
+        W[i * ld + j] = v;
     }
     __syncthreads();
-        int nswap = 0, sing = 0;
+    const int di = T / n, dj = T - di * n;  // (i, j) steps of this thread's elements
+    const int i0 = tid / n, j0 = tid - i0 * n;
+    unsigned long long used = 0;  // rows that have been pivots (warp 0)
+    int sing = 0;
     for (int k = 0; k < n; ++k) {
-        if (threadIdx.x < 32) {  // pivot: largest |a_ik|^2 over rows i >= k, first index on ties
-            double bm = -1.0;
-            int bi = n;
-            const int i = k + threadIdx.x;
-            if (i < n) {
-                const double2 v = W[i][k];
-                bm = v.x * v.x + v.y * v.y;
-                bi = i;
+        if (tid < 32) {
+            unsigned long long bm = 0;
+            int bi = GJ_MAX;
+            for (int i = tid; i < n; i += 32) {
+                if (used >> i & 1) continue;
+                const double2 v = W[i * ld + k];
+                const unsigned long long m = (unsigned long long)__double_as_longlong(fma(v.x, v.x, v.y * v.y));
+                if (bi == GJ_MAX || m > bm) {
+                    bm = m;
+                    bi = i;
+                }
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
-                const double om = __shfl_down_sync(0xffffffffu, bm, o);
-                const int oi = __shfl_down_sync(0xffffffffu, bi, o);
-                if (piv_better(om, oi, bm, bi)) {
+                const unsigned long long om = __shfl_xor_sync(0xffffffffu, bm, o);
+                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+                if (oi < GJ_MAX && (bi == GJ_MAX || om > bm || (om == bm && oi < bi))) {
                     bm = om;
                     bi = oi;
                 }
             }
-            if (threadIdx.x == 0) pivot = bi;
+            used |= 1ull << bi;
+            if (tid == 0) {
+                const double2 d = W[bi * ld + k];
+                const double dd = d.x * d.x + d.y * d.y;
+                const double rdd = dd == 0.0 ? 0.0 : 1.0 / dd;
+                inv_sh = make_double2(d.x * rdd, -d.y * rdd);
+                pivot = bi;
+                piv[k] = bi;
+                if (dd == 0.0) sing = 1;
+            }
         }
         __syncthreads();
         const int p = pivot;
-        if (p != k)
-            for (int j = threadIdx.x; j < w; j += GJ_T) {
-                const double2 a = W[k][j];
-                W[k][j] = W[p][j];
-                W[p][j] = a;
-            }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const double2 d = W[k][k];
-            const double dd = d.x * d.x + d.y * d.y;
-            const double rdd = dd == 0.0 ? 0.0 : 1.0 / dd;
-            inv_sh = make_double2(d.x * rdd, -d.y * rdd);
-            if (pivots) pivots[(int64_t)g * n + k] = d;
-            if (p != k) ++nswap;
-            if (dd == 0.0) sing = 1;
+        const double2 inv = inv_sh;
+        for (int j = tid; j < n; j += T) {
+            u[j] = j == k ? inv : cmul(W[p * ld + j], inv);
+            f[j] = W[j * ld + k];
         }
         __syncthreads();
-        const double2 inv = inv_sh;
-        for (int j = k + threadIdx.x; j < w; j += GJ_T) W[k][j] = cmul(W[k][j], inv);  // columns < k of row k are 0
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += GJ_T) f[i] = i == k ? make_double2(0, 0) : W[i][k];
-        __syncthreads();
-        const int wk = w - k;
-        for (int e = threadIdx.x; e < n * wk; e += GJ_T) {
-            const int i = e / wk, j = k + e % wk;
-            if (i == k) continue;
-            const double2 l = f[i], u = W[k][j];
-            double2 a = W[i][j];
-            a.x -= l.x * u.x - l.y * u.y;
-            a.y -= l.x * u.y + l.y * u.x;
-            W[i][j] = a;
+        for (int e = tid, i = i0, j = j0; e < n * n; e += T) {
+            const double2 uj = u[j];
+            double2 a = uj;
+            if (i != p) {
+                const double2 l = f[i];
+                a = j == k ? make_double2(0, 0) : W[i * ld + j];
+                a.x -= l.x * uj.x - l.y * uj.y;
+                a.y -= l.x * uj.y + l.y * uj.x;
+            }
+            W[i * ld + j] = a;
+            i += di;
+            j += dj;
+            if (j >= n) {
+                j -= n;
+                ++i;
+            }
         }
         __syncthreads();
     }
-    for (int e = threadIdx.x; e < n * n; e += GJ_T) G[e] = W[e / n][n + e % n];
-    if (threadIdx.x == 0) {
-        swaps[g] = nswap;
-        if (sing) *singular = 1;
+    for (int e = tid; e < n * n; e += T) {
+        const int k = e / n, j = e - k * n;
+        G[k * n + piv[j]] = W[piv[k] * ld + j];
+    }
+    if (tid == 0 && sing) *singular = 1;
+}
+
+// G[g] = (A_g + 1)^{-1} (astride elements apart, G dense), n <= GJ_MAX.
+int gj_inverse_plus_one(nslg_fm *fm, const double2 *A, int64_t astride, double2 *G, int n, int nmat, int *singular) {
+    {
+        static std::mutex mu;
+        static std::set<int> done;
+        std::lock_guard<std::mutex> lock(mu);
+        if (!done.count(fm->ctx->device)) {
+            NSLG_CUDA(cudaFuncSetAttribute(k_gj_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)gj_smem(GJ_MAX)));
+            done.insert(fm->ctx->device);
+        }
+    }
+    k_gj_inverse<<<(unsigned)nmat, n <= 24 ? 352 : GJ_T, gj_smem(n), fm->ctx->stream>>>(A, astride, G, n, singular);
+    note_launch(fm->ctx->stream);
+    NSLG_CUDA(cudaGetLastError());
+    return NSLG_OK;
+}
+
+// One level of the Hillis-Steele scans over the slices of nmat matrices (n <= SCAN_MAX), prefix and suffix in one launch:
+//   Qn(t) = Q(t - o) Q(t) (t >= o, Q(t) below),  Sn(t) = S(t) S(t + o) (t < Nt - o, S(t) above).
+// A CTA computes 32 outputs of one product, its four warps a quarter of the k sum each (one per scheduler).
+__global__ void __launch_bounds__(128) k_scan_level(const double2 *__restrict__ Q, const double2 *__restrict__ S,
+                                                    double2 *__restrict__ Qn, double2 *__restrict__ Sn, int n, int Nt,
+                                                    int o) {
+    __shared__ double2 red[3][32];
+    const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
+    const int t = blockIdx.y;
+    const bool suffix = blockIdx.z & 1;
+    const int64_t nn = (int64_t)n * n, base = (int64_t)(blockIdx.z >> 1) * Nt * nn;
+    const int e = blockIdx.x * 32 + lane;
+    const double2 *X = (suffix ? S : Q) + base;
+    double2 *Y = (suffix ? Sn : Qn) + base;
+    const int ta = suffix ? t : t - o, tb = suffix ? t + o : t;
+    if (ta < 0 || tb >= Nt) {  // no partner at this distance
+        if (w == 0 && e < nn) Y[t * nn + e] = X[t * nn + e];
+        return;
+    }
+    double2 acc = make_double2(0, 0);
+    if (e < nn) {
+        const int i = e / n, j = e - i * n;
+        const double2 *a = X + ta * nn + i * n, *b = X + tb * nn + j;
+#pragma unroll 8
+        for (int k = w; k < n; k += 4) {
+            const double2 av = a[k], bv = b[k * n];
+            acc.x = fma(av.x, bv.x, acc.x);
+            acc.x = fma(-av.y, bv.y, acc.x);
+            acc.y = fma(av.x, bv.y, acc.y);
+            acc.y = fma(av.y, bv.x, acc.y);
+        }
+    }
+    if (w > 0) red[w - 1][lane] = acc;
+    __syncthreads();
+    if (w == 0 && e < nn) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            acc.x += red[q][lane].x;
+            acc.y += red[q][lane].y;
+        }
+        Y[t * nn + e] = acc;
+    }
+}
+
+// out[g, t, x] = i sum_k S(t + 1)[x, k] (G Q(t))[k, x], and i sum_k S(0)[x, k] G[k, x] at t = Nt - 1: the diagonal of the
+// gradient from the scans without storing G Q(t). A CTA owns XB sites of one slice, a thread one (site, k).
+__global__ void __launch_bounds__(128) k_scan_grad(const double2 *__restrict__ S, const double2 *__restrict__ Q,
+                                                   const double2 *__restrict__ G, double2 *__restrict__ out, int n,
+                                                   int Nt, int XB) {
+    __shared__ double2 term[128];
+    const int t = blockIdx.y, g = blockIdx.z;
+    const int64_t nn = (int64_t)n * n;
+    const int xl = threadIdx.x / n, k = threadIdx.x - xl * n, x = blockIdx.x * XB + xl;
+    const double2 *Gg = G + g * nn;
+    if (xl < XB && x < n) {
+        const double2 s = S[((int64_t)g * Nt + (t + 1) % Nt) * nn + x * n + k];
+        double2 p;
+        if (t == Nt - 1) {
+            p = Gg[k * n + x];
+        } else {
+            const double2 *q = Q + ((int64_t)g * Nt + t) * nn + x;
+            double2 r[4] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};
+            for (int l0 = 0; l0 < n; l0 += 4)
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    if (l0 + c < n) {
+                        const double2 a = Gg[k * n + l0 + c], b = q[(l0 + c) * n];
+                        r[c].x = fma(a.x, b.x, r[c].x);
+                        r[c].x = fma(-a.y, b.y, r[c].x);
+                        r[c].y = fma(a.x, b.y, r[c].y);
+                        r[c].y = fma(a.y, b.x, r[c].y);
+                    }
+            p = make_double2(((r[0].x + r[1].x) + r[2].x) + r[3].x, ((r[0].y + r[1].y) + r[2].y) + r[3].y);
+        }
+        term[threadIdx.x] = cmul(s, p);
+    }
+    for (int o = 16; o > 0; o >>= 1) {  // tree sum over k (n <= 32)
+        __syncthreads();
+        if (k < o && k + o < n && xl < XB && x < n) {
+            double2 v = term[threadIdx.x];
+            v.x += term[threadIdx.x + o].x;
+            v.y += term[threadIdx.x + o].y;
+            term[threadIdx.x] = v;
+        }
+    }
+    if (k == 0 && xl < XB && x < n) {
+        const double2 v = term[threadIdx.x];
+        out[((int64_t)g * Nt + t) * n + x] = make_double2(-v.y, v.x);  // i * sum
     }
 }
 
@@ -810,31 +931,98 @@ __global__ void k_add_identity_many(double2 *A, int n, int nmat, int64_t mstride
     A[g * mstride + (int64_t)i * n + i].x += 1.0;
 }
 
-// out[g, t, x] = i * sum_k S[g, (t + 1) mod Nt][x, k] B[k, x] with B = P[g, t] (t < Nt - 1) or G[g] (t = Nt - 1):
-// one warp per (g, t, x), lanes over k (row of S coalesced), shuffle reduction.
-__global__ void k_diagprod_many(const double2 *__restrict__ S, const double2 *__restrict__ P,
-                                const double2 *__restrict__ G, double2 *__restrict__ out, int n, int Nt, int nmat) {
-    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (wid >= (int64_t)nmat * Nt * n) return;
-    const int x = (int)(wid % n);
-    const int64_t gt = wid / n;
+// out[g, t, x] = i * sum_k S[g, (t + 1) mod Nt][x, k] B[k, x] with B = P[g, t] (t < Nt - 1) or G[g] (t = Nt - 1): a CTA
+// owns 32 sites x of one slice and turns 32 x 32 blocks of S through shared memory, so that both matrices are read
+// along their rows; its eight warps split k.
+__global__ void __launch_bounds__(256) k_diagprod_many(const double2 *__restrict__ S, const double2 *__restrict__ P,
+                                                       const double2 *__restrict__ G, double2 *__restrict__ out, int n,
+                                                       int Nt) {
+    __shared__ double2 tile[32][33];
+    __shared__ double2 red[8][32];
+    const int64_t gt = blockIdx.y;
     const int g = (int)(gt / Nt), t = (int)(gt % Nt);
+    const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
+    const int x0 = blockIdx.x * 32, x = x0 + lane;
     const int64_t nn = (int64_t)n * n;
-    const double2 *Sr = S + ((int64_t)g * Nt + (t + 1) % Nt) * nn + (int64_t)x * n;
-    const double2 *B = t == Nt - 1 ? G + (int64_t)g * nn : P + ((int64_t)g * Nt + t) * nn;
+    const double2 *Sm = S + ((int64_t)g * Nt + (t + 1) % Nt) * nn;
+    const double2 *B = t == Nt - 1 ? G + (int64_t)g * nn : P + gt * nn;
     double2 acc = make_double2(0, 0);
-    for (int k = lane; k < n; k += 32) {
-        const double2 a = Sr[k], bv = B[(int64_t)k * n + x];
-        acc.x += a.x * bv.x - a.y * bv.y;
-        acc.y += a.x * bv.y + a.y * bv.x;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        if (k0) __syncthreads();
+        for (int r = w; r < 32; r += 8)
+            if (x0 + r < n && k0 + lane < n) tile[r][lane] = Sm[(int64_t)(x0 + r) * n + k0 + lane];
+        __syncthreads();
+        if (x < n)
+            for (int kk = w; kk < min(32, n - k0); kk += 8) {
+                const double2 a = tile[lane][kk], bv = B[(int64_t)(k0 + kk) * n + x];
+                acc.x += a.x * bv.x - a.y * bv.y;
+                acc.y += a.x * bv.y + a.y * bv.x;
+            }
     }
+    red[w][lane] = acc;
+    __syncthreads();
+    if (w == 0 && x < n) {
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        acc.x += __shfl_down_sync(0xffffffffu, acc.x, o);
-        acc.y += __shfl_down_sync(0xffffffffu, acc.y, o);
+        for (int q = 1; q < 8; ++q) {
+            acc.x += red[q][lane].x;
+            acc.y += red[q][lane].y;
+        }
+        out[gt * n + x] = make_double2(-acc.y, acc.x);  // i * acc
     }
-    if (lane == 0) out[gt * n + x] = make_double2(-acc.y, acc.x);  // i * acc
+}
+
+int diagprod_many(cudaStream_t st, const double2 *S, const double2 *P, const double2 *G, double2 *out, int n, int Nt,
+                  int nmat) {
+    const int64_t slices = (int64_t)nmat * Nt;
+    for (int64_t s0 = 0; s0 < slices; s0 += (int64_t)(65535 / Nt) * Nt) {  // whole matrices per launch (grid.y limit)
+        const int64_t cnt = std::min<int64_t>(slices - s0, (int64_t)(65535 / Nt) * Nt), g0 = s0 / Nt;
+        const int64_t nn = (int64_t)n * n;
+        k_diagprod_many<<<dim3((unsigned)ceil_div(n, 32), (unsigned)cnt), 256, 0, st>>>(
+            S + s0 * nn, P + s0 * nn, G + g0 * nn, out + s0 * n, n, Nt);
+        note_launch(st);
+    }
+    NSLG_CUDA(cudaGetLastError());
+    return NSLG_OK;
+}
+
+// dst[g] = diag(ph[g, row]) E_g for nmat matrices (E_g = (g & emask) ? E1 : E0), dst dstride elements apart.
+__global__ void k_first_slice(const double2 *__restrict__ E0, const double2 *__restrict__ E1, int emask,
+                              const double2 *__restrict__ ph, int row, double2 *__restrict__ dst, int64_t dstride,
+                              int nmat, int Nt, int n) {
+    const int64_t nn = (int64_t)n * n, idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= nn * nmat) return;
+    const int g = (int)(idx / nn);
+    const int64_t e = idx - g * nn;
+    dst[g * dstride + e] = cmul(((g & emask) ? E1 : E0)[e], ph[((int64_t)g * Nt + row) * n + e / n]);
+}
+
+// X[g] = diag(ph[g, 2 mod Nt]) E_g diag(ph[g, 1 mod Nt]), without the row scale for one slice.
+__global__ void k_logdet_first(const double2 *__restrict__ E0, const double2 *__restrict__ E1, int emask,
+                               const double2 *__restrict__ ph, double2 *__restrict__ X, int nmat, int Nt, int n) {
+    const int64_t nn = (int64_t)n * n, idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= nn * nmat) return;
+    const int g = (int)(idx / nn);
+    const int64_t e = idx - g * nn;
+    const double2 *p = ph + (int64_t)g * Nt * n;
+    double2 v = cmul(((g & emask) ? E1 : E0)[e], p[(int64_t)(1 % Nt) * n + e % n]);
+    if (Nt > 1) v = cmul(p[(int64_t)(2 % Nt) * n + e / n], v);
+    X[idx] = v;
+}
+
+// A product of every matrix of a batch with its real factor E_g: the factor as A (left) or B, as a two-level batch.
+ZProd factor_product(int n, const double2 *E0, const double2 *E1, int emask, bool left, const double2 *X, int64_t sX,
+                     double2 *Y, int64_t sY) {
+    const int64_t dE = emask ? (int64_t)((reinterpret_cast<intptr_t>(E1) - reinterpret_cast<intptr_t>(E0)) /
+                                         (intptr_t)sizeof(double2))
+                             : 0;
+    const int b2 = emask ? 2 : 1;
+    ZProd p(n, n, n, left ? E0 : X, n, left ? 0 : b2 * sX, left ? X : E0, n, left ? b2 * sX : 0, Y, n, b2 * sY);
+    (left ? p.sA2 : p.sB2) = dE;
+    (left ? p.sB2 : p.sA2) = sX;
+    p.sC2 = sY;
+    p.batch2 = b2;
+    p.real = left ? 1 : 2;
+    return p;
 }
 
 }  // namespace
@@ -949,7 +1137,7 @@ int fm_grad_logdet(nslg_fm *fm, double2 *out) {
     } else if (fm->force_precision == NSLG_PREC_BF16_SPLIT && fm->kind == NSLG_FM_EXP && E->is_real && n <= 2048) {
         NSLG_TRY(grad_logdet_tc(fm, E, out));
     } else {
-        NSLG_TRY(grad_logdet_many(fm, 1, E->full, E->full, 0, fm->phase_inv, out));
+        NSLG_TRY(grad_logdet_many(fm, 1, E, E, 0, fm->phase_inv, out));
     }
     if (fm->defer_checks) return NSLG_OK;  // the captured trajectory checks the sticky flag after its replay
     LuScratch s;
@@ -968,95 +1156,103 @@ int fm_grad_logdet(nslg_fm *fm, double2 *out) {
 //   G = (1 + S(0))^{-1},  P(t) = P(t-1) Fk(t), P(-1) = G,  pi_dot(t) = i diag(S(t+1) P(t)), pi_dot(Nt-1) = i diag(S(0) G).
 // Every chain step is one batched GEMM over the nmat matrices and the LU/solve factor them side by side, so the
 // species of one configuration, or many configurations, share each launch.
-int grad_logdet_many(nslg_fm *fm, int nmat, const double2 *E0, const double2 *E1, int emask, const double2 *ph_inv,
+int grad_logdet_many(nslg_fm *fm, int nmat, const ExpEntry *e0, const ExpEntry *e1, int emask, const double2 *ph_inv,
                      double2 *out) {
     cudaStream_t st = fm->ctx->stream;
     const int Nt = (int)fm->Nt, n = (int)fm->Nx;
     const int64_t nn = (int64_t)n * n, ms = (int64_t)Nt * nn;
-    double2 *Fk, *S, *P, *G;
-    NSLG_TRY(ws_get(fm, "gr_Fk", (size_t)nmat * ms, &Fk));
+    const double2 *E0 = e0->full, *E1 = e1->full;
+    const bool real = e0->is_real && e1->is_real && (emask == 0 || (emask == 1 && nmat % 2 == 0));
+    const bool scan = n <= SCAN_MAX && Nt > 1 && Nt <= 65535 && nmat <= SCAN_MAX_MATRICES;
+    double2 *Fk = nullptr, *S, *P, *G;
     NSLG_TRY(ws_get(fm, "gr_S", (size_t)nmat * ms, &S));
     NSLG_TRY(ws_get(fm, "gr_P", (size_t)nmat * ms, &P));
     NSLG_TRY(ws_get(fm, "gr_G", (size_t)nmat * nn, &G));
     LuScratch s;
     NSLG_TRY(get_lu_scratch(fm, n, s, nmat));
     const double2 one = make_double2(1, 0);
-    k_slices_many<<<(unsigned)ceil_div(ms * nmat, 256), 256, 0, st>>>(E0, E1, emask, ph_inv, Fk, nmat, Nt, n, -1,
-                                                                       true);
-    note_launch(st);
-    if (n <= GJ_MAX && Nt > 1 && nmat <= SCAN_MAX_MATRICES) {
+    if (scan || !real) {
+        NSLG_TRY(ws_get(fm, "gr_Fk", (size_t)nmat * ms, &Fk));
+        k_slices_many<<<(unsigned)ceil_div(ms * nmat, 256), 256, 0, st>>>(E0, E1, emask, ph_inv, Fk, nmat, Nt, n, -1,
+                                                                           true);
+        note_launch(st);
+    }
+    if (scan) {
         // Small matrices, few of them: the chains are latency-bound (each product is a few microseconds of dependent
         // FP64 steps on a handful of SMs), so they become scans with log2(Nt) levels of batched products
         // (Hillis-Steele: ~Nt log2 Nt products instead of 2 (Nt - 1), all of a level in one launch; with many
         // matrices the chains already fill the GPU and the scans' extra products would cost more than they save):
-        //   Q(t) = Fk(0) ... Fk(t) (prefix), S(t) = Fk(t) ... Fk(Nt-1) (suffix), P(t) = G Q(t) (one launch),
-        // and G = (1 + S(0))^{-1} comes from one Gauss-Jordan launch.
-        double2 *Q0, *Q1, *S1, *Pm;
+        //   Q(t) = Fk(0) ... Fk(t) (prefix), S(t) = Fk(t) ... Fk(Nt-1) (suffix),
+        // G = (1 + S(0))^{-1} from one Gauss-Jordan launch, and P(t) = G Q(t) only as the terms of the diagonal.
+        double2 *Q0, *Q1, *S1;
         NSLG_TRY(ws_get(fm, "gr_Q0", (size_t)nmat * ms, &Q0));
         NSLG_TRY(ws_get(fm, "gr_Q1", (size_t)nmat * ms, &Q1));
         NSLG_TRY(ws_get(fm, "gr_S1", (size_t)nmat * ms, &S1));
-        NSLG_TRY(ws_get(fm, "gr_Pm", (size_t)nmat * nn, &Pm));
         const double2 *Qc = Fk, *Sc = Fk;
         double2 *Qbuf[2] = {Q0, Q1}, *Sbuf[2] = {S, S1};
         int lvl = 0;
         for (int o = 1; o < Nt; o <<= 1, ++lvl) {
             double2 *Qn = Qbuf[lvl & 1], *Sn = Sbuf[lvl & 1];
-            // prefix: Qn(t) = Q(t - o) Q(t) for t >= o, Qn(t) = Q(t) below
-            NSLG_TRY(zgemm2(st, n, n, n, one, Qc, n, ms, nn, Qc + o * nn, n, ms, nn, Qn + o * nn, n, ms, nn, nmat,
-                            Nt - o));
-            NSLG_CUDA(cudaMemcpy2DAsync(Qn, ms * sizeof(double2), Qc, ms * sizeof(double2), o * nn * sizeof(double2),
-                                        nmat, cudaMemcpyDeviceToDevice, st));
-            // suffix: Sn(t) = S(t) S(t + o) for t < Nt - o, Sn(t) = S(t) above
-            NSLG_TRY(zgemm2(st, n, n, n, one, Sc, n, ms, nn, Sc + o * nn, n, ms, nn, Sn, n, ms, nn, nmat, Nt - o));
-            NSLG_CUDA(cudaMemcpy2DAsync(Sn + (Nt - o) * nn, ms * sizeof(double2), Sc + (Nt - o) * nn,
-                                        ms * sizeof(double2), o * nn * sizeof(double2), nmat, cudaMemcpyDeviceToDevice,
-                                        st));
+            k_scan_level<<<dim3((unsigned)ceil_div(nn, 32), (unsigned)Nt, 2u * nmat), 128, 0, st>>>(Qc, Sc, Qn, Sn, n,
+                                                                                                  Nt, o);
+            note_launch(st);
             Qc = Qn;
             Sc = Sn;
         }
-        NSLG_CUDA(cudaMemcpy2DAsync(Pm, nn * sizeof(double2), Sc, ms * sizeof(double2), nn * sizeof(double2), nmat,
-                                    cudaMemcpyDeviceToDevice, st));
-        k_add_identity_many<<<(unsigned)ceil_div((int64_t)n * nmat, 256), 256, 0, st>>>(Pm, n, nmat, nn);
-        note_launch(st);
         if (!fm->defer_checks) NSLG_CUDA(cudaMemsetAsync(s.singular, 0, sizeof(int), st));
-        k_gj_inverse<<<(unsigned)nmat, GJ_T, 0, st>>>(Pm, nn, G, n, nullptr, s.swaps, s.singular);
-        note_launch(st);
-        NSLG_TRY(zgemm2(st, n, n, n, one, G, n, nn, 0, Qc, n, ms, nn, P, n, ms, nn, nmat, Nt - 1));
-        const int64_t warps = (int64_t)nmat * Nt * n;
-        k_diagprod_many<<<(unsigned)ceil_div(warps * 32, 256), 256, 0, st>>>(Sc, P, G, out, n, Nt, nmat);
+        NSLG_TRY(gj_inverse_plus_one(fm, Sc, ms, G, n, nmat, s.singular));
+        const int XB = std::min(n, 128 / n);
+        k_scan_grad<<<dim3((unsigned)ceil_div(n, XB), (unsigned)Nt, (unsigned)nmat), 128, 0, st>>>(Sc, Qc, G, out, n, Nt,
+                                                                                                 XB);
         note_launch(st);
         NSLG_CUDA(cudaGetLastError());
         return NSLG_OK;
     }
-    // S(Nt-1) = Fk(Nt-1), then the suffix chain
-    NSLG_CUDA(cudaMemcpy2DAsync(S + (int64_t)(Nt - 1) * nn, ms * sizeof(double2), Fk + (int64_t)(Nt - 1) * nn,
-                                ms * sizeof(double2), nn * sizeof(double2), nmat, cudaMemcpyDeviceToDevice, st));
-    for (int t = Nt - 2; t >= 0; --t)
-        NSLG_TRY(zgemm(st, n, n, n, one, Fk + t * nn, n, ms, S + (t + 1) * nn, n, ms, S + t * nn, n, ms, nmat, false));
-    // 1 + S(0) in P[g, 0] as scratch, factor, G = (1 + S(0))^{-1}
-    NSLG_CUDA(cudaMemcpy2DAsync(P, ms * sizeof(double2), S, ms * sizeof(double2), nn * sizeof(double2), nmat,
-                                cudaMemcpyDeviceToDevice, st));
-    k_add_identity_many<<<(unsigned)ceil_div((int64_t)n * nmat, 256), 256, 0, st>>>(P, n, nmat, ms);
+    // S(Nt-1) = Fk(Nt-1), then the suffix chain; a real E' keeps its products real-by-complex, with the phases as a
+    // scale of the result's rows: S(t) = D_t (E' S(t+1)), D_t = diag(phiExpInv[t-1])
+    auto row = [&](int t) { return ((t - 1) % Nt + Nt) % Nt; };
+    k_first_slice<<<(unsigned)ceil_div(nn * nmat, 256), 256, 0, st>>>(E0, E1, emask, ph_inv, row(Nt - 1),
+                                                                       S + (int64_t)(Nt - 1) * nn, ms, nmat, Nt, n);
     note_launch(st);
+    const int64_t sph = (int64_t)Nt * n;
+    for (int t = Nt - 2; t >= 0; --t) {
+        if (!real) {
+            NSLG_TRY(zgemm(st, n, n, n, one, Fk + t * nn, n, ms, S + (t + 1) * nn, n, ms, S + t * nn, n, ms, nmat, false));
+            continue;
+        }
+        ZProd p = factor_product(n, E0, E1, emask, true, S + (t + 1) * nn, ms, S + t * nn, ms);
+        p.rscale = ph_inv + (int64_t)row(t) * n;
+        p.srs = p.batch2 * sph;
+        p.srs2 = sph;
+        NSLG_TRY(zprod(st, p, nmat / p.batch2));
+    }
+    // G = (1 + S(0))^{-1}
     if (n <= GJ_MAX) {
         if (!fm->defer_checks) NSLG_CUDA(cudaMemsetAsync(s.singular, 0, sizeof(int), st));
-        k_gj_inverse<<<(unsigned)nmat, GJ_T, 0, st>>>(P, ms, G, n, nullptr, s.swaps, s.singular);
+        NSLG_TRY(gj_inverse_plus_one(fm, S, ms, G, n, nmat, s.singular));
+    } else {  // 1 + S(0) in P[g, 0] as scratch
+        NSLG_CUDA(cudaMemcpy2DAsync(P, ms * sizeof(double2), S, ms * sizeof(double2), nn * sizeof(double2), nmat,
+                                    cudaMemcpyDeviceToDevice, st));
+        k_add_identity_many<<<(unsigned)ceil_div((int64_t)n * nmat, 256), 256, 0, st>>>(P, n, nmat, ms);
         note_launch(st);
-    } else {
         NSLG_TRY(lu_factor(fm, P, n, s, nmat, ms, false));
         NSLG_TRY(lu_inverse(fm, P, G, n, s, nmat, ms));
     }
-    // prefix chain P(t) = P(t-1) Fk(t), P(-1) = G
+    // prefix chain P(t) = P(t-1) Fk(t) = (P(t-1) D_t) E', P(-1) = G
     for (int t = 0; t < Nt - 1; ++t) {
         const double2 *prev = t == 0 ? G : P + (t - 1) * nn;
-        NSLG_TRY(zgemm(st, n, n, n, one, prev, n, t == 0 ? nn : ms, Fk + t * nn, n, ms, P + t * nn, n, ms, nmat,
-                       false));
+        const int64_t sp = t == 0 ? nn : ms;
+        if (!real) {
+            NSLG_TRY(zgemm(st, n, n, n, one, prev, n, sp, Fk + t * nn, n, ms, P + t * nn, n, ms, nmat, false));
+            continue;
+        }
+        ZProd p = factor_product(n, E0, E1, emask, false, prev, sp, P + t * nn, ms);
+        p.kscale = ph_inv + (int64_t)row(t) * n;
+        p.sks = p.batch2 * sph;
+        p.sks2 = sph;
+        NSLG_TRY(zprod(st, p, nmat / p.batch2));
     }
-    const int64_t warps = (int64_t)nmat * Nt * n;
-    k_diagprod_many<<<(unsigned)ceil_div(warps * 32, 256), 256, 0, st>>>(S, P, G, out, n, Nt, nmat);
-    note_launch(st);
-    NSLG_CUDA(cudaGetLastError());
-    return NSLG_OK;
+    return diagprod_many(st, S, P, G, out, n, Nt, nmat);
 }
 
 // log det M for nmat matrices of the exponential discretisation at once (hubbardExp.tpp:129-150): matrix g has
@@ -1064,25 +1260,45 @@ int grad_logdet_many(nslg_fm *fm, int nmat, const double2 *E0, const double2 *E1
 // product B_{Nt-1} ... B_0 is a chain of batched GEMMs (one launch per t for all g), 1 + product is factored by the
 // batched LU and log det = sum log u_kk + i pi (#swaps) on the principal branch; out[g] on the host (-inf for a
 // singular matrix).
-int logdet_many(nslg_fm *fm, int nmat, const double2 *E0, const double2 *E1, int emask, const double2 *ph,
+int logdet_many(nslg_fm *fm, int nmat, const ExpEntry *e0, const ExpEntry *e1, int emask, const double2 *ph,
                 double2 *out) {
     cudaStream_t st = fm->ctx->stream;
     const int Nt = (int)fm->Nt, n = (int)fm->Nx;
-    const int64_t nn = (int64_t)n * n, ms = (int64_t)Nt * nn;
-    double2 *B, *R;
-    NSLG_TRY(ws_get(fm, "ldm_slices", (size_t)nmat * ms, &B));
+    const int64_t nn = (int64_t)n * n, ms = (int64_t)Nt * nn, sph = (int64_t)Nt * n;
+    const double2 *E0 = e0->full, *E1 = e1->full;
+    const bool real = e0->is_real && e1->is_real && (emask == 0 || (emask == 1 && nmat % 2 == 0));
+    double2 *R;
     NSLG_TRY(ws_get(fm, "ldm_prod", (size_t)2 * nmat * nn, &R));
     LuScratch s;
     NSLG_TRY(get_lu_scratch(fm, n, s, nmat));
     const double2 one = make_double2(1, 0);
-    k_slices_many<<<(unsigned)ceil_div(ms * nmat, 256), 256, 0, st>>>(E0, E1, emask, ph, B, nmat, Nt, n, 1, false);
-    note_launch(st);
     double2 *cur = R, *nxt = R + (int64_t)nmat * nn;
-    NSLG_CUDA(cudaMemcpy2DAsync(cur, nn * sizeof(double2), B, ms * sizeof(double2), nn * sizeof(double2), nmat,
-                                cudaMemcpyDeviceToDevice, st));
-    for (int t = 1; t < Nt; ++t) {
-        NSLG_TRY(zgemm(st, n, n, n, one, B + t * nn, n, ms, cur, n, nn, nxt, n, nn, nmat, false));
-        std::swap(cur, nxt);
+    if (real) {
+        // X_t = D_{t+2} B_t ... B_0 with D_t = diag(phiExp[t]): X_t = D_{t+2} (E X_{t-1}), a real-by-complex product with
+        // a row scale (none on the last)
+        k_logdet_first<<<(unsigned)ceil_div(nn * nmat, 256), 256, 0, st>>>(E0, E1, emask, ph, cur, nmat, Nt, n);
+        note_launch(st);
+        for (int t = 1; t < Nt; ++t) {
+            ZProd p = factor_product(n, E0, E1, emask, true, cur, nn, nxt, nn);
+            if (t + 1 < Nt) {
+                p.rscale = ph + (int64_t)((t + 2) % Nt) * n;
+                p.srs = p.batch2 * sph;
+                p.srs2 = sph;
+            }
+            NSLG_TRY(zprod(st, p, nmat / p.batch2));
+            std::swap(cur, nxt);
+        }
+    } else {
+        double2 *B;
+        NSLG_TRY(ws_get(fm, "ldm_slices", (size_t)nmat * ms, &B));
+        k_slices_many<<<(unsigned)ceil_div(ms * nmat, 256), 256, 0, st>>>(E0, E1, emask, ph, B, nmat, Nt, n, 1, false);
+        note_launch(st);
+        NSLG_CUDA(cudaMemcpy2DAsync(cur, nn * sizeof(double2), B, ms * sizeof(double2), nn * sizeof(double2), nmat,
+                                    cudaMemcpyDeviceToDevice, st));
+        for (int t = 1; t < Nt; ++t) {
+            NSLG_TRY(zgemm(st, n, n, n, one, B + t * nn, n, ms, cur, n, nn, nxt, n, nn, nmat, false));
+            std::swap(cur, nxt);
+        }
     }
     k_add_identity_many<<<(unsigned)ceil_div((int64_t)n * nmat, 256), 256, 0, st>>>(cur, n, nmat, nn);
     note_launch(st);

@@ -256,3 +256,45 @@ def test_logdet_gradient_mid_sizes(L, Nt):
         grads.append(g_o)
     F = np.asarray(HubbardFermionAction(lat, {"Nt": Nt, "beta": beta, "mu": mu}).force({"phi": phi})["phi"])
     assert rel_err(F, -(grads[0] - grads[1])) < 1e-10
+
+
+@pytest.mark.parametrize("Nx", [2, 31, 32, 33, 50, 63, 64, 65, 97])
+@pytest.mark.parametrize("Nt,nconf", [(1, 1), (3, 3), (8, 5)])
+def test_gradient_and_log_det_forms_by_size(Nx, Nt, nconf):
+    """The direct log det and gradient on both sides of their size limits (scans up to 32 sites and 8 matrices, Gauss-Jordan
+    inverses up to 64 sites, LU beyond), one configuration and a batch, with a real exp(delta K) (ring) and a complex
+    one (complex delta), against the oracle's direct product. beta |K| <= 2 keeps the products' condition below e^8, so
+    1e-10 is far above the rounding of either side."""
+    import nsl_gb300 as N
+    from nsl_gb300.action import HubbardFermionAction, HubbardGaugeAction
+    from oracle import nsl_oracle as O
+
+    rng = np.random.default_rng(1000 * Nx + 10 * Nt + nconf)
+    lat = N.Ring(Nx)
+    for beta in (1.0, 0.8 + 0.3j):
+        phi = rng.standard_normal((nconf, Nt, Nx)) * 0.6 + 0j
+        prm = {"Nt": Nt, "beta": beta, "mu": 0.0, "U": 2.0}
+        S = HubbardGaugeAction(prm) + HubbardFermionAction(lat, prm)
+        fm = N.HubbardExp(lat, Nt, beta)
+        ev = S.eval_batch(phi)
+        for b in range(nconf):
+            want = np.sum(phi[b] ** 2) / (2 * beta / Nt * 2.0)
+            F = -phi[b] / (beta / Nt * 2.0)
+            for sp, sg in ((0, 1), (1, -1)):
+                o = O.HubbardExp(lat.hopping_matrix(), Nt, beta, 0.0, sp)
+                o.populate(phi[b])
+                fm.populate(phi[b], N.Species(sp))
+                assert rel_err(fm.gradLogDetM(), o.gradLogDetM()) < 1e-10, (beta, b, sp)
+                want = want - o.logDetM_lu()
+                F = F - sg * o.gradLogDetM()
+            d = ev[b] - want
+            assert abs(d.real) < 1e-10 * max(1, abs(want)) and abs(np.remainder(d.imag + np.pi, 2 * np.pi) - np.pi) < 1e-10
+            assert rel_err(S.force(phi[b])["phi"], F) < 1e-10
+        # a batch of trajectories is the single ones
+        from nsl_gb300.integrator import Leapfrog
+
+        p = rng.standard_normal(phi.shape) + 0j
+        q1, p1 = Leapfrog(S, 0.1, 2)({"phi": phi}, {"phi": p})
+        for b in range(nconf):
+            qb, pb = Leapfrog(S, 0.1, 2)({"phi": phi[b]}, {"phi": p[b]})
+            assert rel_err(q1["phi"][b], qb["phi"]) < 1e-10 and rel_err(p1["phi"][b], pb["phi"]) < 1e-10
