@@ -240,16 +240,16 @@ struct LuScratch {
 // Scratch of a batch of nmat LU factorisations of size n; `tag` names an independent set (two factorisations whose
 // pivots are both needed later take different tags).
 int get_lu_scratch(nslg_fm *fm, int n, LuScratch &s, int nmat = 1, const char *tag = nullptr);
-// Right-looking blocked LU of nmat matrices at A + g * mstride (mstride 0: n * n), in place. With pivoting: partial
-// pivoting (largest modulus, first index on ties); without: the diagonal is the pivot (Hermitian positive definite
-// matrices, where it is the Cholesky factorisation with U = diag(U) L^H).
+// Right-looking blocked LU of nmat matrices at A + g * mstride (mstride 0: n * n), in place, with partial pivoting
+// (largest modulus, first index on ties).
 int lu_factor(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat = 1, int64_t mstride = 0,
-              bool want_logsum = true, bool pivoting = true);
+              bool want_logsum = true);
 // G[g] = A_g^{-1} from the factors (G dense (nmat, n, n)).
 int lu_inverse(nslg_fm *fm, const double2 *LU, double2 *G, int n, const LuScratch &s, int nmat = 1,
                int64_t lu_stride = 0);
-// B[g] = L_g^{-1} B[g] (n x n right-hand sides) with the unit lower factor of an unpivoted LU.
-int lu_forward(nslg_fm *fm, const double2 *LU, double2 *B, int n, int nmat, int64_t lu_stride, int64_t b_stride);
+// Y[g] = A_g^{-1} W[g] from the factors (n x n right-hand sides, W and Y dense (nmat, n, n), W untouched).
+int lu_solve(nslg_fm *fm, const double2 *LU, const double2 *W, double2 *Y, int n, const LuScratch &s, int nmat,
+             int64_t lu_stride);
 int compute_hops_norm(nslg_fm *fm);
 
 // Tensor-core operator: planes of a real exp(d K) (built once per entry) and the fused M / Mdag launch.

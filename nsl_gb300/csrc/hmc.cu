@@ -297,7 +297,15 @@ int hubbard_force_dev(nslg_fm *fm, const double2 *phi, double2 Ut, int terms, in
     return NSLG_OK;
 }
 
+int hubbard_eval_batch_dev(nslg_fm *fm, const double2 *phi, int64_t nconf, double2 Ut, int terms, double2 *S,
+                           const double2 *Ut_cfg);
+
 int hubbard_eval_dev(nslg_fm *fm, const double2 *phi, double2 Ut, int terms, double2 *S) {
+    // the stratified log dets of both species as one batch (their launches are the same, and each fills half the GPU)
+    if ((terms & 2) && use_stratified(fm)) {
+        NSLG_TRY(hubbard_eval_batch_dev(fm, phi, 1, Ut, terms, S, nullptr));
+        return populate_dev(fm, phi, NSLG_HOLE);
+    }
     double2 total = make_double2(0, 0);
     cudaStream_t st = fm->ctx->stream;
     if (terms & 1) {

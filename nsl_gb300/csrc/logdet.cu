@@ -86,7 +86,7 @@ constexpr int LT = 1024;
 inline int panel_width(int n) { return n <= 64 ? 32 : 8; }
 
 __global__ void __launch_bounds__(LT) k_lu_panel(double2 *A, int n, int k0, int nb, int *piv, double2 *pivots,
-                                                 int *swaps, int *singular, int64_t mstride, bool pivoting) {
+                                                 int *swaps, int *singular, int64_t mstride) {
     // matrix blockIdx.x of a batch
     A += blockIdx.x * mstride;
     piv += (int64_t)blockIdx.x * n;
@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(LT) k_lu_panel(double2 *A, int n, int k0, int 
     for (int k = k0; k < k0 + nb; ++k) {
         double bv = -1.0;
         int bi = n;
-        for (int i = k + threadIdx.x; i < (pivoting ? n : k + 1); i += LT) {  // without pivoting: row k only
+        for (int i = k + threadIdx.x; i < n; i += LT) {
             const double2 v = A[(int64_t)i * n + k];
             const double m = hypot(v.x, v.y);
             if (m > bv || (m == bv && i < bi)) {
@@ -164,7 +164,7 @@ __device__ __forceinline__ bool piv_better(double m, int i, double bm, int bi) {
 
 template <int LPT, int NB>
 __global__ void __launch_bounds__(LPT) k_lu_panel_smem(double2 *A, int n, int k0, int nb, int *piv, double2 *pivots,
-                                                       int *swaps, int *singular, int64_t mstride, bool pivoting) {
+                                                       int *swaps, int *singular, int64_t mstride) {
     constexpr int PS = NB + 1;
     extern __shared__ double2 Ps[];  // (n - k0) x PS
     // matrix blockIdx.x of a batch (LPT threads: 512 for large panels, 128 for small matrices)
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(LPT) k_lu_panel_smem(double2 *A, int n, int k0
         // pivot: largest |a_ik|^2 over rows i >= kk, first index on ties
         double bm = -1.0;
         int bi = rows;
-        for (int i = kk + threadIdx.x; i < (pivoting ? rows : kk + 1); i += LPT) {  // without pivoting: row kk only
+        for (int i = kk + threadIdx.x; i < rows; i += LPT) {
             const double2 v = Ps[i * PS + kk];
             const double m = v.x * v.x + v.y * v.y;
             if (piv_better(m, i, bm, bi)) {
@@ -451,7 +451,7 @@ __global__ void k_pivot_logsum(const double2 *__restrict__ pivots, int n, double
 
 namespace {
 template <int NB>
-int lu_factor_nb(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t mstride, bool pivoting) {
+int lu_factor_nb(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t mstride) {
     cudaStream_t st = fm->ctx->stream;
     const double2 minus_one = make_double2(-1, 0);
     for (int k0 = 0; k0 < n; k0 += NB) {
@@ -459,14 +459,14 @@ int lu_factor_nb(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t
         const size_t smem = (size_t)(n - k0) * (NB + 1) * sizeof(double2);
         if (n - k0 <= 64)
             k_lu_panel_smem<128, NB><<<nmat, 128, smem, st>>>(A, n, k0, nb, s.piv, s.pivots, s.swaps, s.singular,
-                                                              mstride, pivoting);
+                                                              mstride);
         else if (smem <= (size_t)PANEL_SMEM)
             k_lu_panel_smem<512, NB><<<nmat, 512, smem, st>>>(A, n, k0, nb, s.piv, s.pivots, s.swaps, s.singular,
-                                                              mstride, pivoting);
+                                                              mstride);
         else
-            k_lu_panel<<<nmat, LT, 0, st>>>(A, n, k0, nb, s.piv, s.pivots, s.swaps, s.singular, mstride, pivoting);
+            k_lu_panel<<<nmat, LT, 0, st>>>(A, n, k0, nb, s.piv, s.pivots, s.swaps, s.singular, mstride);
         note_launch(st);
-        if (n > nb && pivoting) {
+        if (n > nb) {
             k_lu_laswp<<<dim3((unsigned)ceil_div(n, 128), (unsigned)nmat), 128, 0, st>>>(A, n, k0, nb, s.piv, mstride);
             note_launch(st);
         }
@@ -490,8 +490,7 @@ int lu_factor_nb(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t
 // Factors nmat matrices at once (matrix g at A + g * mstride, mstride 0 = n * n): each panel step is one launch
 // over the whole batch, so independent matrices (the two species, many configurations) factor side by side on
 // different SMs. Pivots, log sums and swap counts are per matrix; the singular flag is shared.
-int lu_factor(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t mstride, bool want_logsum,
-              bool pivoting) {
+int lu_factor(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t mstride, bool want_logsum) {
     cudaStream_t st = fm->ctx->stream;
     if (mstride == 0) mstride = (int64_t)n * n;
     {
@@ -514,8 +513,8 @@ int lu_factor(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t ms
     }
     NSLG_CUDA(cudaMemsetAsync(s.swaps, 0, (size_t)nmat * sizeof(int), st));
     if (!fm->defer_checks) NSLG_CUDA(cudaMemsetAsync(s.singular, 0, sizeof(int), st));
-    if (panel_width(n) == 32) NSLG_TRY(lu_factor_nb<32>(fm, A, n, s, nmat, mstride, pivoting));
-    else NSLG_TRY(lu_factor_nb<8>(fm, A, n, s, nmat, mstride, pivoting));
+    if (panel_width(n) == 32) NSLG_TRY(lu_factor_nb<32>(fm, A, n, s, nmat, mstride));
+    else NSLG_TRY(lu_factor_nb<8>(fm, A, n, s, nmat, mstride));
     if (want_logsum) {
         k_pivot_logsum<<<(unsigned)nmat, 256, 0, st>>>(s.pivots, n, s.logsum);
         note_launch(st);
@@ -526,8 +525,7 @@ int lu_factor(nslg_fm *fm, double2 *A, int n, LuScratch &s, int nmat, int64_t ms
 
 namespace {
 template <int NB>
-int lu_solve_nb(nslg_fm *fm, const double2 *LU, double2 *B, int n, int nmat, int64_t lu_stride, int64_t b_stride,
-                bool backward = true) {
+int lu_solve_nb(nslg_fm *fm, const double2 *LU, double2 *B, int n, int nmat, int64_t lu_stride, int64_t b_stride) {
     cudaStream_t st = fm->ctx->stream;
     const double2 minus_one = make_double2(-1, 0);
     const dim3 gc((unsigned)ceil_div(n, TRSM_T), (unsigned)nmat);
@@ -541,7 +539,6 @@ int lu_solve_nb(nslg_fm *fm, const double2 *LU, double2 *B, int n, int nmat, int
                            B + (int64_t)k0 * n, n, b_stride, B + (int64_t)(k0 + nb) * n, n, b_stride, nmat, false,
                            true));
     }
-    if (!backward) return NSLG_OK;
     for (int k0 = ((n - 1) / NB) * NB; k0 >= 0; k0 -= NB) {  // backward: U x = y
         const int nb = std::min(NB, n - k0);
         k_trsm_upper_block<NB><<<gc, TRSM_T, 0, st>>>(LU, B, n, k0, nb, lu_stride, b_stride);
@@ -553,10 +550,10 @@ int lu_solve_nb(nslg_fm *fm, const double2 *LU, double2 *B, int n, int nmat, int
     return NSLG_OK;
 }
 
-// B[g] = P_g I: the identity with the factorisation's row swaps applied in order (row k of the result is row
-// perm[k] of I, perm the composition of the swaps). Each block rebuilds perm in shared memory with one thread, then
+// B[g] = P_g W[g] (the identity for a null W): the factorisation's row swaps applied in order (row k of the result is row
+// perm[k], perm the composition of the swaps). Each block rebuilds perm in shared memory with one thread, then
 // its threads write rows [row0, row0 + rows_per_block) of matrix blockIdx.x.
-__global__ void k_perm_identity(double2 *B, int n, const int *piv, int64_t bstride, int rows_per_block) {
+__global__ void k_perm_rows(double2 *B, const double2 *W, int n, const int *piv, int64_t bstride, int rows_per_block) {
     extern __shared__ int perm[];
     const int g = blockIdx.x;
     piv += (int64_t)g * n;
@@ -574,7 +571,7 @@ __global__ void k_perm_identity(double2 *B, int n, const int *piv, int64_t bstri
     const int r0 = blockIdx.y * rows_per_block, r1 = min(n, r0 + rows_per_block);
     for (int64_t e = (int64_t)r0 * n + threadIdx.x; e < (int64_t)r1 * n; e += blockDim.x) {
         const int k = (int)(e / n), j = (int)(e % n);
-        B[e] = make_double2(j == perm[k] ? 1.0 : 0.0, 0.0);
+        B[e] = W ? W[g * bstride + (int64_t)perm[k] * n + j] : make_double2(j == perm[k] ? 1.0 : 0.0, 0.0);
     }
 }
 
@@ -798,8 +795,8 @@ int lu_inverse(nslg_fm *fm, const double2 *LU, double2 *G, int n, const LuScratc
     const int64_t nn = (int64_t)n * n;
     if (lu_stride == 0) lu_stride = nn;
     const int rpb = 32;
-    k_perm_identity<<<dim3((unsigned)nmat, (unsigned)ceil_div(n, rpb)), 256, (size_t)n * sizeof(int), st>>>(
-        G, n, s.piv, nn, rpb);
+    k_perm_rows<<<dim3((unsigned)nmat, (unsigned)ceil_div(n, rpb)), 256, (size_t)n * sizeof(int), st>>>(
+        G, nullptr, n, s.piv, nn, rpb);
     note_launch(st);
     if (panel_width(n) == 32) NSLG_TRY(lu_solve_nb<32>(fm, LU, G, n, nmat, lu_stride, nn));
     else NSLG_TRY(lu_solve_nb<8>(fm, LU, G, n, nmat, lu_stride, nn));
@@ -807,10 +804,19 @@ int lu_inverse(nslg_fm *fm, const double2 *LU, double2 *G, int n, const LuScratc
     return NSLG_OK;
 }
 
-// Forward substitution only: B[g] = L_g^{-1} B[g] with the unit lower factor of an LU computed without pivoting.
-int lu_forward(nslg_fm *fm, const double2 *LU, double2 *B, int n, int nmat, int64_t lu_stride, int64_t b_stride) {
-    if (panel_width(n) == 32) return lu_solve_nb<32>(fm, LU, B, n, nmat, lu_stride, b_stride, false);
-    return lu_solve_nb<8>(fm, LU, B, n, nmat, lu_stride, b_stride, false);
+// Y[g] = A_g^{-1} W[g]: the right-hand sides' rows in pivot order, then both substitutions.
+int lu_solve(nslg_fm *fm, const double2 *LU, const double2 *W, double2 *Y, int n, const LuScratch &s, int nmat,
+             int64_t lu_stride) {
+    cudaStream_t st = fm->ctx->stream;
+    const int64_t nn = (int64_t)n * n;
+    const int rpb = 32;
+    k_perm_rows<<<dim3((unsigned)nmat, (unsigned)ceil_div(n, rpb)), 256, (size_t)n * sizeof(int), st>>>(Y, W, n, s.piv, nn,
+                                                                                                    rpb);
+    note_launch(st);
+    if (panel_width(n) == 32) NSLG_TRY(lu_solve_nb<32>(fm, LU, Y, n, nmat, lu_stride, nn));
+    else NSLG_TRY(lu_solve_nb<8>(fm, LU, Y, n, nmat, lu_stride, nn));
+    NSLG_CUDA(cudaGetLastError());
+    return NSLG_OK;
 }
 
 int get_lu_scratch(nslg_fm *fm, int n, LuScratch &s, int nmat, const char *tag) {

@@ -16,9 +16,7 @@
 // L_j = Fk(s_j) ... Fk(Nt-1) = U_L D_L T_L and the adjoint of the prefix product R_j = Fk(0) ... Fk(s_j - 1),
 // R_j^H = U_R D_R T_R, each as a unitary U, graded positive scales D (sorted descending) and a well-conditioned T.
 // A stack step multiplies the next chunk product into U (Z = C U, condition number that of C), takes the QR
-// factorisation Z = Q R by two Cholesky-QR passes (Gram matrix, unpivoted LU of the Hermitian positive definite Gram
-// = Cholesky, forward substitution with the Cholesky factor: all batched GEMMs and the batched LU), and folds R into
-// D and T:
+// factorisation Z = Q R by two Cholesky-QR passes (see below), and folds R into D and T:
 // D' = diag(R) D, T' = D'^{-1} R D T, followed by a sort of D' (permuting U's columns and T's rows).
 // At a boundary, with D = D_b D_s split into the parts above and below 1,
 //   1 + L R = U_L D_Lb X D_Rb U_R^H,   X = D_Lb^{-1} (U_L^H U_R) D_Rb^{-1} + D_Ls (T_L T_R^H) D_Rs,
@@ -97,47 +95,185 @@ __global__ void k_ones(double *d, Bat b, int n, int nmat) {
     d[b.off(idx / n) + idx % n] = 1.0;
 }
 
-// After the unpivoted LU of a Hermitian positive definite Gram matrix G = L U (U = D L^H, D = diag(U) > 0), the
-// Cholesky factor R = D^{-1/2} U (upper triangle, real diagonal sqrt(D)). Q^H = R^{-H} Z^H is then solved with R
-// itself, not with the LU's L: L and U carry independent rounding, and pairing one with the other loses
-// ~cond(Z)^2 eps in Q R = Z. R^H = L'' diag(R) with the unit lower L''_ij = conj(R_ji) / R_jj, written into the LU
-// matrix's strictly lower part (k_chol_lower) so that the batched unit-lower forward substitution applies, and the
-// rows are divided by R_ii afterwards (k_rows_div_rdiag).
-__global__ void k_chol_r(const double2 *__restrict__ LU, double2 *__restrict__ R, int n, int nmat) {
+// ---- Cholesky-QR ------------------------------------------------------------------------------------------------------
+// Z = Q R from G = Z^H Z = R^H R, both in one blocked sweep over NB columns: the panel kernel factors the diagonal block,
+// forms its rows of R and the block column of Q = Z R^{-1}, and two rank-NB products update what is left of G (its upper
+// triangle) and of Z. Nothing is transposed and R is used for both, so Q R = Z to rounding.
+//
+// FP64 runs at ~2 FMAs per clock per SM here, so a triangular solve per column would be a chain of NB^2 / 2 dependent
+// FP64 steps; instead every CTA eliminates the small diagonal block redundantly (256 threads, one element each, one
+// barrier per column; the next pivot's reciprocal is formed by the thread that updates it) together with the identity,
+// which gives R_kk^{-H}, and the panel is a product with it, one output per thread.
+// Measured, one step of both stacks of both species (four matrices, n = 288): 10.2 ms with panel LU, triangular solves and
+// rank-8 updates in two passes, 4.4 ms with this sweep and the first-order second pass below.
+constexpr int CQ_NB = 16;
+
+__global__ void __launch_bounds__(CQ_NB *CQ_NB) k_cholqr_panel(const double2 *__restrict__ G, double2 *__restrict__ R,
+                                                               double2 *__restrict__ Z, int n, int k0, int nb,
+                                                               int ngb, bool refine, int *singular) {
+    constexpr int NB = CQ_NB;
+    __shared__ double2 D[NB][NB + 1], L[NB][NB + 1], T[NB][NB + 1];
+    __shared__ double rd[NB], sd[NB], dd[NB];  // 1 / d, 1 / sqrt(d), d
+    const int i = threadIdx.x / NB, j = threadIdx.x % NB;
     const int64_t nn = (int64_t)n * n;
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= nn * nmat) return;
-    const int64_t z = idx / nn, e = idx % nn;
-    const int i = (int)(e / n), j = (int)(e % n);
-    const double dii = LU[z * nn + (int64_t)i * n + i].x;
-    const double s = dii > 0.0 ? 1.0 / sqrt(dii) : 0.0;
-    if (j > i) {
-        const double2 u = LU[idx];
-        R[idx] = make_double2(u.x * s, u.y * s);
+    G += blockIdx.y * nn;
+    R += blockIdx.y * nn;
+    Z += blockIdx.y * nn;
+    // this CTA's part of the panel: NB columns of R's block row (blockIdx.x < ngb) or NB rows of Z
+    const bool gpart = blockIdx.x < ngb;
+    const int o0 = gpart ? k0 + nb + blockIdx.x * NB : (int)(blockIdx.x - ngb) * NB;
+    {
+        double2 v = make_double2(0, 0), t = make_double2(0, 0);
+        if (i < nb && j < nb && j >= i) v = G[(int64_t)(k0 + i) * n + k0 + j];
+        if (gpart) {
+            if (i < nb && o0 + j < n) t = G[(int64_t)(k0 + i) * n + o0 + j];  // T[q][column]
+        } else {
+            if (j < nb && o0 + i < n) t = Z[(int64_t)(o0 + i) * n + k0 + j];  // T[row][q]
+        }
+        D[i][j] = v;
+        T[i][j] = t;
+        L[i][j] = make_double2(i == j ? 1.0 : 0.0, 0.0);
+        if (threadIdx.x == 0) {
+            dd[0] = v.x;
+            rd[0] = v.x > 0.0 ? 1.0 / v.x : 0.0;
+        }
+    }
+    __syncthreads();
+    // rows i > q: upper part j >= i of the block, columns j <= q of the identity; row q is final after step q - 1
+    for (int q = 0; q + 1 < nb; ++q) {
+        if (i > q && i < nb && (j >= i || j <= q) && j < nb) {
+            const double r = rd[q];
+            const double2 u = D[q][i];  // multiplier conj(D_qi) / d_q
+            const double2 m = make_double2(u.x * r, -u.y * r);
+            const double2 x = j >= i ? D[q][j] : L[q][j];
+            double2 a = j >= i ? D[i][j] : L[i][j];
+            a.x = fma(-m.x, x.x, fma(m.y, x.y, a.x));
+            a.y = fma(-m.x, x.y, fma(-m.y, x.x, a.y));
+            if (j >= i) D[i][j] = a;
+            else L[i][j] = a;
+            if (i == q + 1 && j == i) {
+                dd[i] = a.x;
+                rd[i] = a.x > 0.0 ? 1.0 / a.x : 0.0;
+            }
+        }
+        __syncthreads();
+    }
+    // R_kk = D^{-1/2} U, W = R_kk^{-H} = D^{-1/2} L^{-1}
+    if (threadIdx.x < nb) sd[threadIdx.x] = dd[threadIdx.x] > 0.0 ? 1.0 / sqrt(dd[threadIdx.x]) : 0.0;
+    __syncthreads();
+    if (blockIdx.x == gridDim.x - 1) {  // one CTA stores the diagonal block
+        if (i < nb && j < nb && j >= i) {
+            const double s = sd[i];
+            R[(int64_t)(k0 + i) * n + k0 + j] =
+                j == i ? make_double2(sqrt(fmax(dd[i], 0.0)), 0.0) : make_double2(D[i][j].x * s, D[i][j].y * s);
+        }
+        if (threadIdx.x < nb && dd[threadIdx.x] == 0.0) *singular = 1;
+    }
+    // gpart: y = L^{-1} t per column (T[q][column]), R_{k0 + i, o0 + j} = y_i / sqrt(d_i).
+    // else: y = L^{-1} conj t per row (T[row][q]), Q_{o0 + i, k0 + j} = conj(y_j) / sqrt(d_j).
+    const int e = gpart ? i : j;  // which of the block's unknowns this thread holds
+    auto tval = [&](int q) -> double2 { return gpart ? T[q][j] : make_double2(T[i][q].x, -T[i][q].y); };
+    auto product = [&]() -> double2 {  // (L^{-1} t)_e
+        double2 acc = make_double2(0, 0);
+        for (int q = 0; q <= e; ++q) {
+            const double2 l = L[e][q], t = tval(q);
+            acc.x = fma(l.x, t.x, fma(-l.y, t.y, acc.x));
+            acc.y = fma(l.x, t.y, fma(l.y, t.x, acc.y));
+        }
+        return acc;
+    };
+    double2 y = e < nb ? product() : make_double2(0, 0);
+    if (refine) {  // y += L^{-1} (t - L y): an ill-conditioned block's explicit inverse alone loses cond eps in Q R = Z
+        double2 r = e < nb ? tval(e) : make_double2(0, 0);
+        __syncthreads();
+        T[i][j] = gpart ? y : make_double2(y.x, -y.y);
+        __syncthreads();
+        if (e < nb) {
+            r.x -= y.x;
+            r.y -= y.y;
+            for (int q = 0; q < e; ++q) {  // L_eq = conj(U_qe) / d_q
+                const double2 u = D[q][e], v = tval(q);
+                const double2 l = make_double2(u.x * rd[q], -u.y * rd[q]);
+                r.x = fma(-l.x, v.x, fma(l.y, v.y, r.x));
+                r.y = fma(-l.x, v.y, fma(-l.y, v.x, r.y));
+            }
+        }
+        __syncthreads();
+        T[i][j] = gpart ? r : make_double2(r.x, -r.y);
+        __syncthreads();
+        if (e < nb) {
+            const double2 c = product();
+            y.x += c.x;
+            y.y += c.y;
+        }
+    }
+    if (e >= nb) return;
+    const double s = sd[e];
+    if (gpart) {
+        if (o0 + j < n) R[(int64_t)(k0 + i) * n + o0 + j] = make_double2(y.x * s, y.y * s);
     } else {
-        R[idx] = make_double2(j == i ? sqrt(fmax(dii, 0.0)) : 0.0, 0.0);
+        if (o0 + i < n) Z[(int64_t)(o0 + i) * n + k0 + j] = make_double2(y.x * s, -y.y * s);
     }
 }
-__global__ void k_chol_lower(const double2 *__restrict__ R, double2 *__restrict__ LU, int n, int nmat) {
+
+// Second pass to first order. Q1 from one pass is orthogonal up to E = Q1^H Q1 - 1, |E| ~ cond(Z)^2 eps (1e-11 and less for
+// the chunk products here); its Cholesky factor is R2 = 1 + T + O(E^2), T the strict upper triangle of E plus half its
+// diagonal, so Q = Q1 (1 - T) and R = (1 + T) R1 to O(E^2) ~ 1e-22. E itself is evaluated in FP64; the corrections
+// Q1 T and T R1, of relative size |E|, are formed in FP32 (an error of 6e-8 |E| < 1e-18) and added in FP64.
+// out = C + sign A B (A, B rounded to FP32) for the matrices of a batch; Eu: the upper triangle of Q1^H Q1, which stands
+// for T as B (t_left = false: A = C = Q1, sign -1) or as A (t_left: B = C = R1, sign +1).
+constexpr int RF = 32;
+__global__ void __launch_bounds__(256) k_refine(const double2 *__restrict__ Eu, const double2 *__restrict__ X,
+                                                double2 *__restrict__ out, int n, bool t_left) {
+    __shared__ float2 As[RF][RF + 1], Bs[RF][RF + 1];
     const int64_t nn = (int64_t)n * n;
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= nn * nmat) return;
-    const int64_t z = idx / nn, e = idx % nn;
-    const int i = (int)(e / n), j = (int)(e % n);
-    if (i <= j) return;
-    const double rjj = R[z * nn + (int64_t)j * n + j].x;
-    const double2 rji = R[z * nn + (int64_t)j * n + i];
-    LU[idx] = rjj > 0.0 ? make_double2(rji.x / rjj, -rji.y / rjj) : make_double2(0.0, 0.0);
-}
-__global__ void k_rows_div_rdiag(double2 *__restrict__ Y, const double2 *__restrict__ R, int n, int nmat) {
-    const int64_t nn = (int64_t)n * n;
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= nn * nmat) return;
-    const int64_t z = idx / nn, e = idx % nn;
-    const int i = (int)(e / n);
-    const double rii = R[z * nn + (int64_t)i * n + i].x;
-    const double s = rii > 0.0 ? 1.0 / rii : 0.0;
-    Y[idx] = make_double2(Y[idx].x * s, Y[idx].y * s);
+    Eu += blockIdx.z * nn;
+    X += blockIdx.z * nn;
+    out += blockIdx.z * nn;
+    const int c0 = blockIdx.x * RF, r0 = blockIdx.y * RF;
+    const int tx = threadIdx.x % 32, ty = threadIdx.x / 32;
+    auto tval = [&](int r, int c) -> float2 {  // T[r][c]
+        if (r >= n || c >= n || c < r) return make_float2(0.f, 0.f);
+        const double2 v = Eu[(int64_t)r * n + c];
+        return r == c ? make_float2((float)(0.5 * (v.x - 1.0)), 0.f) : make_float2((float)v.x, (float)v.y);
+    };
+    auto xval = [&](int r, int c) -> float2 {
+        if (r >= n || c >= n) return make_float2(0.f, 0.f);
+        const double2 v = X[(int64_t)r * n + c];
+        return make_float2((float)v.x, (float)v.y);
+    };
+    float2 acc[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
+    // T[k][c] is zero for k > c; T[r][k] for k < r, and R1[k][c] for k > c
+    const int kend = min(n, c0 + RF);
+    for (int k0 = t_left ? r0 : 0; k0 < kend; k0 += RF) {
+        for (int r = ty; r < RF; r += 8) {
+            As[r][tx] = t_left ? tval(r0 + r, k0 + tx) : xval(r0 + r, k0 + tx);
+            Bs[r][tx] = t_left ? xval(k0 + r, c0 + tx) : tval(k0 + r, c0 + tx);
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int k = 0; k < RF; ++k) {
+            const float2 b = Bs[k][tx];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float2 a = As[ty + 8 * i][k];
+                acc[i].x = fmaf(a.x, b.x, fmaf(-a.y, b.y, acc[i].x));
+                acc[i].y = fmaf(a.x, b.y, fmaf(a.y, b.x, acc[i].y));
+            }
+        }
+        __syncthreads();
+    }
+    const int c = c0 + tx;
+    const double sg = t_left ? 1.0 : -1.0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = r0 + ty + 8 * i;
+        if (r >= n || c >= n) continue;
+        const double2 x = X[(int64_t)r * n + c];
+        out[(int64_t)r * n + c] = make_double2(x.x + sg * (double)acc[i].x, x.y + sg * (double)acc[i].y);
+    }
 }
 
 // UDT step, scales: dn[z][i] = R[z]_ii * d[z][i] (R_ii real positive), then R[z]_ij *= d_j / dn_i.
@@ -162,20 +298,24 @@ __global__ void k_udt_scale_r(double2 *__restrict__ R, const double *__restrict_
     R[idx] = make_double2(r.x * f, r.y * f);
 }
 
-// rank[z][i] = position of dn[z][i] in descending order (ties: lower index first).
+// rank[z][i] = position of dn[z][i] in descending order (ties: lower index first). One warp per element; the scales are
+// positive, so they are compared as integers (an FP64 comparison costs a warp 64 cycles).
 __global__ void k_rank_desc(const double *__restrict__ dn, int *__restrict__ rank, int n, int nmat) {
-    const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= (int64_t)n * nmat) return;
-    const int64_t z = idx / n;
-    const int i = (int)(idx % n);
-    const double *v = dn + z * n;
-    const double di = v[i];
+    const int64_t wid = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x % 32;
+    if (wid >= (int64_t)n * nmat) return;
+    const int64_t z = wid / n;
+    const int i = (int)(wid % n);
+    const long long *v = reinterpret_cast<const long long *>(dn + z * n);
+    const long long di = v[i];
     int r = 0;
-    for (int j = 0; j < n; ++j) {
-        const double dj = v[j];
+    for (int j = lane; j < n; j += 32) {
+        const long long dj = v[j];
         r += (dj > di) || (dj == di && j < i);
     }
-    rank[idx] = r;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    if (lane == 0) rank[wid] = r;
 }
 
 // U[z][:, rank_j] = Q[z][:, j], T[z][rank_i, :] = Tn[z][i, :], d[z][rank_i] = dn[z][i].
@@ -282,16 +422,17 @@ __global__ void k_grad_rows(const double2 *__restrict__ G, double2 *__restrict__
     out[((int64_t)g * Nt + t) * n + x] = make_double2(v.y, 1.0 - v.x);  // i (1 - v)
 }
 
-// sum over z of log(max(d, 1)) (the big scales of the suffix stack at s = 0), per matrix; and the log of the phase
-// rows sum_{t,x} Log(phiExp) (principal logs), one block per matrix.
+// Partial sums of sum_i log(max(d_i, 1)) (the big scales of the suffix stack at s = 0) and sum_{t,x} Log(phiExp) (principal
+// logs), block blockIdx.y of LT_BLOCKS of matrix blockIdx.x.
+constexpr int LT_BLOCKS = 32;
 __global__ void k_logdet_terms(const double *__restrict__ dL, Bat bd, const double2 *__restrict__ ph, int n, int Nt,
                                double2 *__restrict__ out) {
     __shared__ double2 red[256];
-    const int g = blockIdx.x;
+    const int g = blockIdx.x, first = blockIdx.y * 256 + threadIdx.x;
     double2 acc = make_double2(0, 0);
-    for (int i = threadIdx.x; i < n; i += 256) acc.x += log(fmax(dL[bd.off(g) + i], 1.0));
+    for (int i = first; i < n; i += 256 * LT_BLOCKS) acc.x += log(fmax(dL[bd.off(g) + i], 1.0));
     const double2 *p = ph + (int64_t)g * Nt * n;
-    for (int64_t e = threadIdx.x; e < (int64_t)Nt * n; e += 256) {
+    for (int64_t e = first; e < (int64_t)Nt * n; e += 256 * LT_BLOCKS) {
         const double2 v = p[e];
         acc.x += log(hypot(v.x, v.y));
         acc.y += atan2(v.y, v.x);
@@ -305,7 +446,7 @@ __global__ void k_logdet_terms(const double *__restrict__ dL, Bat bd, const doub
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) out[g] = red[0];
+    if (threadIdx.x == 0) out[g * LT_BLOCKS + blockIdx.y] = red[0];
 }
 
 inline unsigned blocks(int64_t n) { return (unsigned)ceil_div(n, EW); }
@@ -322,11 +463,12 @@ struct Strat {
     int n = 0, Nt = 0, nmat = 0, k = 1, J = 1, q = 1, r = 0;
     bool real = false;                          // every E' and E real: their products skip the imaginary parts
     double2 *Ep = nullptr, *E = nullptr;        // E' = exp(-sgn delta K), E = exp(sgn delta K) per matrix
-    double2 *C = nullptr, *CH = nullptr;        // chunk products and their adjoints (nmat, J, n, n)
+    double2 *C = nullptr;                       // chunk products (nmat, J, n, n)
+    bool first_order = true;                    // second QR pass to first order (chunks of bounded condition)
     double2 *SU = nullptr, *ST = nullptr;       // suffix stack (nmat, J + 1, n, n)
     double2 *PU = nullptr, *PT = nullptr;       // prefix stack (adjoint) (nmat, J + 1, n, n)
     double *Sd = nullptr, *Pd = nullptr;        // (nmat, J + 1, n)
-    double2 *Z, *Q, *R, *ZH, *Gm, *Y, *YH, *R1, *R2, *Tn;  // QR work (2 nmat, n, n)
+    double2 *Z, *Q, *R, *Gm, *R1, *R2, *Tn;     // QR work (2 nmat, n, n)
     double *dn = nullptr;
     int *rank = nullptr;
 };
@@ -372,7 +514,6 @@ int strat_setup(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry
     NSLG_TRY(ws_get(fm, "st_Sd", (size_t)nmat * (J + 1) * S.n, &S.Sd));
     const int side = need_prefix ? 2 : 1;
     if (need_prefix) {
-        NSLG_TRY(ws_get(fm, "st_CH", (size_t)nmat * J * nn, &S.CH));
         NSLG_TRY(ws_get(fm, "st_PU", (size_t)nmat * (J + 1) * nn, &S.PU));
         NSLG_TRY(ws_get(fm, "st_PT", (size_t)nmat * (J + 1) * nn, &S.PT));
         NSLG_TRY(ws_get(fm, "st_Pd", (size_t)nmat * (J + 1) * S.n, &S.Pd));
@@ -381,19 +522,20 @@ int strat_setup(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry
     NSLG_TRY(ws_get(fm, "st_Z", qn, &S.Z));
     NSLG_TRY(ws_get(fm, "st_Q", qn, &S.Q));
     NSLG_TRY(ws_get(fm, "st_R", qn, &S.R));
-    NSLG_TRY(ws_get(fm, "st_ZH", qn, &S.ZH));
     NSLG_TRY(ws_get(fm, "st_Gm", qn, &S.Gm));
-    NSLG_TRY(ws_get(fm, "st_Y", qn, &S.Y));
-    NSLG_TRY(ws_get(fm, "st_YH", qn, &S.YH));
     NSLG_TRY(ws_get(fm, "st_R1", qn, &S.R1));
     NSLG_TRY(ws_get(fm, "st_R2", qn, &S.R2));
     NSLG_TRY(ws_get(fm, "st_Tn", qn, &S.Tn));
     NSLG_TRY(ws_get(fm, "st_dn", (size_t)side * nmat * S.n, &S.dn));
     NSLG_TRY(ws_get(fm, "st_rank", (size_t)side * nmat * S.n, &S.rank));
+    // condition of a chunk product: at most exp(2 k |delta| rho). Up to 200 (the automatic chunk length keeps 81) the
+    // first QR pass leaves |E| < 1e-10 and its second order below rounding; one slice of a very large delta exceeds it.
+    const double kd = (double)(S.q + (S.r > 0)) * std::hypot(fm->delta.x, fm->delta.y) * fm->hops_norm1;
+    S.first_order = kd <= 0.5 * std::log(200.0);
     return NSLG_OK;
 }
 
-// Chunk products C[g, j] = Fk(s_j) ... Fk(s_{j+1} - 1) for every matrix and chunk (and their adjoints).
+// Chunk products C[g, j] = Fk(s_j) ... Fk(s_{j+1} - 1) for every matrix and chunk.
 int strat_chunks(nslg_fm *fm, Strat &S, const double2 *pinv) {
     cudaStream_t st = fm->ctx->stream;
     const int n = S.n, J = S.J;
@@ -415,42 +557,66 @@ int strat_chunks(nslg_fm *fm, Strat &S, const double2 *pinv) {
         NSLG_CUDA(cudaMemcpy2DAsync(S.C, (size_t)J * nn * sizeof(double2), buf, (size_t)J * nn * sizeof(double2),
                                     (size_t)nch * nn * sizeof(double2), S.nmat, cudaMemcpyDeviceToDevice, st));
     }
-    if (S.CH) NSLG_TRY(ctrans(st, S.C, flat(nn), S.CH, flat(nn), n, S.nmat * J));
     NSLG_CUDA(cudaGetLastError());
     return NSLG_OK;
 }
 
-// Z (cnt matrices, contiguous) = Q R by two Cholesky-QR passes.
+// One Cholesky-QR pass over cnt contiguous matrices: Gm = Z^H Z, its factor into R (upper triangle, zero below), Z <- Q.
+int cholqr_pass(nslg_fm *fm, Strat &S, double2 *R, int cnt) {
+    cudaStream_t st = fm->ctx->stream;
+    const int n = S.n;
+    const int64_t nn = (int64_t)n * n;
+    int *singular;
+    NSLG_TRY(ws_get(fm, "lu_singular", 1, &singular));
+    ZProd gram(n, n, n, S.Z, n, nn, S.Z, n, nn, S.Gm, n, nn);
+    gram.a_adjoint = true;
+    gram.upper = true;
+    NSLG_TRY(zprod(st, gram, cnt));
+    NSLG_CUDA(cudaMemsetAsync(R, 0, (size_t)(nn * cnt) * sizeof(double2), st));
+    for (int k0 = 0; k0 < n; k0 += CQ_NB) {
+        const int nb = std::min(CQ_NB, n - k0), rest = n - k0 - nb;
+        const int ngb = (int)ceil_div(rest, CQ_NB), nzb = (int)ceil_div(n, CQ_NB);
+        k_cholqr_panel<<<dim3((unsigned)(ngb + nzb), (unsigned)cnt), CQ_NB * CQ_NB, 0, st>>>(S.Gm, R, S.Z, n, k0, nb, ngb,
+                                                                                          !S.first_order, singular);
+        note_launch(st);
+        if (rest == 0) break;
+        const double2 *Rk = R + (int64_t)k0 * n + k0 + nb;
+        ZProd pg(rest, rest, nb, Rk, n, nn, Rk, n, nn, S.Gm + (int64_t)(k0 + nb) * (n + 1), n, nn);
+        pg.a_adjoint = pg.upper = pg.accumulate = true;
+        pg.alpha = make_double2(-1, 0);
+        NSLG_TRY(zprod(st, pg, cnt));
+        ZProd pz(n, rest, nb, S.Z + k0, n, nn, Rk, n, nn, S.Z + k0 + nb, n, nn);
+        pz.accumulate = true;
+        pz.alpha = make_double2(-1, 0);
+        NSLG_TRY(zprod(st, pz, cnt));
+    }
+    NSLG_CUDA(cudaGetLastError());
+    return NSLG_OK;
+}
+
+// Z (cnt matrices, contiguous) = S.Q S.R by two Cholesky-QR passes (the second one to first order where the chunks'
+// condition allows); Z is overwritten.
 int cholqr2(nslg_fm *fm, Strat &S, int cnt) {
     cudaStream_t st = fm->ctx->stream;
     const int n = S.n;
-    const int64_t nn = (int64_t)n * n, tot = nn * cnt;
-    const double2 one = make_double2(1, 0);
-    LuScratch ls;
-    NSLG_TRY(get_lu_scratch(fm, n, ls, cnt, "st_chol"));
-    // pass 1: G = Z^H Z = L U, R1 = D^{-1/2} U, Y = R1^{-H} Z^H = Q1^H
-    NSLG_TRY(ctrans(st, S.Z, flat(nn), S.ZH, flat(nn), n, cnt));
-    NSLG_TRY(zgemm(st, n, n, n, one, S.ZH, n, nn, S.Z, n, nn, S.Gm, n, nn, cnt, false));
-    NSLG_TRY(lu_factor(fm, S.Gm, n, ls, cnt, nn, false, false));
-    k_chol_r<<<blocks(tot), EW, 0, st>>>(S.Gm, S.R1, n, cnt);
-    k_chol_lower<<<blocks(tot), EW, 0, st>>>(S.R1, S.Gm, n, cnt);
-    note_launch(st, 2);
-    NSLG_CUDA(cudaMemcpyAsync(S.Y, S.ZH, tot * sizeof(double2), cudaMemcpyDeviceToDevice, st));
-    NSLG_TRY(lu_forward(fm, S.Gm, S.Y, n, cnt, nn, nn));
-    k_rows_div_rdiag<<<blocks(tot), EW, 0, st>>>(S.Y, S.R1, n, cnt);
-    note_launch(st);
-    // pass 2 on Q1: G = Q1^H Q1 = Y Y^H
-    NSLG_TRY(ctrans(st, S.Y, flat(nn), S.YH, flat(nn), n, cnt));
-    NSLG_TRY(zgemm(st, n, n, n, one, S.Y, n, nn, S.YH, n, nn, S.Gm, n, nn, cnt, false));
-    NSLG_TRY(lu_factor(fm, S.Gm, n, ls, cnt, nn, false, false));
-    k_chol_r<<<blocks(tot), EW, 0, st>>>(S.Gm, S.R2, n, cnt);
-    k_chol_lower<<<blocks(tot), EW, 0, st>>>(S.R2, S.Gm, n, cnt);
-    note_launch(st, 2);
-    NSLG_TRY(lu_forward(fm, S.Gm, S.Y, n, cnt, nn, nn));
-    k_rows_div_rdiag<<<blocks(tot), EW, 0, st>>>(S.Y, S.R2, n, cnt);
-    note_launch(st);
-    NSLG_TRY(zgemm(st, n, n, n, one, S.R2, n, nn, S.R1, n, nn, S.R, n, nn, cnt, false));
-    NSLG_TRY(ctrans(st, S.Y, flat(nn), S.Q, flat(nn), n, cnt));
+    const int64_t nn = (int64_t)n * n;
+    NSLG_TRY(cholqr_pass(fm, S, S.R1, cnt));
+    if (S.first_order) {
+        ZProd gram(n, n, n, S.Z, n, nn, S.Z, n, nn, S.Gm, n, nn);
+        gram.a_adjoint = true;
+        gram.upper = true;
+        NSLG_TRY(zprod(st, gram, cnt));
+        const dim3 grid((unsigned)ceil_div(n, RF), (unsigned)ceil_div(n, RF), (unsigned)cnt);
+        k_refine<<<grid, 256, 0, st>>>(S.Gm, S.Z, S.Q, n, false);
+        k_refine<<<grid, 256, 0, st>>>(S.Gm, S.R1, S.R, n, true);
+        note_launch(st, 2);
+    } else {
+        NSLG_TRY(cholqr_pass(fm, S, S.R2, cnt));
+        ZProd rr(n, n, n, S.R2, n, nn, S.R1, n, nn, S.R, n, nn);
+        rr.a_upper = true;
+        NSLG_TRY(zprod(st, rr, cnt));
+        NSLG_CUDA(cudaMemcpyAsync(S.Q, S.Z, (size_t)(nn * cnt) * sizeof(double2), cudaMemcpyDeviceToDevice, st));
+    }
     NSLG_CUDA(cudaGetLastError());
     return NSLG_OK;
 }
@@ -462,7 +628,6 @@ int udt_fold(nslg_fm *fm, Strat &S, int z0, const double *d_prev, const double2 
     cudaStream_t st = fm->ctx->stream;
     const int n = S.n, nmat = S.nmat;
     const int64_t nn = (int64_t)n * n;
-    const double2 one = make_double2(1, 0);
     double2 *R = S.R + z0 * nn, *Q = S.Q + z0 * nn, *Tn = S.Tn + z0 * nn;
     double *dn = S.dn + (int64_t)z0 * n;
     int *rank = S.rank + (int64_t)z0 * n;
@@ -470,8 +635,10 @@ int udt_fold(nslg_fm *fm, Strat &S, int z0, const double *d_prev, const double2 
     note_launch(st);
     k_udt_scale_r<<<blocks(nn * nmat), EW, 0, st>>>(R, d_prev, flat(dstride), dn, n, nmat);
     note_launch(st);
-    NSLG_TRY(zgemm(st, n, n, n, one, R, n, nn, T_prev, n, mstride, Tn, n, nn, nmat, false));
-    k_rank_desc<<<blocks((int64_t)n * nmat), EW, 0, st>>>(dn, rank, n, nmat);
+    ZProd rt(n, n, n, R, n, nn, T_prev, n, mstride, Tn, n, nn);
+    rt.a_upper = true;
+    NSLG_TRY(zprod(st, rt, nmat));
+    k_rank_desc<<<blocks((int64_t)32 * n * nmat), EW, 0, st>>>(dn, rank, n, nmat);
     note_launch(st);
     k_udt_permute<<<blocks(nn * nmat), EW, 0, st>>>(Q, Tn, dn, rank, Uo, To, flat(mstride), d_out, flat(dstride), n,
                                                     nmat);
@@ -502,9 +669,11 @@ int strat_stacks(nslg_fm *fm, Strat &S) {
         const int js = J - 1 - i;  // suffix: L_js = C_js L_{js+1}
         NSLG_TRY(zgemm(st, n, n, n, one, S.C + js * nn, n, (int64_t)J * nn, S.SU + (js + 1) * nn, n, ms, S.Z, n, nn,
                        nmat, false));
-        if (prefix)  // prefix (adjoint): R_{i+1}^H = C_i^H R_i^H
-            NSLG_TRY(zgemm(st, n, n, n, one, S.CH + i * nn, n, (int64_t)J * nn, S.PU + i * nn, n, ms,
-                           S.Z + nmat * nn, n, nn, nmat, false));
+        if (prefix) {  // prefix (adjoint): R_{i+1}^H = C_i^H R_i^H
+            ZProd pz(n, n, n, S.C + i * nn, n, (int64_t)J * nn, S.PU + i * nn, n, ms, S.Z + nmat * nn, n, nn);
+            pz.a_adjoint = true;
+            NSLG_TRY(zprod(st, pz, nmat));
+        }
         NSLG_TRY(cholqr2(fm, S, prefix ? 2 * nmat : nmat));
         NSLG_TRY(udt_fold(fm, S, 0, S.Sd + (int64_t)(js + 1) * n, S.ST + (js + 1) * nn, S.SU + js * nn,
                           S.ST + js * nn, S.Sd + (int64_t)js * n, ms, ds));
@@ -554,14 +723,13 @@ int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const Ex
     const int64_t nb = (int64_t)nmat * J, tot = nb * nn;
     const double2 one = make_double2(1, 0);
     // boundary Green functions G(s_j) for every matrix and chunk
-    double2 *ULH, *THH, *M1, *M2, *X, *W, *Xi, *G0, *Gf, *Gb, *Wt;
+    double2 *ULH, *THH, *M1, *M2, *X, *W, *G0, *Gf, *Gb, *Wt;
     NSLG_TRY(ws_get(fm, "stb_ULH", (size_t)tot, &ULH));
     NSLG_TRY(ws_get(fm, "stb_THH", (size_t)tot, &THH));
     NSLG_TRY(ws_get(fm, "stb_M1", (size_t)tot, &M1));
     NSLG_TRY(ws_get(fm, "stb_M2", (size_t)tot, &M2));
     NSLG_TRY(ws_get(fm, "stb_X", (size_t)tot, &X));
     NSLG_TRY(ws_get(fm, "stb_W", (size_t)tot, &W));
-    NSLG_TRY(ws_get(fm, "stb_Xi", (size_t)tot, &Xi));
     NSLG_TRY(ws_get(fm, "stb_G0", (size_t)tot, &G0));
     NSLG_TRY(ws_get(fm, "stb_Gf", (size_t)tot, &Gf));
     NSLG_TRY(ws_get(fm, "stb_Gb", (size_t)tot, &Gb));
@@ -579,10 +747,9 @@ int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const Ex
     LuScratch ls;
     NSLG_TRY(get_lu_scratch(fm, n, ls, (int)nb, "st_x"));
     if (!fm->defer_checks) NSLG_CUDA(cudaMemsetAsync(ls.singular, 0, sizeof(int), st));
-    NSLG_TRY(lu_factor(fm, X, n, ls, (int)nb, nn, false, true));
-    NSLG_TRY(lu_inverse(fm, X, Xi, n, ls, (int)nb, nn));
+    NSLG_TRY(lu_factor(fm, X, n, ls, (int)nb, nn, false));
     // Y = X^{-1} W, rows / D_Rb, G = U_R Y
-    NSLG_TRY(zgemm(st, n, n, n, one, Xi, n, nn, W, n, nn, M1, n, nn, (int)nb, false));
+    NSLG_TRY(lu_solve(fm, X, W, M1, n, ls, (int)nb, nn));
     k_rows_div_big<<<blocks(tot), EW, 0, st>>>(M1, S.Pd, dstack, n, (int)nb);
     note_launch(st);
     NSLG_TRY(zgemm2(st, n, n, n, one, S.PU, n, ms, nn, M1, n, (int64_t)J * nn, nn, G0, n, (int64_t)J * nn, nn, nmat,
@@ -625,7 +792,8 @@ int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const Ex
 
 // log det M for nmat matrices (as above; ph[g] = phiExp rows, sgn_g the species sign of matrix g): the suffix stack
 // to s = 0, then log det(1 + C(0)) = log det U_L + sum log D_Lb + log det X with X = D_Lb^{-1} U_L^H + D_Ls T_L,
-// plus log det of the slices' inverses, Nt sgn delta tr K + sum Log phiExp. out[g] on the host, imaginary part on
+// plus log det of the slices' inverses, Nt sgn delta tr K + sum Log phiExp. The LUs of X and of U_L (unitary: its phase)
+// are one batch: their panels are chains of dependent steps on one SM per matrix. out[g] on the host, imaginary part on
 // the principal branch; -inf for a singular X.
 int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, const int *sgn,
                  const double2 *ph, const double2 *pinv, double2 *out) {
@@ -636,11 +804,10 @@ int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntr
     NSLG_TRY(strat_stacks(fm, S));
     const int n = S.n, J = S.J;
     const int64_t nn = (int64_t)n * n, ms = (int64_t)(J + 1) * nn, ds = (int64_t)(J + 1) * n;
-    double2 *ULH, *X, *Uc, *terms;
+    double2 *ULH, *X, *terms;  // X: the nmat boundary matrices, then nmat copies of U_L
     NSLG_TRY(ws_get(fm, "stl_ULH", (size_t)nmat * nn, &ULH));
-    NSLG_TRY(ws_get(fm, "stl_X", (size_t)nmat * nn, &X));
-    NSLG_TRY(ws_get(fm, "stl_U", (size_t)nmat * nn, &Uc));
-    NSLG_TRY(ws_get(fm, "stl_terms", (size_t)nmat, &terms));
+    NSLG_TRY(ws_get(fm, "stl_X", (size_t)2 * nmat * nn, &X));
+    NSLG_TRY(ws_get(fm, "stl_terms", (size_t)nmat * LT_BLOCKS, &terms));
     NSLG_TRY(ctrans(st, S.SU, flat(ms), ULH, flat(nn), n, nmat));
     // X = D_Lb^{-1} U_L^H + D_Ls T_L (the boundary formula with an identity prefix)
     double *ones;
@@ -651,26 +818,22 @@ int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntr
                                                    nullptr, n, nmat);
     note_launch(st);
     NSLG_CUDA(cudaGetLastError());
-    NSLG_CUDA(cudaMemcpy2DAsync(Uc, nn * sizeof(double2), S.SU, ms * sizeof(double2), nn * sizeof(double2), nmat,
+    NSLG_CUDA(cudaMemcpy2DAsync(X + nmat * nn, nn * sizeof(double2), S.SU, ms * sizeof(double2), nn * sizeof(double2), nmat,
                                 cudaMemcpyDeviceToDevice, st));
-    LuScratch lx, lu;
-    NSLG_TRY(get_lu_scratch(fm, n, lx, nmat, "stl_x"));
-    NSLG_TRY(get_lu_scratch(fm, n, lu, nmat, "stl_u"));
+    LuScratch lx;
+    NSLG_TRY(get_lu_scratch(fm, n, lx, 2 * nmat, "stl_x"));
     NSLG_CUDA(cudaMemsetAsync(lx.singular, 0, sizeof(int), st));
-    NSLG_TRY(lu_factor(fm, X, n, lx, nmat, nn, true, true));
-    std::vector<double2> lsx(nmat), lsu(nmat), tm(nmat);
-    std::vector<int> swx(nmat), swu(nmat);
-    int sing = 0;
-    NSLG_CUDA(cudaMemcpyAsync(lsx.data(), lx.logsum, nmat * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    NSLG_CUDA(cudaMemcpyAsync(swx.data(), lx.swaps, nmat * sizeof(int), cudaMemcpyDeviceToHost, st));
-    NSLG_CUDA(cudaMemcpyAsync(&sing, lx.singular, sizeof(int), cudaMemcpyDeviceToHost, st));
-    NSLG_TRY(lu_factor(fm, Uc, n, lu, nmat, nn, true, true));  // det U_L (unitary: its phase)
-    k_logdet_terms<<<(unsigned)nmat, 256, 0, st>>>(S.Sd, flat(ds), ph, n, (int)fm->Nt, terms);
+    NSLG_TRY(lu_factor(fm, X, n, lx, 2 * nmat, nn, true));
+    k_logdet_terms<<<dim3((unsigned)nmat, LT_BLOCKS), 256, 0, st>>>(S.Sd, flat(ds), ph, n, (int)fm->Nt, terms);
     note_launch(st);
     NSLG_CUDA(cudaGetLastError());
-    NSLG_CUDA(cudaMemcpyAsync(lsu.data(), lu.logsum, nmat * sizeof(double2), cudaMemcpyDeviceToHost, st));
-    NSLG_CUDA(cudaMemcpyAsync(swu.data(), lu.swaps, nmat * sizeof(int), cudaMemcpyDeviceToHost, st));
-    NSLG_CUDA(cudaMemcpyAsync(tm.data(), terms, nmat * sizeof(double2), cudaMemcpyDeviceToHost, st));
+    std::vector<double2> ls((size_t)2 * nmat), tm((size_t)nmat * LT_BLOCKS);
+    std::vector<int> sw((size_t)2 * nmat);
+    int sing = 0;
+    NSLG_CUDA(cudaMemcpyAsync(ls.data(), lx.logsum, ls.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
+    NSLG_CUDA(cudaMemcpyAsync(sw.data(), lx.swaps, sw.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
+    NSLG_CUDA(cudaMemcpyAsync(&sing, lx.singular, sizeof(int), cudaMemcpyDeviceToHost, st));
+    NSLG_CUDA(cudaMemcpyAsync(tm.data(), terms, tm.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
     NSLG_CUDA(cudaStreamSynchronize(st));
     for (int g = 0; g < nmat; ++g) {
         if (sing) {
@@ -680,8 +843,14 @@ int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntr
         // Nt sgn delta tr K
         const double2 dtr = make_double2(sgn[g] * fm->delta.x * fm->hops_trace.x - sgn[g] * fm->delta.y * fm->hops_trace.y,
                                          sgn[g] * fm->delta.x * fm->hops_trace.y + sgn[g] * fm->delta.y * fm->hops_trace.x);
-        double re = lsx[g].x + lsu[g].x + tm[g].x + (double)fm->Nt * dtr.x;
-        double im = lsx[g].y + lsu[g].y + tm[g].y + (double)fm->Nt * dtr.y + ((swx[g] + swu[g]) & 1 ? M_PI : 0.0);
+        double2 t = make_double2(0, 0);
+        for (int k = 0; k < LT_BLOCKS; ++k) {
+            t.x += tm[(size_t)g * LT_BLOCKS + k].x;
+            t.y += tm[(size_t)g * LT_BLOCKS + k].y;
+        }
+        double re = ls[g].x + ls[nmat + g].x + t.x + (double)fm->Nt * dtr.x;
+        double im = ls[g].y + ls[nmat + g].y + t.y + (double)fm->Nt * dtr.y +
+                    ((sw[g] + sw[nmat + g]) & 1 ? M_PI : 0.0);
         im = std::remainder(im, 2.0 * M_PI);
         if (im <= -M_PI) im += 2.0 * M_PI;
         out[g] = make_double2(re, im);

@@ -184,3 +184,34 @@ def test_split_force_keeps_direct_product_to_beta_rho_28():
         h.populate(phi)
         out[fp] = np.asarray(h.gradLogDetM())
     assert np.array_equal(out["bf16split"], out["fp64"])
+
+
+@pytest.mark.parametrize("Nx", [1, 2, 15, 16, 17, 31, 32, 33, 48, 65])
+@pytest.mark.parametrize("Nt,beta", [(12, 9.0), (7, 8.0), (5, 8.25)])
+def test_stratified_panel_edges(Nx, Nt, beta):
+    """The Cholesky-QR sweep at the edges of its 16-column panels, with several slices per chunk, one slice per chunk within
+    the first-order second pass, and one slice per chunk of a condition beyond it (exp(2 delta rho) = e^6.6): gradient and
+    log det of both species against the dense inverse of M. Bar: relative perturbations of 256 eps of the slices (the
+    rounding of a few hundred operations each) move M^-1 by 256 eps |M^-1|^2 |M| and log det M by n 256 eps |M^-1| |M|;
+    1e-13 where that is smaller."""
+    import nsl_gb300 as N
+
+    eps = 256 * 2.0 ** -53
+    lat = N.Ring(Nx)
+    phi = _field(Nx, Nt, beta, 100 + Nx)
+    for species in (0, 1):
+        h = N.HubbardExp(lat, Nt, beta, 0.0, N.Species(species))
+        h.set_stabilisation("stratified")
+        h.populate(phi)
+        ho = O.HubbardExp(lat.hopping_matrix(), Nt, beta, 0.0, species)
+        ho.populate(phi)
+        n = Nt * Nx
+        Md = ho.M_dense().reshape(n, n)
+        inv = np.linalg.inv(Md)
+        nM, nI = np.linalg.norm(Md, 2), np.linalg.norm(inv, 2)
+        want = 1j * np.diag(inv).reshape(Nt, Nx)
+        err = np.abs(np.asarray(h.gradLogDetM()) - want).max()
+        assert err <= max(1e-13 * np.abs(want).max(), eps * nI ** 2 * nM), (species, err)
+        s, l = np.linalg.slogdet(Md)
+        ref = complex(l, np.angle(s))
+        assert abs(mod2pi(h.logDetM() - ref)) <= max(1e-13 * abs(ref), n * eps * nI * nM)
