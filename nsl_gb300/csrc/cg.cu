@@ -22,6 +22,8 @@
 // FP64 operator; FP64-class systems stop, unconverged, once their true residual no longer improves (the accuracy
 // FP64 can certify). Keeping the vectors in FP64 is what lets the low-precision operators reach that accuracy.
 
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <mutex>
 #include <set>
@@ -895,7 +897,13 @@ template <typename Top> int run_chunk(CgRun &R) {
 // ----- resident systems -----------------------------------------------------------------------------------------
 // Systems of at most RES_MAX_LEN elements on lattices of at most RES_MAX_NX sites whose shared-memory need fits
 // RES_MAX_SMEM, with a mixed-precision request, run in the resident kernel (cg_resident.cuh, float-float iteration);
-// NSLG_CG_RESIDENT=0 keeps every system on the launch-per-step solver.
+// NSLG_CG_RESIDENT=0 keeps every system on the launch-per-step solver. FP64 requests under the reference's recurrence rule
+// run on clusters (k_cg_cluster) while RC_CTAS SMs do an iteration's products faster than five launches take: up to
+// RC_WORK = elements x sites, the systems together on the SMs there are. Measured per iteration at Nt = 16: honeycomb
+// 3x3 (5184) 21.4 us in launches, 7.7 us on a cluster; honeycomb 6x6 (82944) 44 and 22 us, ring 128,
+// Nt = 8 (131072) 51 and 25 us; beyond, the cluster loses its lead (two FP64 FMAs per clock and SM) and its shared memory.
+constexpr int64_t RC_WORK = 131072;
+constexpr size_t RC_MAX_SMEM = 200 * 1024;
 constexpr int64_t RES_MAX_LEN = 2048;
 constexpr int RES_MAX_NX = 64;
 constexpr size_t RES_MAX_SMEM = 220 * 1024;
@@ -908,7 +916,29 @@ struct ResRun {
     CgState *d_st = nullptr;
     size_t smem = 0;
     int budget = 0;
+    bool cluster = false;  // FP64 recurrence systems on clusters
     RArgs args;
+    int launch(cudaStream_t st, unsigned count) const {
+        if (!cluster) {
+            k_cg_resident<<<count, RT, smem, st>>>(args);
+        } else {
+            cudaLaunchConfig_t cfg = {};
+            cfg.gridDim = dim3(count * RC_CTAS);
+            cfg.blockDim = dim3(RT);
+            cfg.dynamicSmemBytes = smem;
+            cfg.stream = st;
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            at.val.clusterDim.x = RC_CTAS;
+            at.val.clusterDim.y = at.val.clusterDim.z = 1;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            NSLG_CUDA(cudaLaunchKernelEx(&cfg, k_cg_cluster, args));
+        }
+        note_launch(st);
+        NSLG_CUDA(cudaGetLastError());
+        return NSLG_OK;
+    }
 };
 
 // Marks the instances whose systems go to the resident kernel; true if any.
@@ -916,12 +946,15 @@ int plan_resident(CgRun &R, int precision, bool *any) {
     *any = false;
     const char *env = std::getenv("NSLG_CG_RESIDENT");
     if (env && env[0] == '0') return NSLG_OK;
-    if (precision == NSLG_PREC_FP64 || (R.op != NSLG_OP_MMDAGGER && R.op != NSLG_OP_MDAGGERM)) return NSLG_OK;
+    if (R.op != NSLG_OP_MMDAGGER && R.op != NSLG_OP_MDAGGERM) return NSLG_OK;
+    const bool fp64 = precision == NSLG_PREC_FP64;
+    if (fp64 && (R.reliable || R.P.nsys * RC_CTAS > R.fm->ctx->num_sms)) return NSLG_OK;
     for (auto &I : R.inst) {
         nslg_fm *f = I.fm;
         const int64_t len = I.rows_per_sys * f->Nx;
-        if (f->kind != NSLG_FM_EXP || f->delta.y != 0.0 || f->Nx > RES_MAX_NX || len > RES_MAX_LEN ||
-            res_smem_bytes(len, (int)f->Nx) > RES_MAX_SMEM)
+        if (f->kind != NSLG_FM_EXP || f->delta.y != 0.0) continue;
+        if (fp64 ? len * f->Nx > RC_WORK || rc_smem_bytes(I.rows_per_sys, (int)f->Nx) > RC_MAX_SMEM
+                 : f->Nx > RES_MAX_NX || len > RES_MAX_LEN || res_smem_bytes(len, (int)f->Nx) > RES_MAX_SMEM)
             continue;
         const ExpEntry *E;
         NSLG_TRY(get_exp(f, make_double2(f->sgn * f->delta.x, 0.0), &E));
@@ -934,10 +967,11 @@ int plan_resident(CgRun &R, int precision, bool *any) {
 
 // Hands the resident systems over (their states move to the kernel's own array, CG_RESIDENT in the solver's) and
 // launches the resident kernel on the first handle's side stream, after everything queued on the solver's stream.
-int resident_start(CgRun &R, const double2 *b, ResRun &Q) {
+int resident_start(CgRun &R, const double2 *b, int precision, ResRun &Q) {
     nslg_fm *fm = R.fm;
     cudaStream_t st = fm->ctx->stream;
     const Plan &P = R.P;
+    Q.cluster = precision == NSLG_PREC_FP64;
     Q.sys.assign((size_t)P.nsys, RSys{});
     double cost = 1;
     for (auto &I : R.inst) {
@@ -956,7 +990,7 @@ int resident_start(CgRun &R, const double2 *b, ResRun &Q) {
             y.len = (int)len;
             Q.list.push_back((int)(I.s0 + k));
         }
-        Q.smem = std::max(Q.smem, res_smem_bytes(len, (int)f->Nx));
+        Q.smem = std::max(Q.smem, Q.cluster ? rc_smem_bytes(I.rows_per_sys, (int)f->Nx) : res_smem_bytes(len, (int)f->Nx));
         cost = std::max(cost, 3.3 * (double)len * (double)f->Nx + 10.0 * (double)len);
     }
     // iterations per launch: ~1e9 cycles of the slowest (FP64-escalated) system, so that one launch stays well
@@ -969,6 +1003,8 @@ int resident_start(CgRun &R, const double2 *b, ResRun &Q) {
         if (!done.count(fm->ctx->device)) {
             NSLG_CUDA(cudaFuncSetAttribute(k_cg_resident, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                            (int)RES_MAX_SMEM));
+            NSLG_CUDA(cudaFuncSetAttribute(k_cg_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)RC_MAX_SMEM));
             done.insert(fm->ctx->device);
         }
     }
@@ -1007,10 +1043,7 @@ int resident_start(CgRun &R, const double2 *b, ResRun &Q) {
     if (!fm->ev_join) NSLG_CUDA(cudaEventCreateWithFlags(&fm->ev_join, cudaEventDisableTiming));
     NSLG_CUDA(cudaEventRecord(fm->ev_fork, st));
     NSLG_CUDA(cudaStreamWaitEvent(fm->side, fm->ev_fork, 0));
-    k_cg_resident<<<(unsigned)count, RT, Q.smem, fm->side>>>(A);
-    note_launch(fm->side);
-    NSLG_CUDA(cudaGetLastError());
-    return NSLG_OK;
+    return Q.launch(fm->side, (unsigned)count);
 }
 
 // Waits for the resident kernel, launches it again for systems that ran out of their per-launch budget, hands the
@@ -1031,9 +1064,7 @@ int resident_finish(CgRun &R, ResRun &Q, int64_t *updates, int64_t *rebases, int
         Q.list = again;
         NSLG_CUDA(cudaMemcpyAsync(Q.d_list, Q.list.data(), Q.list.size() * sizeof(int), cudaMemcpyHostToDevice,
                                   fm->side));
-        k_cg_resident<<<(unsigned)Q.list.size(), RT, Q.smem, fm->side>>>(Q.args);
-        note_launch(fm->side);
-        NSLG_CUDA(cudaGetLastError());
+        NSLG_TRY(Q.launch(fm->side, (unsigned)Q.list.size()));
     }
     NSLG_CUDA(cudaEventRecord(fm->ev_join, fm->side));
     NSLG_CUDA(cudaStreamWaitEvent(st, fm->ev_join, 0));
@@ -1218,7 +1249,7 @@ int cg_run(CgRun &R, const double2 *b, const double2 *x0, double2 *x, double2 *x
     NSLG_CUDA(cudaGetLastError());
     ResRun Q;
     if (resident) {  // the small systems leave for the resident kernel, which runs beside the loop below
-        NSLG_TRY(resident_start(R, b, Q));
+        NSLG_TRY(resident_start(R, b, precision, Q));
         for (auto &I : R.inst) I.idle = I.resident;
         R.skip_idle = true;
     }

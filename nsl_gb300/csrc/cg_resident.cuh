@@ -24,7 +24,7 @@
 // (two float-float operand vectors, or two FP64 vectors), exp(delta K) transposed as float-float and in FP64
 // (16 Nx^2 bytes).
 //
-// (Included inside cg.cu's anonymous namespace.)
+// (Included inside cg.cu's anonymous namespace, after <cooperative_groups.h>.)
 
 struct RSys {
     const double2 *ph;  // phases exp(i sgn phi + sgn mu~) (Nt, Nx) of the system's fermion matrix
@@ -563,6 +563,205 @@ __global__ void __launch_bounds__(RT) k_cg_resident(RArgs A) {
         A.counts[3 * s + 1] = n_reb;
         A.counts[3 * s + 2] = n_esc;
     }
+}
+
+// ----- FP64 systems on a cluster ---------------------------------------------------------------------------------------
+// The reference's rule (recurrence, FP64 operator) for one small system on a cluster of RC_CTAS CTAs. One SM does ~2 FP64
+// FMAs per clock, so a resident FP64 iteration is bound by its own products; here the system's rows (time slices) are
+// dealt to the CTAs. Every CTA holds all of p and of the second factor's operand w (its rows' new values are written
+// into every CTA's shared memory), and its rows of x, r, t and the first factor's result; a dot product is a sum per
+// warp, exchanged the same way and added in one order by every CTA, so all take the same decisions. Four cluster
+// barriers per iteration. KS threads share one output's sum over y while a CTA has fewer outputs than threads.
+// Measured per iteration, honeycomb 3x3, Nt = 16: 21.4 us as five launches, 14.1 us on one SM, 7.7 us here.
+constexpr int RC_CTAS = 8;
+
+__host__ __device__ constexpr size_t rc_smem_bytes(int64_t rows, int Nx) {
+    const size_t own = (size_t)((rows + RC_CTAS - 1) / RC_CTAS) * Nx;
+    return (size_t)rows * Nx * 32 + own * 80 + (size_t)Nx * Nx * 8;
+}
+
+__global__ void __launch_bounds__(RT) k_cg_cluster(RArgs A) {
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    extern __shared__ __align__(16) unsigned char smem[];
+    constexpr int NW = RT / 32;
+    __shared__ double2 slot[2][RC_CTAS * NW];  // partial sums of every warp of the cluster: <p, A p> and |r|^2
+    __shared__ double2 alpha_sh;
+    __shared__ double rn_sh, beta_sh;
+    const int rank = (int)cl.block_rank();
+    const int s = A.list[blockIdx.x / RC_CTAS];
+    const RSys Y = A.sys[s];
+    const int Nt = Y.Nt, Nx = Y.Nx, n = Y.len, rows = n / Nx;
+    const int64_t off = Y.off;
+    const int tid = threadIdx.x;
+    const int maxown = (rows + RC_CTAS - 1) / RC_CTAS;
+    const int row0 = min(rows, rank * maxown), row1 = min(rows, row0 + maxown);
+    const int m = (row1 - row0) * Nx, e0 = row0 * Nx;  // own elements [e0, e0 + m)
+    double2 *p = reinterpret_cast<double2 *>(smem);
+    double2 *w = p + n;
+    double2 *x = w + n, *r = x + maxown * Nx, *t = r + maxown * Nx, *h = t + maxown * Nx, *ph = h + maxown * Nx;
+    double *Et = reinterpret_cast<double *>(ph + maxown * Nx);
+    CgState S = A.st[s];
+    if (S.status != CG_ACTIVE) return;  // the same for every CTA of the cluster
+    const bool mmdag = A.op == NSLG_OP_MMDAGGER;
+    for (int i = tid; i < n; i += RT) {
+        const double2 v = A.p[off + i];
+        p[i] = v;
+        if (!mmdag) w[i] = r_cmul(Y.ph[i % (Nt * Nx)], v);
+    }
+    for (int i = tid; i < m; i += RT) {
+        x[i] = A.x[off + e0 + i];
+        r[i] = A.r[off + e0 + i];
+        ph[i] = Y.ph[(e0 + i) % (Nt * Nx)];
+    }
+    for (int i = tid; i < Nx * Nx; i += RT) {
+        const int xx = i / Nx, yy = i - xx * Nx;
+        Et[yy * Nx + xx] = Y.E[i];
+    }
+    int ks = 1;  // threads per output
+    while (ks < 4 && 2 * ks * m <= RT) ks *= 2;
+    const int per = RT / ks, kq = tid % ks;
+    const int m_all = (m + per - 1) / per * per;  // whole passes: every lane takes part in the shuffles
+    auto rowdot = [&](const double2 *v, int xs, bool act) -> double2 {
+        double2 a = make_double2(0, 0);
+        if (act)
+            for (int y = kq; y < Nx; y += ks) {
+                const double e = Et[y * Nx + xs];
+                const double2 c = v[y];
+                a.x = fma(e, c.x, a.x);
+                a.y = fma(e, c.y, a.y);
+            }
+        for (int o = 1; o < ks; o <<= 1) {
+            a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+            a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+        }
+        return a;
+    };
+    auto publish = [&](double2 *buf, int i, double2 v) {  // element e0 + i of a replicated vector
+#pragma unroll
+        for (int c = 0; c < RC_CTAS; ++c) cl.map_shared_rank(buf, c)[e0 + i] = v;
+    };
+    const int lane = tid % 32, warp = tid / 32;
+    // this warp's sum of v into every CTA's slots (values sit in every `first`-th lane; `any`: the warp has some)
+    auto contribute = [&](int which, double2 v, int first, bool any) {
+        if (any)
+            for (int o = 16; o >= first; o >>= 1) {
+                v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+                if (which == 0) v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+            }
+        // lane 0 holds the sum; eight lanes store it, one CTA each
+        v.x = __shfl_sync(0xffffffffu, v.x, 0);
+        v.y = __shfl_sync(0xffffffffu, v.y, 0);
+        if (lane < RC_CTAS) cl.map_shared_rank(&slot[which][0], lane)[rank * NW + warp] = v;
+    };
+    auto total = [&](int which) -> double2 {  // warp 0: the slots in a fixed order
+        double2 v = slot[which][lane];
+        for (int k = 32; k < RC_CTAS * NW; k += 32) {
+            v.x += slot[which][k + lane].x;
+            v.y += slot[which][k + lane].y;
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+            if (which == 0) v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        }
+        return v;
+    };
+    cl.sync();
+    int steps = 0;
+    while (S.status == CG_ACTIVE && steps < A.budget) {
+        ++steps;
+        // first factor: h = M^dagger p, w = phase o h (M M^dagger), or h = M p from w = phase o p, then w = h
+        for (int i = tid / ks; i < m_all; i += per) {
+            const bool act = i < m;
+            const RIdx q = r_index(e0 + (act ? i : 0), Nt, Nx);
+            double2 z = rowdot(mmdag ? p + q.rowD : w + q.rowM, q.x, act);
+            if (act && kq == 0) {
+                if (mmdag) z = r_cmulc(ph[i], z);
+                const double sg = mmdag ? q.sD : q.sM;
+                const double2 pv = p[e0 + i];
+                h[i] = make_double2(pv.x - sg * z.x, pv.y - sg * z.y);
+            }
+        }
+        if (!mmdag) cl.sync();  // every CTA has read w = phase o p before it is overwritten
+        else __syncthreads();
+        for (int i = tid; i < m; i += RT) publish(w, i, mmdag ? r_cmul(ph[i], h[i]) : h[i]);
+        cl.sync();
+        // second factor t = A p, <p, t>
+        double2 acc = make_double2(0, 0);
+        for (int i = tid / ks; i < m_all; i += per) {
+            const bool act = i < m;
+            const RIdx q = r_index(e0 + (act ? i : 0), Nt, Nx);
+            double2 z = rowdot(mmdag ? w + q.rowM : w + q.rowD, q.x, act);
+            if (act && kq == 0) {
+                if (!mmdag) z = r_cmulc(ph[i], z);
+                const double sg = mmdag ? q.sM : q.sD;
+                const double2 hv = h[i], pv = p[e0 + i];
+                const double2 o = make_double2(hv.x - sg * z.x, hv.y - sg * z.y);
+                acc.x += pv.x * o.x + pv.y * o.y;
+                acc.y += pv.x * o.y - pv.y * o.x;
+                t[i] = o;
+            }
+        }
+        contribute(0, acc, ks, warp * 32 / ks < m);
+        cl.sync();
+        if (warp == 0) {  // alpha = |r|^2 / <p, A p> (CG.tpp:45-52)
+            const double2 pt = total(0);
+            if (lane == 0) {
+                const double den = pt.x * pt.x + pt.y * pt.y;
+                alpha_sh = make_double2(S.rsq * pt.x / den, -S.rsq * pt.y / den);
+            }
+        }
+        __syncthreads();
+        const double ar = alpha_sh.x, ai = alpha_sh.y;
+        double rr = 0;
+        for (int i = tid; i < m; i += RT) {
+            const double2 pv = p[e0 + i], tv = t[i];
+            double2 xv = x[i], rv = r[i];
+            xv.x += ar * pv.x - ai * pv.y;
+            xv.y += ar * pv.y + ai * pv.x;
+            rv.x -= ar * tv.x - ai * tv.y;
+            rv.y -= ar * tv.y + ai * tv.x;
+            x[i] = xv;
+            r[i] = rv;
+            rr += rv.x * rv.x + rv.y * rv.y;
+        }
+        contribute(1, make_double2(rr, 0.0), 1, warp * 32 < m);
+        cl.sync();
+        if (warp == 0) {
+            const double v = total(1).x;
+            if (lane == 0) {
+                rn_sh = v;
+                beta_sh = v / S.rsq;
+            }
+        }
+        __syncthreads();
+        const double rn = rn_sh;
+        CgState N = S;  // the transitions of k_cg_p under the recurrence rule
+        N.iters = S.iters + 1;
+        if (rn <= S.eps2) N.status = CG_CONVERGED;
+        else if (N.iters >= A.max_iter) N.status = CG_EXHAUSTED;
+        if (N.status == CG_ACTIVE) {
+            N.rsq = rn;
+            N.maxr = fmax(S.maxr, rn);
+            const double beta = beta_sh;
+            for (int i = tid; i < m; i += RT) {
+                double2 pv = p[e0 + i];
+                const double2 rv = r[i];
+                pv.x = rv.x + beta * pv.x;
+                pv.y = rv.y + beta * pv.y;
+                publish(p, i, pv);
+                if (!mmdag) publish(w, i, r_cmul(ph[i], pv));
+            }
+        }
+        S = N;
+        cl.sync();  // p is complete everywhere; no CTA leaves while another still writes into it
+    }
+    for (int i = tid; i < m; i += RT) {
+        A.x[off + e0 + i] = x[i];
+        A.r[off + e0 + i] = r[i];
+        A.p[off + e0 + i] = p[e0 + i];
+    }
+    if (rank == 0 && tid == 0) A.st[s] = S;
 }
 
 // status of the flagged systems <- CG_RESIDENT (their own copy in rst), or back from rst

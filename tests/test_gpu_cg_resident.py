@@ -121,3 +121,43 @@ def test_group_mixes_resident_and_launch_per_step(monkeypatch):
         assert res.max() <= eps * 1.01
         xa, loa, _ = _solve(monkeypatch, h, "MMdagger", b, eps, "bf16split", "true_residual_dd")
         assert rel_err(np.asarray(x) + np.asarray(lo), xa + loa) < 1e-6
+
+
+@pytest.mark.parametrize("Nx,Nt,R", [(1, 1, 1), (2, 3, 1), (7, 8, 1), (18, 16, 1), (18, 9, 5), (50, 20, 1), (128, 8, 1), (33, 13, 2)])
+@pytest.mark.parametrize("op", ["MMdagger", "MdaggerM"])
+@pytest.mark.parametrize("mode", ["shared", "per_rhs"])
+def test_fp64_recurrence_on_a_cluster(Nx, Nt, R, op, mode, monkeypatch):
+    """FP64 systems under the reference's rule on a thread-block cluster (fewer rows than CTAs, rows that do not divide,
+    one to five right-hand sides) against the launch-per-step solver: both stop at |r| <= eps, so the solutions differ by
+    at most 2 eps |A^-1| plus the recurrences' drift, 1e-12 |A| |x| |A^-1|; and an exhausted solve returns its iterate."""
+    import nsl_gb300 as N
+    from oracle import nsl_oracle as O
+
+    rng = np.random.default_rng(10 * Nx + Nt)
+    lat = N.Ring(Nx)
+    phi = rng.standard_normal((Nt, Nx)) * 0.3 + 0j
+    b = rng.standard_normal((R, Nt, Nx)) + 1j * rng.standard_normal((R, Nt, Nx))
+    fm = N.HubbardExp(lat, Nt, 0.1 * Nt)
+    fm.populate(phi)
+    o = O.HubbardExp(lat.hopping_matrix(), Nt, 0.1 * Nt)
+    o.populate(phi)
+    n = Nt * Nx
+    M = o.M_dense().reshape(n, n)
+    A = M @ M.conj().T if op == "MMdagger" else M.conj().T @ M
+    eps = 1e-10
+    out = {}
+    for flag in ("1", "0"):
+        monkeypatch.setenv("NSLG_CG_RESIDENT", flag)
+        cg = N.CG(fm, getattr(N.MatrixCombination, op), eps, 100000, mode=mode)
+        out[flag] = (np.asarray(cg(b)), cg.stats)
+        few = N.CG(fm, getattr(N.MatrixCombination, op), eps, 3, mode=mode)
+        out[flag] += (np.asarray(few(b)), few.stats)
+    (x1, s1, y1, t1), (x0, s0, y0, t0) = out["1"], out["0"]
+    assert s1["converged"] == s0["converged"] == s1["systems"]
+    assert abs(s1["iterations"] - s0["iterations"]) <= max(2, 0.02 * s0["iterations"])
+    inv, nA = np.linalg.norm(np.linalg.inv(A), 2), np.linalg.norm(A, 2)
+    for r in range(R):
+        bound = 2 * eps * inv + 1e-12 * nA * np.linalg.norm(x0[r]) * inv
+        assert np.linalg.norm(x1[r] - x0[r]) <= bound
+    assert t1["iterations"] == t0["iterations"] and t1["converged"] == t0["converged"]
+    assert np.linalg.norm(y1 - y0) <= 1e-10 * np.linalg.norm(y0)
