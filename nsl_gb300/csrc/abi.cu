@@ -380,6 +380,12 @@ NSLG_API int nslg_fm_destroy(nslg_fm *fm) {
             cudaFree(kv.second.tc->lo);
             delete kv.second.tc;
         }
+        if (kv.second.dd) {
+            cudaFree(kv.second.dd->planes);
+            cudaFree(kv.second.dd->col_exp);
+            cudaFree(kv.second.dd->klist);
+            delete kv.second.dd;
+        }
         if (kv.second.oz) {
             cudaFree(kv.second.oz->planes);
             cudaFree(kv.second.oz->col_exp);
@@ -537,7 +543,7 @@ NSLG_API int nslg_fm_apply_dd(nslg_fm *fm, int op, const nslg_c128 *psi_hi, cons
     if (!ld) NSLG_CUDA(cudaMemcpyAsync(out_lo, ol, bytes, cudaMemcpyDeviceToHost, st));
     bool ih;
     NSLG_TRY(device_ptr(fm, psi_hi, &ih));
-    if (!hd || !ld || !ih) NSLG_CUDA(cudaStreamSynchronize(st));
+    if (!hd || !ld || !ih) return check_tc_error(fm);  // synchronises
     return NSLG_OK;
 }
 

@@ -101,54 +101,6 @@ static_assert(OZ_ZSHIFT == 53, "recombination scale");
 constexpr int OZ_EXACT = 4;
 constexpr int OZ_ERR_BOUND = 31;  // tensor-core error code: exp(delta K) fails the digit-sum bound
 
-// Shared-memory matrix descriptor: K-major operand rows of 32 B, 32-byte swizzle, 8-row core groups 256 B apart.
-__device__ __forceinline__ uint64_t sdesc_kmajor_sw32(uint32_t saddr) {
-    uint64_t d = 0;
-    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
-    d |= (uint64_t)1 << 16;           // leading byte offset (unused for swizzled K-major)
-    d |= (uint64_t)(256 >> 4) << 32;  // stride byte offset: 8 rows x 32 B
-    d |= (uint64_t)1 << 46;           // descriptor version (sm_100)
-    d |= (uint64_t)6 << 61;           // layout: SWIZZLE_32B
-    return d;
-}
-
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
-    return (1u << 4)     // D: F32
-           | (1u << 7)   // A: BF16
-           | (1u << 10)  // B: BF16
-           | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-// D[tmem] (+)= A[smem] * B[smem]^T, kind::f16 (BF16 operands, FP32 accumulation), issued by one thread.
-// (The A collector buffer does not change the instruction rate measured on this part, ~44 cycles per N = 32 MMA.)
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                         uint32_t accumulate) {
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
-            d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-// zint 2^e as an FP64 value (rounded to nearest, ties away from zero) from integer operations only: GB300 runs an
-// integer -> FP64 conversion and the scaling multiply on its FP64 pipe, ~2 operations per clock per SM.
-__device__ __forceinline__ double scaled_to_double(long long zint, int e) {
-    if (zint == 0) return 0.0;
-    const unsigned long long sign = zint < 0 ? (1ull << 63) : 0ull;
-    unsigned long long u = zint < 0 ? 0ull - (unsigned long long)zint : (unsigned long long)zint;
-    const int lz = __clzll((long long)u);
-    u <<= lz;                                                 // leading one at bit 63: |zint| = u 2^-lz
-    unsigned long long m = (u >> 11) + ((u >> 10) & 1ull);    // 53 significant bits, rounded
-    int ex = e + 63 - lz;                                     // |zint| 2^e = (m / 2^52) 2^ex
-    if (m >> 53) {                                            // the rounding carried into a 54th bit
-        m >>= 1;
-        ++ex;
-    }
-    if (ex < -1022) return __longlong_as_double((long long)sign);                         // below the normal range: 0
-    if (ex > 1023) return __longlong_as_double((long long)(sign | 0x7FF0000000000000ull));  // above it: infinity
-    return __longlong_as_double((long long)(sign | ((unsigned long long)(ex + 1023) << 52) | (m & 0xFFFFFFFFFFFFFull)));
-}
-
 template <int MODE>
 __device__ __forceinline__ double2 oz_operand(const double2 *__restrict__ psi, const double2 *__restrict__ phase,
                                               int64_t grow, int t, int Nx, int y) {
@@ -319,7 +271,7 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
     } else if (warp == 1) {
         if (lane == 0) {  // MMA issuer
             int it = 0, tc_n = 0;
-            const uint64_t dsm0 = sdesc_kmajor_sw32(tc::smem_addr(smem));  // descriptor of stage 0, slice 0
+            const uint64_t dsm0 = tc::sdesc_kmajor_sw32(tc::smem_addr(smem));  // descriptor of stage 0, slice 0
             for (int t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x) {
                 if (!live(t)) continue;
                 const int buf = tc_n & 1, use = tc_n >> 1;
@@ -356,8 +308,8 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
                     for (int a = 0; a < OZ_S; ++a) {
                         if (a >= OZ_S - b0) break;
                         const int n = min(b1, OZ_S - 1 - a) - b0 + 1;
-                        mma_bf16(dbase + (uint32_t)((a + b0) * BN), dst + (uint64_t)((a * OZ_A_SLICE) >> 4), db,
-                                 idesc_bf16(OZ_BM, n * BN), (i == 1 && a == 0) ? 0u : 1u);
+                        tc::mma_bf16(dbase + (uint32_t)((a + b0) * BN), dst + (uint64_t)((a * OZ_A_SLICE) >> 4), db,
+                                 tc::idesc_bf16(OZ_BM, n * BN), (i == 1 && a == 0) ? 0u : 1u);
                     }
                     tc::mma_commit(&bar_empty[s]);
                 }

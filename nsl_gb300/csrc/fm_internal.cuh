@@ -38,6 +38,13 @@ struct OzPlanes {
     int ld = 0;
 };
 
+// Double-double digit planes of a real exp(d K) (fm_apply_ddtc.cu): its FP64 entries in twelve digits.
+struct DdPlanes {
+    void *planes = nullptr;  // BF16
+    int *col_exp = nullptr;  // (Nx)
+    int *klist = nullptr;    // per tile of output sites: k-blocks, digits present, ends of exact segments
+};
+
 // exp(d K) memo entry (SpatialLattice::exp_hopping_matrix, lattice.tpp:52-58), kept in the layouts the kernels read.
 struct ExpEntry {
     double2 *full = nullptr;  // complex (Nx, Nx) row-major
@@ -50,6 +57,7 @@ struct ExpEntry {
     bool is_real = true;
     TcPlanes *tc = nullptr;   // built on first tensor-core use
     OzPlanes *oz = nullptr;   // built on first split-BF16 use
+    DdPlanes *dd = nullptr;   // built on first double-double tensor-core use
 };
 
 // Operator-arithmetic tags for the tensor-core operators (3xTF32; split BF16 with exact accumulation).
@@ -219,6 +227,11 @@ int cg_solve_group(int nfm, nslg_fm *const *fms, int op, const double2 *const *b
 // only the rows of systems s (sys_rows rows each) with sys_mask[s] != 0 are written.
 int fm_apply_dd(nslg_fm *fm, int op, const double2 *xh, const double2 *xl, double2 *oh, double2 *ol, int64_t nbatch,
                 const int *sys_mask, int64_t sys_rows);
+// Its tensor-core form (fm_apply_ddtc.cu) for one factor with a real exp(d K): whether it applies to this size, and one M
+// or M^dagger application.
+bool ddtc_applies(const ExpEntry *e, int Nx, int64_t rows);
+int fm_apply_ddtc(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *xh, const double2 *xl, double2 *oh,
+                  double2 *ol, int64_t rows, const int *sys_mask, int64_t sys_rows);
 // Stratified (UDT) log det and gradient (stable.cu): whether the handle uses them, and the batched forms over nmat
 // matrices with factors Ep[g] = exp(-sgn_g delta K), E[g] = exp(sgn_g delta K) and phase rows ph / pinv
 // (nmat, Nt, Nx).

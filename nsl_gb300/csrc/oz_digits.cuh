@@ -60,6 +60,25 @@ __device__ __forceinline__ int scale_exponent(unsigned long long maxbits) {
     return maxbits == 0 ? 0 : (int)(maxbits >> 52) - 1022;
 }
 
+// zint 2^e as an FP64 value (rounded to nearest, ties away from zero) from integer operations only: GB300 runs an
+// integer -> FP64 conversion and the scaling multiply on its FP64 pipe, ~2 operations per clock per SM.
+__device__ __forceinline__ double scaled_to_double(long long zint, int e) {
+    if (zint == 0) return 0.0;
+    const unsigned long long sign = zint < 0 ? (1ull << 63) : 0ull;
+    unsigned long long u = zint < 0 ? 0ull - (unsigned long long)zint : (unsigned long long)zint;
+    const int lz = __clzll((long long)u);
+    u <<= lz;                                                 // leading one at bit 63: |zint| = u 2^-lz
+    unsigned long long m = (u >> 11) + ((u >> 10) & 1ull);    // 53 significant bits, rounded
+    int ex = e + 63 - lz;                                     // |zint| 2^e = (m / 2^52) 2^ex
+    if (m >> 53) {                                            // the rounding carried into a 54th bit
+        m >>= 1;
+        ++ex;
+    }
+    if (ex < -1022) return __longlong_as_double((long long)sign);                         // below the normal range: 0
+    if (ex > 1023) return __longlong_as_double((long long)(sign | 0x7FF0000000000000ull));  // above it: infinity
+    return __longlong_as_double((long long)(sign | ((unsigned long long)(ex + 1023) << 52) | (m & 0xFFFFFFFFFFFFFull)));
+}
+
 // Digit planes in memory: the operand of the tensor-core kernel, already in the layout of its shared-memory stages, so
 // that a k-block's digits of a tile are one contiguous bulk copy (a 2-D tensor copy of 32-byte rows costs the copy engine
 // about a cycle per row, which bounded the kernel). GEMM rows are grouped by `tile` (128 for the operand, 32 for

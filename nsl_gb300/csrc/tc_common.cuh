@@ -170,6 +170,35 @@ __device__ __forceinline__ uint64_t sdesc_kmajor_sw128(uint32_t saddr) {
     return d;
 }
 
+// Shared-memory matrix descriptor: K-major operand rows of 32 B, 32-byte swizzle, 8-row core groups 256 B apart.
+__device__ __forceinline__ uint64_t sdesc_kmajor_sw32(uint32_t saddr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((saddr >> 4) & 0x3FFF);
+    d |= (uint64_t)1 << 16;           // leading byte offset (unused for swizzled K-major)
+    d |= (uint64_t)(256 >> 4) << 32;  // stride byte offset: 8 rows x 32 B
+    d |= (uint64_t)1 << 46;           // descriptor version (sm_100)
+    d |= (uint64_t)6 << 61;           // layout: SWIZZLE_32B
+    return d;
+}
+
+__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
+    return (1u << 4)     // D: F32
+           | (1u << 7)   // A: BF16
+           | (1u << 10)  // B: BF16
+           | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// D[tmem] (+)= A[smem] * B[smem]^T, kind::f16 (BF16 operands, FP32 accumulation), issued by one thread.
+// (The A collector buffer does not change the instruction rate measured on this part, ~44 cycles per N = 32 MMA.)
+__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                         uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n" ::"r"(
+            d_tmem),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+
 // Instruction descriptor, kind::tf32 with FP32 accumulation, both operands K-major.
 __host__ __device__ constexpr uint32_t idesc_tf32(int M, int N) {
     return (1u << 4)                      // D format: F32

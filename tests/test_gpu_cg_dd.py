@@ -139,3 +139,46 @@ def test_dd_solve_plain_fp64_configuration_1e10():
     assert cg.stats["converged"] == 2, cg.stats
     res = _dd_residuals(ho, "MMdagger", b, x, np.asarray(cg.x_lo_))
     assert res.max() <= eps * 1.01, (res, eps)
+
+
+@pytest.mark.parametrize("L,Nt,R", [((3, 3), 16, 15), (33, 9, 14), ((5, 5), 7, 12), (64, 64, 1), ((6, 11), 3, 11), ((12, 12), 5, 3),
+                                    (1, 64, 64), (17, 1, 256)])
+@pytest.mark.parametrize("op", ["M", "Mdagger", "MMdagger", "MdaggerM"])
+def test_apply_dd_tensor_core_sizes(L, Nt, R, op):
+    """The tensor-core form of the double-double operator (vectors of 4096 elements and more) at ragged tiles (sites of
+    1 to 288, rows that do not fill a tile, one slice), rows of very different size, against the oracle's: 1e-28 of the
+    result's size per row, as test_apply_dd_against_oracle."""
+    import nsl_gb300 as N
+
+    lat = N.Honeycomb(L) if isinstance(L, tuple) else N.Ring(L)
+    Nx = lat.sites()
+    rng = np.random.default_rng(Nx + Nt)
+    phi = rng.standard_normal((Nt, Nx)) * 0.8 + 0j
+    h = N.HubbardExp(lat, Nt, 0.125 * Nt)
+    h.populate(phi)
+    ho = _same_operator(h, phi)
+    xh = (rng.standard_normal((R, Nt, Nx)) + 1j * rng.standard_normal((R, Nt, Nx))) * np.exp(rng.uniform(-20, 20, (R, 1, 1)))
+    xl = xh * 1e-17 * rng.standard_normal(xh.shape)
+    gh, gl = h.apply_dd(getattr(N.MatrixCombination, op), xh, xl)
+    oh, ol = O.apply_dd(ho, op, xh, xl)
+    d = (np.asarray(gh) - oh) + (np.asarray(gl) - ol)
+    size = np.abs(oh).max(axis=(1, 2), keepdims=True)
+    assert np.all(np.abs(d) <= 1e-28 * size), (np.abs(d) / size).max()
+
+
+def test_apply_dd_reports_non_finite_rows():
+    """A NaN or an infinity in a row of the operand reaches the rows that read it, and no others."""
+    import nsl_gb300 as N
+
+    Nt, Nx, R = 16, 18, 16
+    h = N.HubbardExp(N.Honeycomb((3, 3)), Nt, 2.0)
+    rng = np.random.default_rng(3)
+    h.populate(rng.standard_normal((Nt, Nx)) + 0j)
+    x = rng.standard_normal((R, Nt, Nx)) + 0j
+    x[2, 5, 7] = np.nan
+    x[9, 15, 0] = np.inf
+    gh, _ = h.apply_dd(N.MatrixCombination.M, x)
+    bad = ~np.isfinite(np.asarray(gh)).all(axis=2)
+    want = np.zeros((R, Nt), dtype=bool)
+    want[2, 5] = want[2, 6] = want[9, 15] = want[9, 0] = True
+    assert np.array_equal(bad, want)
