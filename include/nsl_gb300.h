@@ -148,6 +148,12 @@ NSLG_API int nslg_fm_get_phases(nslg_fm *fm, nslg_c128 *out);
 NSLG_API int nslg_fm_apply(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch,
                            int precision);
 
+/* nslg_fm_apply ordered with another stream of the caller's (a cudaStream_t): the application starts after the work
+ * queued on `stream` so far, and work queued there later starts after it. Saves a caller with device buffers on its own
+ * stream two event objects per call. No counterpart in the reference. */
+NSLG_API int nslg_fm_apply_on(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch,
+                              int precision, void *stream);
+
 /* op applied in double-double arithmetic (~1e-30 relative to |op| |psi|): (out_hi + out_lo) = op (psi_hi + psi_lo)
  * with the handle's FP64 exp(delta K) and phases, the residual evaluation of NSLG_STOP_TRUE_RESIDUAL_DD. psi_lo may
  * be NULL (zero). Exponential discretisation only; buffers (nbatch, Nt, Nx), host or device, the outputs not

@@ -70,6 +70,7 @@ SIGNATURES = {
     "nslg_fm_populate": (C.c_int, [_P, _P, C.c_int]),
     "nslg_fm_get_phases": (C.c_int, [_P, _P]),
     "nslg_fm_apply": (C.c_int, [_P, C.c_int, _P, _P, _I64, C.c_int]),
+    "nslg_fm_apply_on": (C.c_int, [_P, C.c_int, _P, _P, _I64, C.c_int, _P]),
     "nslg_fm_apply_noalloc": (C.c_int, [_P, C.c_int, _P, _P, _I64, C.c_int]),
     "nslg_fm_apply_dd": (C.c_int, [_P, C.c_int, _P, _P, _P, _P, _I64]),
     "nslg_fm_set_force_precision": (C.c_int, [_P, C.c_int]),

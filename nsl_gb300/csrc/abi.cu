@@ -125,9 +125,14 @@ void note_launch(cudaStream_t st, uint64_t n) {
 uint64_t launches() { return g_launches.load(); }
 
 int num_sms() {
+    static std::atomic<int> known[64] = {};  // per device ordinal (0: not looked up yet)
     int dev = 0, n = 0;
     cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+    if (dev >= 0 && dev < 64) n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        if (dev >= 0 && dev < 64) known[dev].store(n, std::memory_order_relaxed);
+    }
     return n;
 }
 
@@ -209,7 +214,7 @@ int apply_one(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *in, doubl
 
 template <typename T>
 int fm_apply_dev(nslg_fm *fm, int op, const double2 *psi, double2 *out, int64_t nbatch, const int *mask,
-                 int64_t sys_rows) {
+                 int64_t sys_rows, double2 *half) {
     NSLG_REQUIRE(fm->populated, NSLG_ERR_STATE, "the fermion matrix has no configuration (call populate first)");
     const double2 d = make_double2(fm->sgn * fm->delta.x, fm->sgn * fm->delta.y);
     const double2 dc = make_double2(fm->sgn * fm->delta.x, -fm->sgn * fm->delta.y);
@@ -222,8 +227,8 @@ int fm_apply_dev(nslg_fm *fm, int op, const double2 *psi, double2 *out, int64_t 
         case NSLG_OP_MDAGGER: return apply_one<T>(fm, MODE_MDAG, Ec, psi, out, rows, mask, sys_rows);
         default: break;
     }
-    double2 *tmp;
-    NSLG_TRY(ws_get(fm, "apply_tmp", rows * fm->Nx, &tmp));
+    double2 *tmp = half;
+    if (!tmp) NSLG_TRY(ws_get(fm, "apply_tmp", rows * fm->Nx, &tmp));
     if (op == NSLG_OP_MMDAGGER) {  // M (M^dagger psi)
         NSLG_TRY(apply_one<T>(fm, MODE_MDAG, Ec, psi, tmp, rows, mask, sys_rows));
         return apply_one<T>(fm, MODE_M, E, tmp, out, rows, mask, sys_rows);
@@ -233,10 +238,10 @@ int fm_apply_dev(nslg_fm *fm, int op, const double2 *psi, double2 *out, int64_t 
     return apply_one<T>(fm, MODE_MDAG, Ec, tmp, out, rows, mask, sys_rows);
 }
 
-template int fm_apply_dev<double>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t);
-template int fm_apply_dev<float>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t);
-template int fm_apply_dev<TF32x3>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t);
-template int fm_apply_dev<BF16Split>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t);
+template int fm_apply_dev<double>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t, double2 *);
+template int fm_apply_dev<float>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t, double2 *);
+template int fm_apply_dev<TF32x3>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t, double2 *);
+template int fm_apply_dev<BF16Split>(nslg_fm *, int, const double2 *, double2 *, int64_t, const int *, int64_t, double2 *);
 
 // Reports (and clears) a timeout recorded by a tensor-core kernel's bounded waits.
 int check_tc_error(nslg_fm *fm) {
@@ -400,6 +405,8 @@ NSLG_API int nslg_fm_destroy(nslg_fm *fm) {
     }
     if (fm->ev_fork) cudaEventDestroy(fm->ev_fork);
     if (fm->ev_join) cudaEventDestroy(fm->ev_join);
+    if (fm->ev_in) cudaEventDestroy(fm->ev_in);
+    if (fm->ev_out) cudaEventDestroy(fm->ev_out);
     for (auto &kv : fm->ws) cudaFree(kv.second.p);
     cudaFree(fm->hops);
     cudaFree(fm->phi);
@@ -500,6 +507,21 @@ NSLG_API int nslg_fm_apply(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 
     // device-buffer calls stay asynchronous: a tensor-core pipeline timeout is reported by the next call on this
     // handle that synchronises
     return NSLG_OK;
+}
+
+NSLG_API int nslg_fm_apply_on(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch,
+                              int precision, void *stream) {
+    NSLG_TRY(check_fm(fm));
+    cudaStream_t other = static_cast<cudaStream_t>(stream), st = fm->ctx->stream;
+    if (other == st) return nslg_fm_apply(fm, op, psi, out, nbatch, precision);
+    if (!fm->ev_in) NSLG_CUDA(cudaEventCreateWithFlags(&fm->ev_in, cudaEventDisableTiming));
+    if (!fm->ev_out) NSLG_CUDA(cudaEventCreateWithFlags(&fm->ev_out, cudaEventDisableTiming));
+    NSLG_CUDA(cudaEventRecord(fm->ev_in, other));
+    NSLG_CUDA(cudaStreamWaitEvent(st, fm->ev_in, 0));
+    const int rc = nslg_fm_apply(fm, op, psi, out, nbatch, precision);
+    NSLG_CUDA(cudaEventRecord(fm->ev_out, st));  // also after an error: work may have been queued
+    NSLG_CUDA(cudaStreamWaitEvent(other, fm->ev_out, 0));
+    return rc;
 }
 
 NSLG_API int nslg_fm_apply_dd(nslg_fm *fm, int op, const nslg_c128 *psi_hi, const nslg_c128 *psi_lo,

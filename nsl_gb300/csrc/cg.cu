@@ -150,7 +150,8 @@ struct Sys {
     }
 };
 
-// partial[s, blk] = sum conj(a) b over the block's chunk of system s
+// partial[s, blk] = sum conj(a) b over the block's chunk of system s (NORM: b = a, the real |a|^2: half the FP64 work)
+template <bool NORM>
 __global__ void __launch_bounds__(RT) k_dot(const double2 *__restrict__ a, const double2 *__restrict__ b, Sys sy,
                                             int nblk, double2 *__restrict__ partial, const CgState *__restrict__ st) {
     const int s = blockIdx.y, blk = blockIdx.x;
@@ -162,15 +163,22 @@ __global__ void __launch_bounds__(RT) k_dot(const double2 *__restrict__ a, const
     b += o;
     double2 acc = make_double2(0, 0);
     for (int64_t i = lo + threadIdx.x; i < hi; i += RT) {
-        const double2 x = a[i], y = b[i];
-        acc.x += x.x * y.x + x.y * y.y;
-        acc.y += x.x * y.y - x.y * y.x;
+        const double2 x = a[i];
+        if (NORM) {
+            acc.x = fma(x.x, x.x, fma(x.y, x.y, acc.x));
+        } else {
+            const double2 y = b[i];
+            acc.x += x.x * y.x + x.y * y.y;
+            acc.y += x.x * y.y - x.y * y.x;
+        }
     }
-    acc = block_sum2(acc);
+    if (NORM) acc.x = block_sum(acc.x);
+    else acc = block_sum2(acc);
     if (threadIdx.x == 0) partial[(int64_t)s * nblk + blk] = acc;
 }
 
-// alpha = rsq / <p, t>;  x += alpha p;  r -= alpha t;  partial |r|^2
+// alpha = rsq / <p, t>;  x += alpha p;  r -= alpha t;  partial |r|^2  (REAL: the curvature, and so alpha, is real)
+template <bool REAL>
 __global__ void __launch_bounds__(RT) k_cg_xr(double2 *__restrict__ x, double2 *__restrict__ r,
                                               const double2 *__restrict__ p, const double2 *__restrict__ t, Sys sy,
                                               int nblk, const double2 *__restrict__ p_pt,
@@ -182,8 +190,12 @@ __global__ void __launch_bounds__(RT) k_cg_xr(double2 *__restrict__ x, double2 *
     if (threadIdx.x < 32) {
         const double2 pt = warp0_sum_partials2(p_pt + (int64_t)s * nblk, nblk);
         if (threadIdx.x == 0) {
-            const double den = pt.x * pt.x + pt.y * pt.y;
-            alpha = make_double2(S.rsq * pt.x / den, -S.rsq * pt.y / den);
+            if (REAL) {
+                alpha = make_double2(S.rsq / pt.x, 0.0);
+            } else {
+                const double den = pt.x * pt.x + pt.y * pt.y;
+                alpha = make_double2(S.rsq * pt.x / den, -S.rsq * pt.y / den);
+            }
         }
     }
     __syncthreads();
@@ -195,10 +207,17 @@ __global__ void __launch_bounds__(RT) k_cg_xr(double2 *__restrict__ x, double2 *
     for (int64_t i = off + lo + threadIdx.x; i < off + hi; i += RT) {
         const double2 pv = p[i], tv = t[i];
         double2 xv = x[i], rv = r[i];
-        xv.x += ar * pv.x - ai * pv.y;
-        xv.y += ar * pv.y + ai * pv.x;
-        rv.x -= ar * tv.x - ai * tv.y;
-        rv.y -= ar * tv.y + ai * tv.x;
+        if (REAL) {
+            xv.x = fma(ar, pv.x, xv.x);
+            xv.y = fma(ar, pv.y, xv.y);
+            rv.x = fma(-ar, tv.x, rv.x);
+            rv.y = fma(-ar, tv.y, rv.y);
+        } else {
+            xv.x += ar * pv.x - ai * pv.y;
+            xv.y += ar * pv.y + ai * pv.x;
+            rv.x -= ar * tv.x - ai * tv.y;
+            rv.y -= ar * tv.y + ai * tv.x;
+        }
         x[i] = xv;
         r[i] = rv;
         acc += rv.x * rv.x + rv.y * rv.y;
@@ -697,6 +716,7 @@ struct CgRun {
     int64_t max_iter;
     int reliable;
     const double2 *half = nullptr;  // M^dagger p (MMdag) or M p (MdagM): the operator's intermediate vector
+    double2 *packed_half = nullptr; // a group's: where the applications of all instances put it (half points there)
     // fused split-BF16 iteration (MMdag / MdagM on the tensor cores): the CG dot products and updates run in the
     // operator's epilogues
     bool fused = false;
@@ -739,7 +759,7 @@ template <typename T> int apply_all(CgRun &R, const double2 *in, double2 *out, c
     for (auto &I : R.inst)
         if (!(R.skip_idle && I.idle))
             NSLG_TRY(fm_apply_dev<T>(I.fm, R.op, in + I.voff, out + I.voff, I.nbatch, flags ? flags + I.s0 : nullptr,
-                                     I.rows_per_sys));
+                                     I.rows_per_sys, R.packed_half ? R.packed_half + I.voff : nullptr));
     return NSLG_OK;
 }
 // op in double-double on the packed pairs, only for the flagged systems when flags is given.
@@ -821,10 +841,14 @@ template <typename Top> int cg_iteration(CgRun &R, CgState *st_a, CgState *st_b,
     dim3 grid(R.P.nblk, (unsigned)R.P.nsys);
     // <p, A p>; for A = M M^dagger (M^dagger M) in the mixed forms as |M^dagger p|^2 (|M p|^2), equal in exact
     // arithmetic but positive by construction when the two factors carry independent rounding
-    if (R.half) k_dot<<<grid, RT, 0, st>>>(R.half, R.half, R.P.sy, R.P.nblk, R.p_pt, st_a);
-    else k_dot<<<grid, RT, 0, st>>>(R.v.p, R.v.t, R.P.sy, R.P.nblk, R.p_pt, st_a);
+    if (R.half) {
+        k_dot<true><<<grid, RT, 0, st>>>(R.half, R.half, R.P.sy, R.P.nblk, R.p_pt, st_a);
+        k_cg_xr<true><<<grid, RT, 0, st>>>(R.v.x, R.v.r, R.v.p, R.v.t, R.P.sy, R.P.nblk, R.p_pt, st_a, R.p_rr);
+    } else {
+        k_dot<false><<<grid, RT, 0, st>>>(R.v.p, R.v.t, R.P.sy, R.P.nblk, R.p_pt, st_a);
+        k_cg_xr<false><<<grid, RT, 0, st>>>(R.v.x, R.v.r, R.v.p, R.v.t, R.P.sy, R.P.nblk, R.p_pt, st_a, R.p_rr);
+    }
     note_launch(st);
-    k_cg_xr<<<grid, RT, 0, st>>>(R.v.x, R.v.r, R.v.p, R.v.t, R.P.sy, R.P.nblk, R.p_pt, st_a, R.p_rr);
     note_launch(st);
     // FP32-class operators also force an update every UPDATE_EVERY iterations (stall detection, mode 2)
     constexpr bool fp32_class = std::is_same_v<Top, float> || std::is_same_v<Top, TF32x3>;
@@ -1195,6 +1219,11 @@ int cg_run(CgRun &R, const double2 *b, const double2 *x0, double2 *x, double2 *x
         double2 *h;
         NSLG_TRY(ws_get(fm, "apply_tmp", total, &h));  // the buffer the two-factor applications write first
         R.half = h;
+    }
+    if (!single_matrix && !all_resident && R.reliable && precision != NSLG_PREC_FP64 &&
+        (op == NSLG_OP_MMDAGGER || op == NSLG_OP_MDAGGERM)) {
+        NSLG_TRY(ws_get(fm, "cg_half", total, &R.packed_half));
+        R.half = R.packed_half;
     }
     if (single && precision == NSLG_PREC_BF16_SPLIT && (op == NSLG_OP_MMDAGGER || op == NSLG_OP_MDAGGERM) &&
         fm->Nx <= 2048 && fm->kind == NSLG_FM_EXP) {

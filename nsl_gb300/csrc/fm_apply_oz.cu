@@ -126,12 +126,13 @@ __device__ __forceinline__ void operand_pair(const double2 *__restrict__ psi, co
 
 // One warp per complex row (r, t): scales e (max |Y| < 2^e, real and imaginary GEMM rows separately) and the digit
 // planes A[l][2 row + c][y] (ld sites, zero padded). Lanes take site pairs (4-byte BF16 stores).
-template <int MODE>
-__global__ void __launch_bounds__(256, 2)
+// NP: site pairs a lane keeps in registers (rows of <= 64 NP sites); short rows take the small variant, whose registers
+// let twice the warps in (their loads' latency is what bounds it: 20 -> 9 us at 4608 rows of 72 sites).
+template <int MODE, int NP>
+__global__ void __launch_bounds__(256, NP <= 2 ? 4 : 2)
     k_oz_digits(const double2 *__restrict__ psi, const double2 *__restrict__ phase, int Nt, int Nx, int64_t rows,
                 int ld, __nv_bfloat16 *__restrict__ planes, int *__restrict__ ex, const int *__restrict__ go,
                 int64_t sys_rows) {
-    constexpr int NP = OZ_CACHE / 2;  // site pairs a lane keeps in registers (rows of <= 64 * NP sites)
     const int64_t grow = (int64_t)blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32;
     const int lane = threadIdx.x % 32;
     if (grow >= rows) return;
@@ -630,6 +631,17 @@ int oz_planes(nslg_fm *fm, const ExpEntry *e, OzPlanes **out) {
 // digits: workspace of S * 2 * rows * ld BF16; rexp: 2 * rows ints.
 namespace {
 
+template <int MODE>
+int launch_digits(const double2 *psi, const double2 *phase, int Nt, int Nx, int64_t rows, int ld, __nv_bfloat16 *planes,
+                  int *ex, const int *go, int64_t sys_rows, cudaStream_t st) {
+    const unsigned blocks = (unsigned)ceil_div(rows, 8);
+    if (Nx <= 128) k_oz_digits<MODE, 2><<<blocks, 256, 0, st>>>(psi, phase, Nt, Nx, rows, ld, planes, ex, go, sys_rows);
+    else k_oz_digits<MODE, OZ_CACHE / 2><<<blocks, 256, 0, st>>>(psi, phase, Nt, Nx, rows, ld, planes, ex, go, sys_rows);
+    note_launch(st);
+    NSLG_CUDA(cudaGetLastError());
+    return NSLG_OK;
+}
+
 template <int EPI>
 void launch_oz(int mode, dim3 grid, cudaStream_t st, const double2 *psi, double2 *out, const double2 *phase,
                const int *rexp, const int *col_exp, const int *klist, const uint8_t *dga, const uint8_t *dgb,
@@ -651,12 +663,9 @@ int oz_gemm(const double2 *Y, double2 *out, const double2 *pro_scale, const doub
             void *digits, int *rexp, int Nx, int64_t rows, int *err, cudaStream_t st) {
     if (rows == 0) return NSLG_OK;
     auto *dg = static_cast<__nv_bfloat16 *>(digits);
-    const unsigned blocks = (unsigned)ceil_div(rows, 8);
     // the operand's digits: Y o pro_scale (one row of Nx per column) or Y itself (one "time slice": Nt = 1)
-    if (pro_scale) k_oz_digits<MODE_M><<<blocks, 256, 0, st>>>(Y, pro_scale, 1, Nx, rows, P.ld, dg, rexp, nullptr, 1);
-    else k_oz_digits<MODE_MDAG><<<blocks, 256, 0, st>>>(Y, nullptr, 1, Nx, rows, P.ld, dg, rexp, nullptr, 1);
-    note_launch(st);
-    NSLG_CUDA(cudaGetLastError());
+    if (pro_scale) NSLG_TRY(launch_digits<MODE_M>(Y, pro_scale, 1, Nx, rows, P.ld, dg, rexp, nullptr, 1, st));
+    else NSLG_TRY(launch_digits<MODE_MDAG>(Y, nullptr, 1, Nx, rows, P.ld, dg, rexp, nullptr, 1, st));
     const auto *dga = static_cast<const uint8_t *>(digits), *dgb = static_cast<const uint8_t *>(P.planes);
     const int nkb = P.ld / OZ_BK;
     const OzEpi plain;
@@ -676,17 +685,14 @@ int fm_apply_oz(int mode, const double2 *psi, double2 *out, const double2 *phase
     NSLG_REQUIRE(E.mode != 2 || (E.sys_rows >= 1 && rows % E.sys_rows == 0), NSLG_ERR_ARG,
                  "split-BF16 CG epilogue: rows per system must divide the rows");
     auto *dg = static_cast<__nv_bfloat16 *>(digits);
-    const unsigned blocks = (unsigned)ceil_div(rows, 8);
     NSLG_REQUIRE(!E.go || (E.sys_rows >= 1 && rows % E.sys_rows == 0), NSLG_ERR_ARG,
                  "split-BF16 system skipping: rows per system must divide the rows");
     if (!E.digits_ready) {
         if (mode == MODE_M && !E.operand)
-            k_oz_digits<MODE_M><<<blocks, 256, 0, st>>>(psi, phase, Nt, Nx, rows, P.ld, dg, rexp, E.go, E.sys_rows);
+            NSLG_TRY(launch_digits<MODE_M>(psi, phase, Nt, Nx, rows, P.ld, dg, rexp, E.go, E.sys_rows, st));
         else  // M^dagger's operand is psi itself; a given operand is used as it is
-            k_oz_digits<MODE_MDAG><<<blocks, 256, 0, st>>>(E.operand ? E.operand : psi, nullptr, Nt, Nx, rows, P.ld,
-                                                           dg, rexp, E.go, E.sys_rows);
-        note_launch(st);
-        NSLG_CUDA(cudaGetLastError());
+            NSLG_TRY(launch_digits<MODE_MDAG>(E.operand ? E.operand : psi, nullptr, Nt, Nx, rows, P.ld, dg, rexp, E.go,
+                                              E.sys_rows, st));
     }
     const auto *dga = static_cast<const uint8_t *>(digits), *dgb = static_cast<const uint8_t *>(P.planes);
     const int nkb = P.ld / OZ_BK;

@@ -16,6 +16,12 @@
 // CTA tile: 128 real rows (64 complex rows) x BN sites, 256 threads, K in 32-site blocks through a 2-stage ring:
 // the threads build stage s+1 while the tensor core works on stage s. One thread issues the MMAs and commits them to
 // an mbarrier per stage. The accumulator (128 lanes x BN FP32 columns) is read back with tcgen05.ld by all 8 warps.
+//
+// What bounds it is not the product but the FP64 pipe (~2 operations per clock per SM) around it: rounding to FP32, the
+// remainders and the widening of the result are integer operations on the bit patterns (same bits), which leaves 6 FP64
+// operations per complex element (16 for M, 22 for M^dagger before). Measured, 144 right-hand sides at honeycomb 6x6,
+// Nt = 32 (72 CTAs of three k-blocks, mostly latency): 41 and 40 -> 36 and 39 us; 64 at 12x12, Nt = 64: 195 and
+// 157 -> 159 and 137 us.
 
 #include <cudaTypedefs.h>
 
@@ -55,6 +61,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 
     const int tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const int64_t grow0 = (int64_t)blockIdx.x * (TC_BM / 2);
+    const int t0 = (int)(grow0 % Nt);
     const int n0 = blockIdx.y * BN;
 
     if (tid == 0) {
@@ -101,11 +108,11 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             double2 v = make_double2(0.0, 0.0);
             if (grow < rows && y < Nx) {
                 v = psi[grow * Nx + y];
-                if (MODE == MODE_M) v = cmul(phase[(int64_t)(grow % Nt) * Nx + y], v);
+                if (MODE == MODE_M) v = cmul(phase[(int64_t)((t0 + j) % Nt) * Nx + y], v);
             }
             float hr, lr, hi_, li;
-            tc::split_tf32(v.x, hr, lr);
-            tc::split_tf32(v.y, hi_, li);
+            tc::split_tf32_int(v.x, hr, lr);
+            tc::split_tf32_int(v.y, hi_, li);
             const uint32_t o_re = tc::sw128_offset(2 * j, k), o_im = tc::sw128_offset(2 * j + 1, k);
             *reinterpret_cast<float *>(a_hi + o_re) = hr;
             *reinterpret_cast<float *>(a_lo + o_re) = lr;
@@ -175,12 +182,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             const float partner = __shfl_xor_sync(0xffffffffu, v[i], 1);
             const int x = n0 + c0 + i;
             if (!ready || grow >= rows || x >= Nx) continue;
-            double z = (double)v[i];
+            double z = tc::widen_int(v[i]);
             if (MODE == MODE_MDAG) {
-                const double zr = comp ? (double)partner : z, zi = comp ? z : (double)partner;
+                // conj(ph) (zr + i zi): ph.x zr + ph.y zi in the real lane, ph.x zi - ph.y zr in the imaginary one
+                const double w = tc::widen_int(comp ? -partner : partner);
                 const double2 ph = phase[(int64_t)to * Nx + x];
-                // conj(ph) * (zr + i zi)
-                z = comp ? (ph.x * zi - ph.y * zr) : (ph.x * zr + ph.y * zi);
+                z = fma(ph.x, z, ph.y * w);
             }
             const int64_t e = (orow + x) * 2 + comp;
             outd[e] = psid[e] - sgn * z;

@@ -106,6 +106,7 @@ struct nslg_fm {
     // from and joined back to ctx->stream with the two events; created on first use
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+    cudaEvent_t ev_in = nullptr, ev_out = nullptr;  // orders ctx->stream after and before a caller's stream
     std::map<std::string, nslg::DevBuf> ws;
     uint64_t ws_generation = 0;  // bumped whenever a workspace buffer moves (invalidates captured graphs)
     std::map<std::string, cudaGraphExec_t> graphs;
@@ -163,10 +164,10 @@ int fm_apply_simt(int mode, const double2 *psi, double2 *out, const cplx_t<T> *p
 
 // out = op(psi) for op in {M, Mdag, MMdag, MdagM} on FP64 device buffers (nbatch, Nt, Nx), products in T. sys_mask
 // (FP64 products only) restricts the work to the rows of flagged systems (sys_rows rows each); the other rows of
-// out are left unspecified.
+// out are left unspecified. half (optional) receives the first factor's result of the two-factor operators.
 template <typename T>
 int fm_apply_dev(nslg_fm *fm, int op, const double2 *psi, double2 *out, int64_t nbatch,
-                 const int *sys_mask = nullptr, int64_t sys_rows = 1);
+                 const int *sys_mask = nullptr, int64_t sys_rows = 1, double2 *half = nullptr);
 
 // One batched complex FP64 product, row-major: C = alpha (A o kscale) B, rows scaled by rscale, (+ I) (+ C). Matrices of
 // a two-level batch (z1, z2) lie at z1 s + z2 s2 elements; the scales alike.

@@ -221,5 +221,36 @@ __device__ __forceinline__ void split_tf32(double v, float &hi, float &lo) {
     lo = (float)(v - (double)hi);
 }
 
+// The same split in integer arithmetic (conversions and subtractions of FP64 numbers run on the FP64 pipe, ~2 per clock per
+// SM), bit for bit: hi is v rounded to FP32 with 13 mantissa bits cleared, lo = (float)(v - hi), v - hi being exact.
+__device__ __forceinline__ void split_tf32_int(double v, float &hi, float &lo) {
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v), a = b & 0x7FFFFFFFFFFFFFFFull;
+    const int e = (int)(a >> 52) - 1023;
+    if (a == 0ull) {
+        hi = lo = 0.f;
+        return;
+    }
+    if (e < -74 || e > 126) {  // hi or lo outside the normal range of FP32, infinities, NaN
+        split_tf32(v, hi, lo);
+        return;
+    }
+    const unsigned long long r = a + 0x0FFFFFFFull + ((a >> 29) & 1ull);  // round to nearest even at FP32's last bit
+    const unsigned h = ((unsigned)(r >> 29) - (896u << 23)) & 0xFFFFE000u;
+    const long long V = (long long)((a & 0xFFFFFFFFFFFFFull) | (1ull << 52));
+    const long long H = (long long)((h & 0x7FFFFFu) | 0x800000u) << (29 + (int)(h >> 23) - 127 - e);  // e, or e + 1 after a carry
+    const float l = __ll2float_rn(V - H) * __uint_as_float((unsigned)(e - 52 + 127) << 23);
+    const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
+    hi = __uint_as_float(h | sign);
+    lo = sign ? -l : l;
+}
+
+// (double)v in integer arithmetic for normal v.
+__device__ __forceinline__ double widen_int(float v) {
+    const unsigned u = __float_as_uint(v), e = u >> 23 & 0xFFu;
+    if (e == 0u || e == 255u) return (double)v;
+    return __longlong_as_double((long long)(((unsigned long long)(u & 0x80000000u) << 32) |
+                                            (((unsigned long long)(u & 0x7FFFFFFFu) + (896ull << 23)) << 29)));
+}
+
 }  // namespace tc
 }  // namespace nslg
