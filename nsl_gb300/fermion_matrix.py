@@ -131,9 +131,12 @@ class HubbardExp:
             raise ValueError(f"psi must have shape (..., Nt, Nx) = (..., {self.Nt}, {self.Nx}), got {shape}")
         nbatch = T.numel(shape[:-2])
         out = T.empty_like(psi)
-        with T.stream_order(self.ctx, psi, out):
-            _lib.check(_lib.load().nslg_fm_apply(self.handle, op, T.ptr(psi), T.ptr(out), nbatch,
-                                                 precision_code(precision)))
+        lib = _lib.load()
+        if T.is_cuda(psi):  # ordered with the caller's current torch stream inside the call
+            _lib.check(lib.nslg_fm_apply_on(self.handle, op, psi.data_ptr(), out.data_ptr(), nbatch,
+                                            precision_code(precision), T.current_stream_ptr(psi.device)))
+        else:
+            _lib.check(lib.nslg_fm_apply(self.handle, op, T.ptr(psi), T.ptr(out), nbatch, precision_code(precision)))
         return out
 
     def M(self, psi, precision="fp64"):

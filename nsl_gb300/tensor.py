@@ -54,6 +54,11 @@ def numel(shape) -> int:
     return n
 
 
+def current_stream_ptr(device) -> int:
+    """The cudaStream_t of the caller's current torch stream on `device`."""
+    return torch.cuda.current_stream(device).cuda_stream
+
+
 @contextlib.contextmanager
 def stream_order(ctx, *tensors):
     """Orders the library's stream after the caller's torch stream (and back) when CUDA tensors are involved."""
