@@ -17,11 +17,12 @@
 // the threads build stage s+1 while the tensor core works on stage s. One thread issues the MMAs and commits them to
 // an mbarrier per stage. The accumulator (128 lanes x BN FP32 columns) is read back with tcgen05.ld by all 8 warps.
 //
-// What bounds it is not the product but the FP64 pipe (~2 operations per clock per SM) around it: rounding to FP32, the
-// remainders and the widening of the result are integer operations on the bit patterns (same bits), which leaves 6 FP64
-// operations per complex element (16 for M, 22 for M^dagger before). Measured, 144 right-hand sides at honeycomb 6x6,
-// Nt = 32 (72 CTAs of three k-blocks, mostly latency): 41 and 40 -> 36 and 39 us; 64 at 12x12, Nt = 64: 195 and
-// 157 -> 159 and 137 us.
+// What bounds it is not the product but what surrounds it: the latency of the operand reads and the FP64 pipe (~2 operations
+// per clock per SM). All reads of a k-block are in flight at once, one k-block ahead; rounding to FP32, the remainders and
+// the widening of the result work on bit patterns (6 FP64 operations per complex element are left, 16 for M and 22 for
+// M^dagger before); the epilogue's lanes finish whole complex values. Measured, M and M^dagger on 144 right-hand sides at
+// honeycomb 6x6, Nt = 32: 43 and 43 -> 28 and 26 us; 64 at 12x12, Nt = 64: 195 and 157 -> 115 and 91 us; 8 at 24x24,
+// Nt = 128: 365 and 262 -> 208 and 149 us.
 
 #include <cudaTypedefs.h>
 
@@ -82,6 +83,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     const uint32_t tmem = *tmem_slot;
     constexpr uint32_t idesc = tc::idesc_tf32(TC_BM, BN);
 
+    // operand rows: 64 complex rows x 32 sites per k-block; a warp reads one 512-byte row segment per step. The next
+    // k-block's reads are issued before this one's MMAs, all eight rows at once.
+    double2 raw[8], fac[8];
+    auto fetch = [&](int kb) {
+        const int y = kb * TC_BK + lane;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int j = warp + 8 * i;  // complex row within the tile
+            const bool in = kb < nkb && grow0 + j < rows && y < Nx;
+            raw[i] = in ? psi[(grow0 + j) * Nx + y] : make_double2(0.0, 0.0);
+            if (MODE == MODE_M) fac[i] = in ? phase[(int64_t)((t0 + j) % Nt) * Nx + y] : make_double2(0.0, 0.0);
+        }
+    };
+    fetch(0);
     for (int kb = 0; kb < nkb; ++kb) {
         const int s = kb & 1;
         uint8_t *a_hi = smem + s * S::STAGE;
@@ -98,27 +113,20 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             tc::tma_load_2d(b_hi, &map_hi, kb * TC_BK, n0, &bar_load[s]);
             tc::tma_load_2d(b_lo, &map_lo, kb * TC_BK, n0, &bar_load[s]);
         }
-        // operand rows: 64 complex rows x 32 sites; a warp reads one 512-byte row segment per step
-        const int k = lane;
-        const int y = kb * TC_BK + k;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int j = warp + 8 * i;  // complex row within the tile
-            const int64_t grow = grow0 + j;
-            double2 v = make_double2(0.0, 0.0);
-            if (grow < rows && y < Nx) {
-                v = psi[grow * Nx + y];
-                if (MODE == MODE_M) v = cmul(phase[(int64_t)((t0 + j) % Nt) * Nx + y], v);
-            }
+            const int j = warp + 8 * i;
+            const double2 v = MODE == MODE_M ? cmul(fac[i], raw[i]) : raw[i];
             float hr, lr, hi_, li;
             tc::split_tf32_int(v.x, hr, lr);
             tc::split_tf32_int(v.y, hi_, li);
-            const uint32_t o_re = tc::sw128_offset(2 * j, k), o_im = tc::sw128_offset(2 * j + 1, k);
+            const uint32_t o_re = tc::sw128_offset(2 * j, lane), o_im = tc::sw128_offset(2 * j + 1, lane);
             *reinterpret_cast<float *>(a_hi + o_re) = hr;
             *reinterpret_cast<float *>(a_lo + o_re) = lr;
             *reinterpret_cast<float *>(a_hi + o_im) = hi_;
             *reinterpret_cast<float *>(a_lo + o_im) = li;
         }
+        fetch(kb + 1);
         tc::fence_proxy_async();
         __syncthreads();
         if (tid == 0) {
@@ -165,32 +173,34 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         sgn = (t == 0) ? -1.0 : 1.0;
     }
     const int64_t orow = (r * Nt + to) * Nx;
-    const double *psid = reinterpret_cast<const double *>(psi);
-    double *outd = reinterpret_cast<double *>(out);
     const uint32_t lane_addr = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-    constexpr int HALF = BN / 2;
-#pragma unroll 1
-    for (int q = 0; q < HALF / 16; ++q) {
-        const int c0 = (warp >> 2) * HALF + 16 * q;
-        float v[16];
-        if (ready) tc::tmem_ld16(lane_addr + c0, v);
+    const int ncols = min(BN, Nx - n0);
+    // eight columns at a time, dealt to the two warps of a lane quarter; the two lanes of a complex row swap halves, so that
+    // each finishes whole complex values at alternate sites (16-byte accesses, 32 contiguous bytes per row)
+    for (int c0 = 8 * (warp >> 2); c0 < ncols; c0 += 16) {
+        double2 pre[4], ph[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const int x = n0 + c0 + 2 * k + comp;
+            const bool use = ready && grow < rows && x < Nx;
+            pre[k] = use ? psi[orow + x] : make_double2(0.0, 0.0);
+            ph[k] = (MODE == MODE_MDAG && use) ? phase[(int64_t)to * Nx + x] : make_double2(0.0, 0.0);
+        }
+        float v[8];
+        if (ready) tc::tmem_ld8(lane_addr + c0, v);
         else
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = 0.f;
+            for (int i = 0; i < 8; ++i) v[i] = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-            const float partner = __shfl_xor_sync(0xffffffffu, v[i], 1);
-            const int x = n0 + c0 + i;
-            if (!ready || grow >= rows || x >= Nx) continue;
-            double z = tc::widen_int(v[i]);
-            if (MODE == MODE_MDAG) {
-                // conj(ph) (zr + i zi): ph.x zr + ph.y zi in the real lane, ph.x zi - ph.y zr in the imaginary one
-                const double w = tc::widen_int(comp ? -partner : partner);
-                const double2 ph = phase[(int64_t)to * Nx + x];
-                z = fma(ph.x, z, ph.y * w);
-            }
-            const int64_t e = (orow + x) * 2 + comp;
-            outd[e] = psid[e] - sgn * z;
+        for (int k = 0; k < 4; ++k) {
+            const float recv = __shfl_xor_sync(0xffffffffu, comp ? v[2 * k] : v[2 * k + 1], 1);
+            const double zr = tc::widen_int(comp ? recv : v[2 * k]), zi = tc::widen_int(comp ? v[2 * k + 1] : recv);
+            const int x = n0 + c0 + 2 * k + comp;
+            double2 z = make_double2(zr, zi);
+            if (MODE == MODE_MDAG)  // conj(ph) (zr + i zi)
+                z = make_double2(fma(ph[k].x, zr, ph[k].y * zi), fma(ph[k].x, zi, -(ph[k].y * zr)));
+            if (ready && grow < rows && x < Nx)
+                out[orow + x] = make_double2(fma(-sgn, z.x, pre[k].x), fma(-sgn, z.y, pre[k].y));
         }
     }
     tc::tc_fence_before();

@@ -221,27 +221,32 @@ __device__ __forceinline__ void split_tf32(double v, float &hi, float &lo) {
     lo = (float)(v - (double)hi);
 }
 
-// The same split in integer arithmetic (conversions and subtractions of FP64 numbers run on the FP64 pipe, ~2 per clock per
-// SM), bit for bit: hi is v rounded to FP32 with 13 mantissa bits cleared, lo = (float)(v - hi), v - hi being exact.
+// The same split without FP64 arithmetic (conversions and subtractions of FP64 numbers run on the FP64 pipe, ~2 per clock per
+// SM): f = v rounded to FP32 from the bit pattern, hi = f with 13 bits cleared, lo = (f - hi) + (v - f), the second term an
+// integer of 30 bits at a power-of-two scale. hi is the same bit for bit, lo to its last bit (the tensor core reads lo's
+// upper 11).
 __device__ __forceinline__ void split_tf32_int(double v, float &hi, float &lo) {
-    const unsigned long long b = (unsigned long long)__double_as_longlong(v), a = b & 0x7FFFFFFFFFFFFFFFull;
-    const int e = (int)(a >> 52) - 1023;
-    if (a == 0ull) {
+    const unsigned h32 = (unsigned)__double2hiint(v), l32 = (unsigned)__double2loint(v);
+    const int e = (int)(h32 >> 20 & 0x7FFu) - 896;  // FP32's biased exponent
+    if (((h32 << 1) | l32) == 0u) {  // zero (padding)
         hi = lo = 0.f;
         return;
     }
-    if (e < -74 || e > 126) {  // hi or lo outside the normal range of FP32, infinities, NaN
+    if (e < 53 || e > 253) {  // hi or lo outside the normal range of FP32, infinities, NaN
         split_tf32(v, hi, lo);
         return;
     }
-    const unsigned long long r = a + 0x0FFFFFFFull + ((a >> 29) & 1ull);  // round to nearest even at FP32's last bit
-    const unsigned h = ((unsigned)(r >> 29) - (896u << 23)) & 0xFFFFE000u;
-    const long long V = (long long)((a & 0xFFFFFFFFFFFFFull) | (1ull << 52));
-    const long long H = (long long)((h & 0x7FFFFFu) | 0x800000u) << (29 + (int)(h >> 23) - 127 - e);  // e, or e + 1 after a carry
-    const float l = __ll2float_rn(V - H) * __uint_as_float((unsigned)(e - 52 + 127) << 23);
-    const unsigned sign = (unsigned)(b >> 32) & 0x80000000u;
-    hi = __uint_as_float(h | sign);
-    lo = sign ? -l : l;
+    unsigned fb = __funnelshift_l(l32, h32 & 0x7FFFFFFFu, 3) - (896u << 23);  // truncated to 24 bits
+    int g = (int)(l32 & 0x1FFFFFFFu);                                          // what was cut off, units of ulp 2^-29
+    if (g > 0x10000000 || (g == 0x10000000 && (fb & 1u))) {                    // round to nearest even
+        ++fb;
+        g -= 0x20000000;
+    }
+    const unsigned hb = fb & 0xFFFFE000u, sign = h32 & 0x80000000u;
+    const float l = fmaf((float)g, __uint_as_float((unsigned)(e - 52) << 23),
+                         __uint_as_float(fb) - __uint_as_float(hb));
+    hi = __uint_as_float(hb | sign);
+    lo = __uint_as_float(__float_as_uint(l) ^ sign);
 }
 
 // (double)v in integer arithmetic for normal v.
