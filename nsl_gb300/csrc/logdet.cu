@@ -578,11 +578,12 @@ __global__ void k_perm_rows(double2 *B, const double2 *W, int n, const int *piv,
 // G[g] = (A_g + 1)^{-1} for small matrices (n <= GJ_MAX) in one launch: in-place Gauss-Jordan elimination with partial
 // pivoting in shared memory, one CTA per matrix. Rows are never swapped: column k's pivot is the largest entry among the
 // rows that have not been pivots yet (first row on ties, the same choice as an LU with row swaps makes up to the row
-// order), and the permutation is applied on the way out, inv[k, p_j] = W[p_k, j]. A step is one warp's pivot search
-// (integer comparisons of the FP64 bit patterns: an FP64 comparison costs a warp 64 cycles), the scaled pivot row, and
-// one update of all n^2 elements, which the FP64 pipe of one SM bounds (n^3 complex FMAs, 2 FP64 FMAs per clock).
-// Measured: 52 us -> 38 us at n = 18; panel factorisation, triangular solves and permutation of 32 matrices of n = 50
-// 690 us -> 293 us.
+// order), and the permutation is applied on the way out, inv[k, p_j] = W[p_k, j]. A step is the scaled pivot row and one
+// update of all n^2 elements, which the FP64 pipe of one SM bounds for large n (n^3 complex FMAs, 2 FP64 FMAs per clock);
+// beside it one warp looks ahead: it forms the next column, finds its pivot (integer comparisons of the FP64 bit patterns:
+// an FP64 comparison costs a warp 64 cycles) and the reciprocal, ~20 dependent FP64 operations that bound small n.
+// Measured: 52 us -> 32 us at n = 18 (38 without the look-ahead); panel factorisation, triangular solves and permutation of
+// 32 matrices of n = 50 690 us -> 254 us (293 without).
 constexpr int GJ_MAX = 64;
 constexpr int GJ_T = 512;
 constexpr int SCAN_MAX = 32;           // the small-lattice gradient uses scans up to this size
@@ -593,7 +594,7 @@ constexpr size_t gj_smem(int n) { return (size_t)n * (n + 1) * sizeof(double2); 
 __global__ void __launch_bounds__(GJ_T) k_gj_inverse(const double2 *__restrict__ A, int64_t astride,
                                                      double2 *__restrict__ G, int n, int *singular) {
     extern __shared__ double2 W[];  // n x (n + 1)
-    __shared__ double2 f[GJ_MAX], u[GJ_MAX];
+    __shared__ double2 f[GJ_MAX], u[GJ_MAX], next[GJ_MAX];
     __shared__ double2 inv_sh;
     __shared__ int pivot, piv[GJ_MAX];
     const int ld = n + 1, T = blockDim.x, tid = threadIdx.x;
@@ -607,75 +608,114 @@ __global__ void __launch_bounds__(GJ_T) k_gj_inverse(const double2 *__restrict__
         W[i * ld + j] = v;
     }
     __syncthreads();
-    const int di = T / n, dj = T - di * n;  // (i, j) steps of this thread's elements
-    const int i0 = tid / n, j0 = tid - i0 * n;
+    // warps 1 .. update all elements; warp 0 only looks ahead: it forms the next column, finds its pivot and the pivot's
+    // reciprocal (a chain of ~10 dependent FP64 steps) while they do
+    const int TB = T - 32, tb = tid - 32;
+    const int di = TB / n, dj = TB - di * n;  // (i, j) steps of this thread's elements
+    const int i0 = tb / n, j0 = tb - i0 * n;
     unsigned long long used = 0;  // rows that have been pivots (warp 0)
     int sing = 0;
-    for (int k = 0; k < n; ++k) {
-        if (tid < 32) {
-            unsigned long long bm = 0;
-            int bi = GJ_MAX;
-            for (int i = tid; i < n; i += 32) {
-                if (used >> i & 1) continue;
-                const double2 v = W[i * ld + k];
-                const unsigned long long m = (unsigned long long)__double_as_longlong(fma(v.x, v.x, v.y * v.y));
-                if (bi == GJ_MAX || m > bm) {
-                    bm = m;
-                    bi = i;
-                }
-            }
+    // pivot of column k among the unused rows, from the column's values c[0], c[1] at rows tid, tid + 32
+    auto choose = [&](int k, const double2 (&c)[2]) {
+        unsigned long long bm = 0;
+        int bi = GJ_MAX;
+        double2 bv = make_double2(0, 0);
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const unsigned long long om = __shfl_xor_sync(0xffffffffu, bm, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (oi < GJ_MAX && (bi == GJ_MAX || om > bm || (om == bm && oi < bi))) {
-                    bm = om;
-                    bi = oi;
-                }
-            }
-            used |= 1ull << bi;
-            if (tid == 0) {
-                const double2 d = W[bi * ld + k];
-                const double dd = d.x * d.x + d.y * d.y;
-                const double rdd = dd == 0.0 ? 0.0 : 1.0 / dd;
-                inv_sh = make_double2(d.x * rdd, -d.y * rdd);
-                pivot = bi;
-                piv[k] = bi;
-                if (dd == 0.0) sing = 1;
+        for (int h = 0; h < 2; ++h) {
+            const int i = tid + 32 * h;
+            if (i >= n || (used >> i & 1)) continue;
+            const unsigned long long m = (unsigned long long)__double_as_longlong(fma(c[h].x, c[h].x, c[h].y * c[h].y));
+            if (bi == GJ_MAX || m > bm) {
+                bm = m;
+                bi = i;
+                bv = c[h];
             }
         }
-        __syncthreads();
+        const int mine = bi;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const unsigned long long om = __shfl_xor_sync(0xffffffffu, bm, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
+            if (oi < GJ_MAX && (bi == GJ_MAX || om > bm || (om == bm && oi < bi))) {
+                bm = om;
+                bi = oi;
+            }
+        }
+        used |= 1ull << bi;
+        if (mine == bi) {  // the lane that holds the pivot
+            const double dd = __longlong_as_double((long long)bm);  // |bv|^2
+            const double rdd = dd == 0.0 ? 0.0 : 1.0 / dd;
+            inv_sh = make_double2(bv.x * rdd, -bv.y * rdd);
+            pivot = bi;
+            piv[k] = bi;
+            if (dd == 0.0) sing = 1;
+        }
+    };
+    if (tid < 32) {
+        const double2 c[2] = {tid < n ? W[tid * ld] : make_double2(0, 0),
+                              tid + 32 < n ? W[(tid + 32) * ld] : make_double2(0, 0)};
+        choose(0, c);
+    }
+    __syncthreads();
+    int last = -1;  // the previous pivot row
+    for (int k = 0; k < n; ++k) {
         const int p = pivot;
         const double2 inv = inv_sh;
         for (int j = tid; j < n; j += T) {
             u[j] = j == k ? inv : cmul(W[p * ld + j], inv);
-            f[j] = W[j * ld + k];
+            f[j] = (k == 0 || j == last) ? W[j * ld + k] : next[j];
         }
         __syncthreads();
-        for (int e = tid, i = i0, j = j0; e < n * n; e += T) {
-            const double2 uj = u[j];
-            double2 a = uj;
-            if (i != p) {
-                const double2 l = f[i];
-                a = j == k ? make_double2(0, 0) : W[i * ld + j];
-                a.x -= l.x * uj.x - l.y * uj.y;
-                a.y -= l.x * uj.y + l.y * uj.x;
+        if (tid < 32) {
+            if (k + 1 < n) {
+                const double2 uj = u[k + 1];
+                double2 c[2];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    const int i = tid + 32 * h;
+                    c[h] = make_double2(0, 0);
+                    if (i < n && i != p) {
+                        const double2 l = f[i];
+                        double2 a = W[i * ld + k + 1];
+                        a.x -= l.x * uj.x - l.y * uj.y;
+                        a.y -= l.x * uj.y + l.y * uj.x;
+                        c[h] = a;
+                        next[i] = a;  // column k + 1 as the next step's multipliers (W keeps its old values, unread)
+                    } else if (i == p) {
+                        c[h] = uj;
+                    }
+                }
+                choose(k + 1, c);
             }
-            W[i * ld + j] = a;
-            i += di;
-            j += dj;
-            if (j >= n) {
-                j -= n;
-                ++i;
+        } else {
+            for (int e = tb, i = i0, j = j0; e < n * n; e += TB) {
+                if (j != k + 1 || i == p) {  // (the rest of column k + 1 is warp 0's)
+                    const double2 uj = u[j];
+                    double2 a = uj;
+                    if (i != p) {
+                        const double2 l = f[i];
+                        a = j == k ? make_double2(0, 0) : W[i * ld + j];
+                        a.x -= l.x * uj.x - l.y * uj.y;
+                        a.y -= l.x * uj.y + l.y * uj.x;
+                    }
+                    W[i * ld + j] = a;
+                }
+                i += di;
+                j += dj;
+                if (j >= n) {
+                    j -= n;
+                    ++i;
+                }
             }
         }
         __syncthreads();
+        last = p;
     }
     for (int e = tid; e < n * n; e += T) {
         const int k = e / n, j = e - k * n;
         G[k * n + piv[j]] = W[piv[k] * ld + j];
     }
-    if (tid == 0 && sing) *singular = 1;
+    if (sing) *singular = 1;
 }
 
 // G[g] = (A_g + 1)^{-1} (astride elements apart, G dense), n <= GJ_MAX.
@@ -690,7 +730,7 @@ int gj_inverse_plus_one(nslg_fm *fm, const double2 *A, int64_t astride, double2 
             done.insert(fm->ctx->device);
         }
     }
-    k_gj_inverse<<<(unsigned)nmat, n <= 24 ? 352 : GJ_T, gj_smem(n), fm->ctx->stream>>>(A, astride, G, n, singular);
+    k_gj_inverse<<<(unsigned)nmat, n <= 18 ? 384 : GJ_T, gj_smem(n), fm->ctx->stream>>>(A, astride, G, n, singular);
     note_launch(fm->ctx->stream);
     NSLG_CUDA(cudaGetLastError());
     return NSLG_OK;
