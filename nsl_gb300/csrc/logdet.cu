@@ -985,10 +985,10 @@ __global__ void __launch_bounds__(256) k_diagprod_many(const double2 *__restrict
                                                        int Nt) {
     __shared__ double2 tile[32][33];
     __shared__ double2 red[8][32];
-    const int64_t gt = blockIdx.y;
+    const int64_t gt = blockIdx.x;
     const int g = (int)(gt / Nt), t = (int)(gt % Nt);
     const int lane = threadIdx.x % 32, w = threadIdx.x / 32;
-    const int x0 = blockIdx.x * 32, x = x0 + lane;
+    const int x0 = blockIdx.y * 32, x = x0 + lane;
     const int64_t nn = (int64_t)n * n;
     const double2 *Sm = S + ((int64_t)g * Nt + (t + 1) % Nt) * nn;
     const double2 *B = t == Nt - 1 ? G + (int64_t)g * nn : P + gt * nn;
@@ -1019,14 +1019,9 @@ __global__ void __launch_bounds__(256) k_diagprod_many(const double2 *__restrict
 
 int diagprod_many(cudaStream_t st, const double2 *S, const double2 *P, const double2 *G, double2 *out, int n, int Nt,
                   int nmat) {
-    const int64_t slices = (int64_t)nmat * Nt;
-    for (int64_t s0 = 0; s0 < slices; s0 += (int64_t)(65535 / Nt) * Nt) {  // whole matrices per launch (grid.y limit)
-        const int64_t cnt = std::min<int64_t>(slices - s0, (int64_t)(65535 / Nt) * Nt), g0 = s0 / Nt;
-        const int64_t nn = (int64_t)n * n;
-        k_diagprod_many<<<dim3((unsigned)ceil_div(n, 32), (unsigned)cnt), 256, 0, st>>>(
-            S + s0 * nn, P + s0 * nn, G + g0 * nn, out + s0 * n, n, Nt);
-        note_launch(st);
-    }
+    // (slices on grid.x: Nt alone may exceed grid.y's 65535)
+    k_diagprod_many<<<dim3((unsigned)((int64_t)nmat * Nt), (unsigned)ceil_div(n, 32)), 256, 0, st>>>(S, P, G, out, n, Nt);
+    note_launch(st);
     NSLG_CUDA(cudaGetLastError());
     return NSLG_OK;
 }

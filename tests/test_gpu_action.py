@@ -298,3 +298,18 @@ def test_gradient_and_log_det_forms_by_size(Nx, Nt, nconf):
         for b in range(nconf):
             qb, pb = Leapfrog(S, 0.1, 2)({"phi": phi[b]}, {"phi": p[b]})
             assert rel_err(q1["phi"][b], qb["phi"]) < 1e-10 and rel_err(p1["phi"][b], pb["phi"]) < 1e-10
+
+
+def test_gradient_at_the_longest_time_extent():
+    """Nt = 65536, one slice more than a grid's y extent holds. Unitary phases and beta |K| <= 2: the rounding of 65536
+    products of 2 x 2 matrices stays below 65536 * 4 eps * e^2 = 4.3e-10, on either side."""
+    import nsl_gb300 as N
+    from oracle import nsl_oracle as O
+
+    Nt, lat = 65536, N.Ring(2)
+    phi = np.random.default_rng(65536).standard_normal((Nt, 2)) * 0.005 + 0j
+    fm = N.HubbardExp(lat, Nt, 1.0)
+    fm.populate(phi, N.Species.Particle)
+    o = O.HubbardExp(lat.hopping_matrix(), Nt, 1.0, 0.0, O.PARTICLE)
+    o.populate(phi)
+    assert rel_err(fm.gradLogDetM(), o.gradLogDetM()) < 1e-9
