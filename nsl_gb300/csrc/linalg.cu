@@ -260,7 +260,9 @@ struct ZSplit {
     int CW, G, TM, threads, gx, gy;
 };
 
-ZSplit zsplit(int M, int N, int64_t nz) {
+size_t zsmem(int G, int TM, int K) { return (size_t)G * TM * (std::min(ZKC, K) + 1) * sizeof(double2); }
+
+ZSplit zsplit(int M, int N, int K, int64_t nz) {
     ZSplit S;
     if (N > ZMAXT) {  // a run of columns of one row group, all runs alike and a whole number of warps
         const int runs = (int)ceil_div(N, 128);
@@ -286,6 +288,7 @@ ZSplit zsplit(int M, int N, int64_t nz) {
     double best = 0;
     S.TM = 1;
     for (int TM = 8; TM >= 1; TM /= 2) {
+        if (TM > 1 && zsmem(S.G, TM, K) > 48 * 1024) continue;  // (one or two columns: many rows of A staged at once)
         const int64_t rb = ceil_div(M, (int64_t)S.G * TM);
         const int64_t warps = rb * S.gy * (S.threads / 32) * nz;
         const double eff = (double)warps / (double)(sched * ceil_div(warps, sched)) * (double)M / (double)(rb * S.G * TM);
@@ -301,7 +304,7 @@ ZSplit zsplit(int M, int N, int64_t nz) {
 
 template <int REAL, bool TA> void launch_zgemm(const ZSplit &S, unsigned nz, const ZProd &p, cudaStream_t st) {
     const dim3 grid((unsigned)S.gx, (unsigned)S.gy, nz);
-    const size_t smem = (size_t)S.G * S.TM * (std::min(ZKC, p.K) + 1) * sizeof(double2);  // <= 37 KB (G N <= 256)
+    const size_t smem = zsmem(S.G, S.TM, p.K);  // <= 48 KB
     if (S.TM == 8) k_zgemm<REAL, TA, 8><<<grid, S.threads, smem, st>>>(p, S.G, S.CW);
     else if (S.TM == 4) k_zgemm<REAL, TA, 4><<<grid, S.threads, smem, st>>>(p, S.G, S.CW);
     else if (S.TM == 2) k_zgemm<REAL, TA, 2><<<grid, S.threads, smem, st>>>(p, S.G, S.CW);
@@ -324,7 +327,7 @@ int zprod(cudaStream_t st, const ZProd &p, int batch) {
         NSLG_CUDA(cudaGetLastError());
         return NSLG_OK;
     }
-    const ZSplit S = zsplit(p.M, p.N, nz);
+    const ZSplit S = zsplit(p.M, p.N, p.K, nz);
     if (p.a_adjoint) launch_zgemm<0, true>(S, (unsigned)nz, p, st);
     else if (p.real == 1) launch_zgemm<1, false>(S, (unsigned)nz, p, st);
     else if (p.real == 2) launch_zgemm<2, false>(S, (unsigned)nz, p, st);
