@@ -1066,6 +1066,130 @@ ZProd factor_product(int n, const double2 *E0, const double2 *E1, int emask, boo
     return p;
 }
 
+// ---- whole chains in one launch --------------------------------------------------------------------------------------
+// The rows of P(t) = (P(t-1) D_t) E' and the columns of S(t) = D_t (E' S(t+1)) (and of the log det's product) are
+// independent through the whole chain, so a CTA takes V of them through all Nt steps: the vectors stay in shared memory
+// beside the real factor, one barrier per step, no launch per time slice. A thread owns one output of one vector and sums it in
+// ascending order whatever the split, so that a batch follows its single configurations bit by bit (and the products of
+// one launch per step). With 2 FP64 FMAs per clock per SM a step is bound by its FMAs once every SM
+// has some ten vectors, by the chain of one output's FMAs below.
+// Measured, 31 steps on 32 matrices of 50 sites: 777 us as one launch per step -> 515 us.
+//
+// FORM 0: rows of P, out[t] stored for t = 0 .. steps - 1, the scale of step t applied to the vector before the product.
+// FORM 1: columns of S, out[Nt - 2 - t] stored, the scale applied to the result. FORM 2: as 1 in increasing t, only the
+// last result stored, unscaled (the log det's product).
+constexpr int CH_T = 512;             // threads per CTA at most
+constexpr size_t CH_SMEM = 200 * 1024;
+
+struct ChainArgs {
+    const double2 *E0, *E1;  // the real factor of matrix g is (g & emask) ? E1 : E0
+    int emask;
+    const double2 *first;    // the starting matrices, sfirst elements apart
+    int64_t sfirst;
+    const double2 *ph;       // scale rows (Nt, n) per matrix
+    double2 *out;            // matrix g, step t at out + g * sout + t * n * n
+    int64_t sout;
+    int Nt, n, steps, V;
+};
+
+inline size_t chain_smem(int n, int V) { return (size_t)n * n * sizeof(double) + (size_t)2 * V * (n | 1) * sizeof(double2); }
+
+template <int FORM> __global__ void __launch_bounds__(CH_T) k_chain(ChainArgs A) {
+    extern __shared__ double2 sm[];
+    const int n = A.n, V = A.V, Nt = A.Nt;
+    const int L = n | 1;  // distance of the vectors: neighbouring ones in different banks
+    const int64_t nn = (int64_t)n * n;
+    double2 *Y = sm;                                              // two buffers of V vectors
+    double *E = reinterpret_cast<double *>(sm + 2 * V * L);       // E[k n + o]: factor from input k to output o
+    const int g = blockIdx.y, v0 = blockIdx.x * V, nv = min(V, n - v0);
+    const double2 *Eg = (g & A.emask) ? A.E1 : A.E0;
+    const double2 *first = A.first + g * A.sfirst, *ph = A.ph + (int64_t)g * Nt * n;
+    double2 *out = A.out + g * A.sout;
+    for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+        const int i = e / n, j = e - i * n;
+        E[FORM == 0 ? e : j * n + i] = Eg[e].x;  // rows: sum_k y_k E'[k, o]; columns: sum_k E'[o, k] y_k
+    }
+    // phase row of step t
+    auto row = [&](int t) -> const double2 * {
+        const int r = FORM == 0 ? t - 1 : FORM == 1 ? Nt - 3 - t : t + 3;
+        return ph + (int64_t)((r + Nt) % Nt) * n;
+    };
+    // element (vector v, index k) of a matrix: row v0 + v, column k, or column v0 + v, row k
+    auto at = [&](int v, int k) -> int64_t { return FORM == 0 ? (int64_t)(v0 + v) * n + k : (int64_t)k * n + v0 + v; };
+    for (int e = threadIdx.x; e < nv * n; e += blockDim.x) {
+        const int v = e / n, k = e - v * n;
+        double2 y = first[at(v, k)];
+        if (FORM == 0) y = cmul(y, row(0)[k]);
+        Y[v * L + k] = y;
+    }
+    __syncthreads();
+    for (int t = 0; t < A.steps; ++t) {
+        const double2 *cur = Y + (t & 1) * V * L;
+        double2 *nxt = Y + ((t + 1) & 1) * V * L;
+        const bool last = t + 1 == A.steps, scaled = !(FORM == 2 && last);
+        const double2 *sc = FORM == 0 ? row(last ? t : t + 1) : row(t);
+        double2 *dst = FORM == 0 ? out + t * nn : FORM == 1 ? out + (int64_t)(Nt - 2 - t) * nn : out;
+        for (int e = threadIdx.x; e < nv * n; e += blockDim.x) {
+            // rows: consecutive threads, consecutive columns; columns: consecutive threads, neighbouring vectors
+            const int v = FORM == 0 ? e / n : e % nv, o = FORM == 0 ? e - v * n : e / nv;
+            const double2 scale = scaled ? sc[o] : make_double2(1, 0);
+            const double2 *y = cur + v * L;
+            const double *w = E + o;
+            double2 acc = make_double2(0, 0);
+#pragma unroll 8
+            for (int k = 0; k < n; ++k) {
+                acc.x = fma(y[k].x, w[k * n], acc.x);
+                acc.y = fma(y[k].y, w[k * n], acc.y);
+            }
+            if (FORM != 0 && scaled) acc = cmul(scale, acc);
+            if (FORM != 2 || last) dst[at(v, o)] = acc;
+            nxt[v * L + o] = FORM == 0 ? cmul(acc, scale) : acc;
+        }
+        __syncthreads();
+    }
+}
+
+// Vectors per CTA: the least estimated time, from the FP64 issue of the busiest SM and the chain of one output. Taken while
+// eight vectors fit beside the factor (n <= 144): a trajectory (2 to 128 matrices, Nt = 16 and 32) against one launch per
+// step was 0.42 to 0.95 of its time at n = 40 to 98, 0.73 to 0.99 at n = 112 and 128, 0.75 to 0.97 at n = 144, but up to
+// 1.04 at n = 150 and 1.08 at n = 156, where one CTA per SM and few vectors leave the pipe waiting at each step.
+bool plan_chain(int n, int nmat, ChainArgs &A, int *threads) {
+    if (n < 2 || chain_smem(n, std::min(n, 8)) > CH_SMEM || nmat > 65535) return false;
+    const int sms = std::max(1, num_sms());
+    double best = 1e300;
+    for (int V = 1; V <= std::min(n, 16) && chain_smem(n, V) <= CH_SMEM; ++V) {
+        const int thr = std::min(CH_T, 32 * (int)ceil_div((int64_t)V * n, 32));
+        const int64_t ctas = ceil_div(n, V) * nmat;
+        const int64_t fit = std::max<int64_t>(1, std::min<int64_t>(1536 / thr, (int64_t)(220 * 1024 / chain_smem(n, V))));
+        const double warps = (double)ceil_div((int64_t)V * n, 32);  // warp-sized pieces of a CTA's step, 2 n FMAs each
+        const double res = (double)std::min<int64_t>(fit, ceil_div(ctas, sms));
+        const double waves = (double)ceil_div(ctas, (int64_t)(sms * res));
+        const double step = std::max(res * warps * 2.0 * n * 16.0, (double)ceil_div((int64_t)V * n, thr) * 2.0 * n * 64.0);
+        if (waves * (step + 1500.0) < best) {  // (barrier, scale and store of a step: some 1500 clocks)
+            best = waves * (step + 1500.0);
+            A.V = V;
+            *threads = thr;
+        }
+    }
+    return true;
+}
+
+template <int FORM> int launch_chain(nslg_fm *fm, const ChainArgs &A, int threads, int nmat) {
+    {
+        static std::mutex mu;
+        static std::set<int> done;
+        std::lock_guard<std::mutex> lock(mu);
+        if (!done.count(fm->ctx->device)) {
+            NSLG_CUDA(cudaFuncSetAttribute(k_chain<FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)CH_SMEM));
+            done.insert(fm->ctx->device);
+        }
+    }
+    k_chain<FORM><<<dim3((unsigned)ceil_div(A.n, A.V), (unsigned)nmat), threads, chain_smem(A.n, A.V), fm->ctx->stream>>>(A);
+    note_launch(fm->ctx->stream);
+    NSLG_CUDA(cudaGetLastError());
+    return NSLG_OK;
+}
+
 }  // namespace
 
 namespace {
@@ -1256,7 +1380,11 @@ int grad_logdet_many(nslg_fm *fm, int nmat, const ExpEntry *e0, const ExpEntry *
                                                                        S + (int64_t)(Nt - 1) * nn, ms, nmat, Nt, n);
     note_launch(st);
     const int64_t sph = (int64_t)Nt * n;
-    for (int t = Nt - 2; t >= 0; --t) {
+    ChainArgs ca{E0, E1, emask, S + (int64_t)(Nt - 1) * nn, ms, ph_inv, S, ms, Nt, n, Nt - 1, 1};
+    int cthreads = 0;
+    const bool chain = real && Nt > 1 && plan_chain(n, nmat, ca, &cthreads);
+    if (chain) NSLG_TRY(launch_chain<1>(fm, ca, cthreads, nmat));
+    for (int t = Nt - 2; t >= 0 && !chain; --t) {
         if (!real) {
             NSLG_TRY(zgemm(st, n, n, n, one, Fk + t * nn, n, ms, S + (t + 1) * nn, n, ms, S + t * nn, n, ms, nmat, false));
             continue;
@@ -1280,7 +1408,13 @@ int grad_logdet_many(nslg_fm *fm, int nmat, const ExpEntry *e0, const ExpEntry *
         NSLG_TRY(lu_inverse(fm, P, G, n, s, nmat, ms));
     }
     // prefix chain P(t) = P(t-1) Fk(t) = (P(t-1) D_t) E', P(-1) = G
-    for (int t = 0; t < Nt - 1; ++t) {
+    if (chain) {
+        ca.first = G;
+        ca.sfirst = nn;
+        ca.out = P;
+        NSLG_TRY(launch_chain<0>(fm, ca, cthreads, nmat));
+    }
+    for (int t = 0; t < Nt - 1 && !chain; ++t) {
         const double2 *prev = t == 0 ? G : P + (t - 1) * nn;
         const int64_t sp = t == 0 ? nn : ms;
         if (!real) {
@@ -1319,7 +1453,14 @@ int logdet_many(nslg_fm *fm, int nmat, const ExpEntry *e0, const ExpEntry *e1, i
         // a row scale (none on the last)
         k_logdet_first<<<(unsigned)ceil_div(nn * nmat, 256), 256, 0, st>>>(E0, E1, emask, ph, cur, nmat, Nt, n);
         note_launch(st);
-        for (int t = 1; t < Nt; ++t) {
+        ChainArgs ca{E0, E1, emask, cur, nn, ph, nxt, nn, Nt, n, Nt - 1, 1};
+        int cthreads = 0;
+        const bool chain = Nt > 1 && plan_chain(n, nmat, ca, &cthreads);
+        if (chain) {
+            NSLG_TRY(launch_chain<2>(fm, ca, cthreads, nmat));
+            std::swap(cur, nxt);
+        }
+        for (int t = 1; t < Nt && !chain; ++t) {
             ZProd p = factor_product(n, E0, E1, emask, true, cur, nn, nxt, nn);
             if (t + 1 < Nt) {
                 p.rscale = ph + (int64_t)((t + 2) % Nt) * n;

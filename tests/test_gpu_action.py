@@ -313,3 +313,35 @@ def test_gradient_at_the_longest_time_extent():
     o = O.HubbardExp(lat.hopping_matrix(), Nt, 1.0, 0.0, O.PARTICLE)
     o.populate(phi)
     assert rel_err(fm.gradLogDetM(), o.gradLogDetM()) < 1e-9
+
+
+@pytest.mark.parametrize("Nx,Nt,nconf", [(33, 2, 1), (34, 5, 9), (144, 3, 2), (145, 3, 2)])
+def test_chains_in_one_launch(Nx, Nt, nconf):
+    """The whole-chain kernel at its shortest chain, with a ragged last group of vectors, and on both sides of its size limit
+    (144 sites): log det and force against the oracle's direct product (as above, beta |K| <= 2), and a batch's bits are
+    those of its single configurations."""
+    import nsl_gb300 as N
+    from nsl_gb300.action import HubbardFermionAction, HubbardGaugeAction
+    from nsl_gb300.integrator import Leapfrog
+    from oracle import nsl_oracle as O
+
+    rng = np.random.default_rng(Nx)
+    lat, prm = N.Ring(Nx), {"Nt": Nt, "beta": 1.0, "mu": 0.0, "U": 2.0}
+    phi = rng.standard_normal((nconf, Nt, Nx)) * 0.6 + 0j
+    S = HubbardGaugeAction(prm) + HubbardFermionAction(lat, prm)
+    ev = S.eval_batch(phi)
+    p = rng.standard_normal(phi.shape) + 0j
+    q1, p1 = Leapfrog(S, 0.1, 2)({"phi": phi}, {"phi": p})
+    for b in range(nconf):
+        want = np.sum(phi[b] ** 2) / (2 / Nt * 2.0)
+        F = -phi[b] / (1 / Nt * 2.0)
+        for sp, sg in ((0, 1), (1, -1)):
+            o = O.HubbardExp(lat.hopping_matrix(), Nt, 1.0, 0.0, sp)
+            o.populate(phi[b])
+            want = want - o.logDetM_lu()
+            F = F - sg * o.gradLogDetM()
+        d = ev[b] - want
+        assert abs(d.real) < 1e-10 * max(1, abs(want)) and abs(np.remainder(d.imag + np.pi, 2 * np.pi) - np.pi) < 1e-10
+        assert rel_err(S.force(phi[b])["phi"], F) < 1e-10
+        qb, pb = Leapfrog(S, 0.1, 2)({"phi": phi[b]}, {"phi": p[b]})
+        assert np.array_equal(q1["phi"][b], qb["phi"]) and np.array_equal(p1["phi"][b], pb["phi"])
