@@ -345,3 +345,22 @@ def test_chains_in_one_launch(Nx, Nt, nconf):
         assert rel_err(S.force(phi[b])["phi"], F) < 1e-10
         qb, pb = Leapfrog(S, 0.1, 2)({"phi": phi[b]}, {"phi": p[b]})
         assert np.array_equal(q1["phi"][b], qb["phi"]) and np.array_equal(p1["phi"][b], pb["phi"])
+
+
+@pytest.mark.parametrize("Nx", [33, 38, 63, 64])
+def test_inverse_on_clusters_has_the_single_ctas_bits(Nx):
+    """A batch of 80 matrices is inverted by one CTA each, a single configuration's two by clusters of four (with column counts
+    that four divides and does not, up to the largest): the trajectories agree bit by bit."""
+    import nsl_gb300 as N
+    from nsl_gb300.action import HubbardFermionAction, HubbardGaugeAction
+    from nsl_gb300.integrator import Leapfrog
+
+    rng = np.random.default_rng(Nx)
+    lat, prm = N.Ring(Nx), {"Nt": 2, "beta": 1.0, "mu": 0.0, "U": 2.0}
+    S = HubbardGaugeAction(prm) + HubbardFermionAction(lat, prm)
+    phi = rng.standard_normal((40, 2, Nx)) * 0.6 + 0j
+    p = rng.standard_normal(phi.shape) + 0j
+    q1, p1 = Leapfrog(S, 0.1, 2)({"phi": phi}, {"phi": p})
+    for b in (0, 17, 39):
+        qb, pb = Leapfrog(S, 0.1, 2)({"phi": phi[b]}, {"phi": p[b]})
+        assert np.array_equal(q1["phi"][b], qb["phi"]) and np.array_equal(p1["phi"][b], pb["phi"])
