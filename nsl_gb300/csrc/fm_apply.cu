@@ -28,8 +28,9 @@
 // site of TM consecutive rows, the threads of a CTA are the flattened (row group, site) pairs of whole rows (Nx <= 256)
 // or a run of sites of one row group, and exp(delta K) is read transposed, straight from L1/L2 (consecutive lanes,
 // consecutive sites). TM shrinks until every scheduler has work. Every output sums over y in ascending order
-// whatever TM is. Measured, MM^dagger on 64 right-hand sides at honeycomb 12x12, Nt = 64: 3540 us -> 2470 us (a 2160 us floor at the FP64 pipe's rate); M on one right-hand
-// side at honeycomb 3x3, Nt = 16: 67 us -> 4 us of kernel time (the figures before are 64 x 64 tiles through shared memory).
+// whatever TM is. Measured, MM^dagger on 64 right-hand sides at honeycomb 12x12, Nt = 64: 3540 us -> 2486 us (a 2160 us
+// floor at the FP64 pipe's rate); M on one right-hand side at honeycomb 3x3, Nt = 16: 67 us -> 4 us of kernel time (the
+// figures before are 64 x 64 tiles through shared memory).
 
 #include <algorithm>
 

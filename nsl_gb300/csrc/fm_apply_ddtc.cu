@@ -18,7 +18,8 @@
 // One persistent CTA per SM as in fm_apply_oz.cu: warp 0 streams k-blocks (one bulk copy per operand), warp 1 issues one
 // MMA per operand digit (N = 16 sites x the digits that meet it), four epilogue warps finish 128 x 16 tiles from one of two
 // accumulator sets while the next segment runs in the other.
-// Measured, M on 64 right-hand sides at honeycomb 12x12, Nt = 64: 23.8 ms on the CUDA cores, 0.49 ms here; on 2 at 24x24, Nt = 128: 23.8 and 0.32 ms.
+// Measured, M on 64 right-hand sides at honeycomb 12x12, Nt = 64: 23.8 ms on the CUDA cores, 0.49 ms here; on 2 at 24x24,
+// Nt = 128: 23.8 and 0.32 ms.
 
 #include <algorithm>
 

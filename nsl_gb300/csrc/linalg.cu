@@ -18,8 +18,8 @@ namespace {
 // have equal work. A thread owns one column of TM consecutive rows; a CTA's threads are the flattened (row group,
 // column) pairs of whole rows (N <= 256) or a run of columns of one row group; A is staged in shared memory, B is read
 // in place (consecutive lanes, consecutive columns). zsplit() picks the split. Every output sums over k in ascending
-// order whatever the split. Measured: the 32 products of 50 x 50 complex matrices of a chain step 58 -> 25 us (of it a factor of two from a real factor), 26 real-by-complex
-// products at n = 288 2.82 -> 2.07 ms (the rate of the FP64 pipe).
+// order whatever the split. Measured: 32 products of 50 x 50 matrices, one factor real, 58 -> 25 us (of it a factor of two
+// from the real factor), 26 real-by-complex products at n = 288 2.82 -> 2.07 ms (the rate of the FP64 pipe).
 // REAL: 1 = A holds real numbers (imaginary parts zero), 2 = B does; the product then skips the FMAs with the zero
 // imaginary parts (2 instead of 4 per term). TA: A is given as its adjoint (A[i, k] = conj(At[k lda + i])).
 constexpr int ZKC = 32;    // reduction depth per staged chunk
