@@ -89,6 +89,7 @@ struct nslg_fm {
     int species = NSLG_PARTICLE;
     int sgn = 1;
     double2 *hops = nullptr;  // K (Nx, Nx)
+    bool hops_real = false;   // K holds finite real numbers
     double hops_norm1 = 0;    // max column sum of |K| (bounds its spectral radius)
     double2 hops_trace{0, 0}; // tr K
     int stabilisation = NSLG_STAB_AUTO;  // log det / gradient form (nslg_stabilisation)
@@ -181,7 +182,7 @@ struct ZProd {
     double2 *C;
     int64_t ldc, sC, sC2 = 0;
     int batch2 = 1;
-    int real = 0;             // 1: A holds real numbers, 2: B does (imaginary parts zero: half the FMAs)
+    int real = 0;             // 1: A holds real numbers, 2: B does, 3: both (imaginary parts zero)
     bool a_adjoint = false;   // A is given as its adjoint (K, M)
     bool a_upper = false;     // A is upper triangular
     bool upper = false;       // only the upper triangle of C is computed
