@@ -66,8 +66,21 @@ constexpr int STALL_LIMIT = 3;      // updates without progress before a system 
 // FP64-class operators: after this many reliable updates without a 4x gain in the true |r|^2 the system has reached
 // the accuracy FP64 can certify (the rounding of b - A x itself) and stops unconverged instead of iterating on.
 constexpr int FLOOR_LIMIT = 4;
+// A reliable update keeps the direction (p = r + beta p) while the recurrence still described the residual. Where the true
+// |r|^2 is more than RESTART times the recurrence's, rounding makes up most of it: r is no longer orthogonal to the old
+// direction and beta = |r|^2 / |r_old|^2 runs up to 100s, so the iteration leaves CG, never meets its next update and runs to
+// max_iter, its vectors growing without bound (3xTF32, 144 systems at honeycomb 6x6, Nt = 32, beta = 4, eps = 1e-11: 8 of 300
+// fields; on one of them the solution was off by 1e24 after the default 1e6 iterations). Such an update starts
+// over from p = r: those 8 stop at their floor after at most 2554 iterations, no further off than the others. Above ten times
+// the floor the ratio is below 1.1 and nothing changes.
+constexpr double RESTART = 2.0;
 
 constexpr int RT = 256;  // threads of the vector kernels
+
+// beta of a reliable update whose true |r|^2 is rn (S: the state before it)
+__device__ __forceinline__ double update_beta(const CgState &S, double rn) {
+    return rn > RESTART * S.trig ? 0.0 : rn / S.rsq;
+}
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -545,7 +558,7 @@ __global__ void __launch_bounds__(RT) k_rel_finish(double2 *__restrict__ r, cons
         new_direction = true;
         N.status = CG_ACTIVE;
     }
-    const double beta = rn / S.rsq;
+    const double beta = update_beta(S, rn);
     for (int64_t i = off + lo + threadIdx.x; i < off + hi; i += RT) {
         const double2 rv = rt[i];
         r[i] = rv;

@@ -532,7 +532,7 @@ __global__ void __launch_bounds__(RT) k_cg_resident(RArgs A) {
                 newdir = 1;
                 N.status = CG_ACTIVE;
             }
-            beta_sh = rn / S.rsq;
+            beta_sh = update_beta(S, rn);
             newdir_sh = newdir;
             S = N;
         }

@@ -192,3 +192,26 @@ def test_cg_species_switch_on_one_handle(monkeypatch, precision, resident):
         x = cg(b)
         assert cg.stats["converged"] == 4, (sp, cg.stats)
         assert true_res(hfm, b, x).max() < 2e-10
+
+
+@pytest.mark.parametrize("L,Nt,precision", [((6, 6), 32, "fp64"), ((6, 6), 32, "tf32x3"), ((6, 6), 32, "bf16split"),
+                                            ((6, 6), 32, "fp32"), ((3, 3), 16, "tf32x3")])
+def test_cg_stops_at_the_attainable_accuracy(L, Nt, precision):
+    """A tolerance below what an FP64 residual can show (eps = 1e-15 on unit sources): the solve stops by itself, unconverged,
+    with the true residual at the rounding of b - A x, u |A| |x| (a bar of ten times that), instead of leaving CG and running
+    to max_iter. (3, 3): the resident kernel; the others: one launch per step."""
+    import nsl_gb300 as N
+
+    beta = 4.0
+    hfm = N.HubbardExp(N.Honeycomb(L), Nt, beta)
+    Nx = hfm.Nx
+    phi = np.random.default_rng(2).standard_normal((Nt, Nx)) * np.sqrt(beta / Nt)
+    hfm.populate(phi.astype(np.complex128))
+    b = np.zeros((12, Nt, Nx), dtype=np.complex128)
+    b[np.arange(12), Nt // 2, np.arange(12)] = 1.0
+    cg = N.CG(hfm, N.MatrixCombination.MMdagger, 1e-15, 20000, mode="per_rhs", precision=precision, stop="true_residual")
+    x = cg(b)
+    assert cg.stats["iterations"] < 20000, cg.stats
+    norm_a = (1 + np.exp(3 * beta / Nt)) ** 2  # |M| <= 1 + exp(delta |K|)
+    bar = 10 * 2.0**-53 * norm_a * np.linalg.norm(x.reshape(12, -1), axis=1)
+    assert (true_res(hfm, b, x) <= bar).all(), (true_res(hfm, b, x), bar)
