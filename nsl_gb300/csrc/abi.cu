@@ -380,23 +380,6 @@ NSLG_API int nslg_fm_destroy(nslg_fm *fm) {
     for (auto &kv : fm->memo) {
         cudaFree(kv.second.full);
         free_planes(kv.second);
-        if (kv.second.tc) {
-            cudaFree(kv.second.tc->hi);
-            cudaFree(kv.second.tc->lo);
-            delete kv.second.tc;
-        }
-        if (kv.second.dd) {
-            cudaFree(kv.second.dd->planes);
-            cudaFree(kv.second.dd->col_exp);
-            cudaFree(kv.second.dd->klist);
-            delete kv.second.dd;
-        }
-        if (kv.second.oz) {
-            cudaFree(kv.second.oz->planes);
-            cudaFree(kv.second.oz->col_exp);
-            cudaFree(kv.second.oz->klist);
-            delete kv.second.oz;
-        }
     }
     cudaFree(fm->tc_err);
     if (fm->side) {

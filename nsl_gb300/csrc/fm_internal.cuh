@@ -152,7 +152,7 @@ int get_lin(nslg_fm *fm, double2 d, int one_minus, const ExpEntry **out);
 // The matrix of one operator factor for the handle's discretisation: exp(d K) or d K.
 int get_factor(nslg_fm *fm, double2 d, const ExpEntry **out);
 int install_exp(nslg_fm *fm, double2 d, const double2 *E_dev);
-void free_planes(ExpEntry &e);  // every plane of an entry but `full`
+void free_planes(ExpEntry &e);  // every plane and digit plane of an entry, all but `full`
 
 // ----- kernels (launchers) ---------------------------------------------------------------------------------------
 // Fused M / Mdag application on FP64 vectors with the product in T (double: FP64 drop-in; float: FP32 operator);

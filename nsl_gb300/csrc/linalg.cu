@@ -390,6 +390,26 @@ void free_planes(ExpEntry &e) {
     cudaFree(e.im32T);
     e.re = e.im = e.reT = e.imT = nullptr;
     e.re32T = e.im32T = nullptr;
+    if (e.tc) {
+        cudaFree(e.tc->hi);
+        cudaFree(e.tc->lo);
+        delete e.tc;
+    }
+    if (e.oz) {
+        cudaFree(e.oz->planes);
+        cudaFree(e.oz->col_exp);
+        cudaFree(e.oz->klist);
+        delete e.oz;
+    }
+    if (e.dd) {
+        cudaFree(e.dd->planes);
+        cudaFree(e.dd->col_exp);
+        cudaFree(e.dd->klist);
+        delete e.dd;
+    }
+    e.tc = nullptr;
+    e.oz = nullptr;
+    e.dd = nullptr;
 }
 
 static int make_entry(nslg_fm *fm, double2 *full, nslg::ExpEntry *e) {
@@ -427,6 +447,12 @@ int install_exp(nslg_fm *fm, double2 d, const double2 *E_dev) {
     if (it != fm->memo.end()) {
         NSLG_CUDA(cudaMemcpyAsync(it->second.full, E_dev, n * sizeof(double2), cudaMemcpyDeviceToDevice,
                                   fm->ctx->stream));
+        // everything derived from the old matrix goes with it: planes and digits (built again on their next use), and the
+        // captured graphs, which hold their addresses (a group's graphs are keyed by ws_generation)
+        NSLG_CUDA(cudaStreamSynchronize(fm->ctx->stream));
+        drop_graphs(fm);
+        fm->lf_seen.clear();
+        ++fm->ws_generation;
         free_planes(it->second);
         return make_entry(fm, it->second.full, &it->second);
     }

@@ -259,3 +259,58 @@ def test_split_operator_skips_zero_digits(Nx, kind):
                            np.roll(np.abs(psi).max(2), -1, 1))):
         err = np.abs(getattr(fm, op)(psi, precision="bf16split") - want).max(2)
         assert np.all(err <= eps * row + 2.0 ** -51 * np.abs(want).max(2)), (op, (err / row).max())
+
+
+def test_replacing_exp_hopping_replaces_what_was_derived_from_it():
+    """set_exp_hopping_matrix on a handle that has used the old exp(+-delta K) in every form (planes, 3xTF32 and digit planes,
+    captured solves and trajectories): afterwards every call gives what a handle that never saw the old matrix gives, and a
+    certified solve solves the new system."""
+    import nsl_gb300 as N
+    from nsl_gb300.action import HubbardFermionAction, HubbardGaugeAction
+    from nsl_gb300.configuration import Configuration
+    from nsl_gb300.integrator import Leapfrog
+    from oracle import nsl_oracle as O
+    from test_gpu_cg_dd import _same_operator
+
+    Nt, beta, R = 32, 2.0, 4  # 2304 elements per right-hand side: past the resident kernel, 9216 in all for double-double
+    rng = np.random.default_rng(8)
+    w, V = np.linalg.eigh(np.array(N.Honeycomb((6, 6)).hopping_matrix()).real)
+    new = {s * beta / Nt: (V * np.exp(0.9 * s * beta / Nt * w)) @ V.T + 0j for s in (1, -1)}
+
+    def build(installed):
+        lat = N.Honeycomb((6, 6))
+        if installed:
+            for d, E in new.items():
+                lat.set_exp_hopping_matrix(d, E)
+        params = {"Nt": Nt, "beta": beta, "U": 1.0}
+        action = HubbardGaugeAction(params) + HubbardFermionAction(lat, params, force_precision="bf16split")
+        return N.HubbardExp(lat, Nt, beta), Leapfrog(action, 1.0, 2)
+
+    phi = (rng.standard_normal((Nt, 72)) * np.sqrt(beta / Nt)).astype(np.complex128)
+    mom = rng.standard_normal((Nt, 72)).astype(np.complex128)
+    b = rng.standard_normal((R, Nt, 72)) + 1j * rng.standard_normal((R, Nt, 72))
+    eps = 1e-12 * np.linalg.norm(b[0])
+
+    def use(fm, lf):
+        fm.populate(phi, N.Species.Particle)
+        out = [getattr(fm, op)(b, precision=p) for op in ("M", "MMdagger") for p in ("fp64", "fp32", "tf32x3", "bf16split")]
+        out += list(fm.apply_dd(N.MatrixCombination.MMdagger, b))
+        for p in ("bf16split", "tf32x3"):
+            cg = N.CG(fm, N.MatrixCombination.MMdagger, eps, 20000, mode="per_rhs", precision=p, stop="true_residual_dd")
+            out += [cg(b), cg.x_lo_]
+            assert cg.stats["converged"] == R, (p, cg.stats)
+        for _ in range(2):  # the second trajectory is captured
+            q, p = lf(Configuration({"phi": phi}), Configuration({"phi": mom}))
+        return out + [q["phi"], p["phi"]]
+
+    fm, lf = build(False)
+    old = use(fm, lf)
+    for h in (fm, lf.action_._mask_and_fm()[1]):
+        for d, E in new.items():
+            h.set_exp_hopping_matrix(d, E)
+    got, want = use(fm, lf), use(*build(True))
+    for k, (g, v, o) in enumerate(zip(got, want, old)):
+        assert np.array_equal(g, v), (k, rel_err(g, v), rel_err(g, o))
+    x, lo = got[10], got[11]
+    ho = _same_operator(fm, phi)
+    assert max(np.linalg.norm(O.residual_dd(ho, "MMdagger", b[r], x[r], lo[r])) for r in range(R)) <= 1.01 * eps
