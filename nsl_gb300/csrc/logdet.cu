@@ -73,8 +73,9 @@ __global__ void k_add_identity(double2 *A, int n) {
 }
 
 // ---- LU with partial pivoting -------------------------------------------------------------------------------------
-// Pivot of column k: p = argmax_{i>=k} |A[i,k]| (first index on ties); the multipliers l_ik = A[i,k] / A[k,k] are
-// stored in place, the running log of the pivots and the number of row swaps give log det.
+// Pivot of column k: p = argmax_{i>=k} |A[i,k]| (first index on ties, k itself where every entry is NaN, so that a row index
+// never leaves the matrix); the multipliers l_ik = A[i,k] / A[k,k] are stored in place, the running log of the pivots and the
+// number of row swaps give log det.
 constexpr int LT = 1024;
 
 // ---- blocked LU: panels of NB columns ------------------------------------------------------------------------------
@@ -98,7 +99,7 @@ __global__ void __launch_bounds__(LT) k_lu_panel(double2 *A, int n, int k0, int 
     __shared__ int bidx[LT];
     for (int k = k0; k < k0 + nb; ++k) {
         double bv = -1.0;
-        int bi = n;
+        int bi = k;
         for (int i = k + threadIdx.x; i < n; i += LT) {
             const double2 v = A[(int64_t)i * n + k];
             const double m = hypot(v.x, v.y);
@@ -188,7 +189,7 @@ __global__ void __launch_bounds__(LPT) k_lu_panel_smem(double2 *A, int n, int k0
     for (int kk = 0; kk < nb; ++kk) {
         // pivot: largest |a_ik|^2 over rows i >= kk, first index on ties
         double bm = -1.0;
-        int bi = rows;
+        int bi = kk;
         for (int i = kk + threadIdx.x; i < rows; i += LPT) {
             const double2 v = Ps[i * PS + kk];
             const double m = v.x * v.x + v.y * v.y;
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(LPT) k_lu_panel_smem(double2 *A, int n, int k0
         __syncthreads();
         if (warp == 0) {
             bm = lane < LPT / 32 ? wbest[lane] : -1.0;
-            bi = lane < LPT / 32 ? widx[lane] : rows;
+            bi = lane < LPT / 32 ? widx[lane] : kk;
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const double om = __shfl_down_sync(0xffffffffu, bm, o);

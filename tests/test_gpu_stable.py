@@ -215,3 +215,31 @@ def test_stratified_panel_edges(Nx, Nt, beta):
         s, l = np.linalg.slogdet(Md)
         ref = complex(l, np.angle(s))
         assert abs(mod2pi(h.logDetM() - ref)) <= max(1e-13 * abs(ref), n * eps * nI * nM)
+
+
+@pytest.mark.parametrize("mode", ["plain", "stratified"])
+@pytest.mark.parametrize("Nx", [5, 32, 33, 72, 130])
+def test_nan_field_stays_inside_the_matrices(Nx, mode):
+    """A field with a NaN turns every matrix into NaN, and no pivot search finds a largest entry: log det and gradient are NaN
+    too (or a reported error), and the handle's next evaluation is what a new handle gives."""
+    import nsl_gb300 as N
+
+    Nt, beta = 6, 3.0
+    phi = _field(Nx, Nt, beta, Nx)
+    bad = phi.copy()
+    bad[2, Nx // 2] = np.nan
+
+    def evaluate(h, f):
+        h.populate(f)
+        return h.logDetM(), np.asarray(h.gradLogDetM())
+
+    h, fresh = N.HubbardExp(N.Ring(Nx), Nt, beta), N.HubbardExp(N.Ring(Nx), Nt, beta)
+    for x in (h, fresh):
+        x.set_stabilisation(mode)
+    try:
+        ld, g = evaluate(h, bad)
+        assert not np.isfinite(ld) and not np.isfinite(g).any()
+    except RuntimeError:
+        pass
+    (ld, g), (ld0, g0) = evaluate(h, phi), evaluate(fresh, phi)
+    assert ld == ld0 and np.array_equal(g, g0)
