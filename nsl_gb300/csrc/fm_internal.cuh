@@ -238,11 +238,15 @@ int fm_apply_ddtc(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *xh, c
 // matrices with factors Ep[g] = exp(-sgn_g delta K), E[g] = exp(sgn_g delta K) and phase rows ph / pinv
 // (nmat, Nt, Nx).
 bool use_stratified(const nslg_fm *fm);
+// Bits of the workspace word "st_flags" (cleared by an evaluation, or before the replay of a captured trajectory):
+constexpr int ST_INEXACT = 1;  // the second QR pass to first order is not exact enough for this field
+// log of the bound exp(2 k |delta| rho + k spread) on a chunk's condition; spread: max - min of Im phi over a slice's sites
+double strat_log_condition(const nslg_fm *fm, double spread);
 bool use_stratified_grad(const nslg_fm *fm);
 int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, const double2 *ph,
                       const double2 *pinv, double2 *out);
 int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, const int *sgn,
-                 const double2 *ph, const double2 *pinv, double2 *out);
+                 const double2 *ph, const double2 *pinv, double2 *out, bool full_pass = false);
 
 // ----- batched dense LU (logdet.cu) --------------------------------------------------------------------------------
 struct LuScratch {

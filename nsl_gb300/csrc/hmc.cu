@@ -10,6 +10,7 @@
 // total force and applies the momentum kick and the following drift.
 
 #include <cmath>
+#include <cstring>
 
 #include <cstdio>
 #include <string>
@@ -210,7 +211,7 @@ int fermion_grads_many(nslg_fm *fm, const double2 *phi, int64_t nconf, double2 *
             Ep[g] = e[g & 1][0];
             Ed[g] = e[g & 1][1];
         }
-        NSLG_TRY(grad_logdet_strat(fm, (int)(2 * nconf), Ep.data(), Ed.data(), ph, ph_inv, g2));
+        return grad_logdet_strat(fm, (int)(2 * nconf), Ep.data(), Ed.data(), ph, ph_inv, g2);
     } else {
         const ExpEntry *EP, *EH;
         NSLG_TRY(grad_factors(fm, &EP, &EH));
@@ -421,6 +422,94 @@ int leapfrog_steps(nslg_fm *fm, double2 *q, double2 *p, double2 Ut, const double
 
 }  // namespace
 
+// A captured trajectory cannot choose the stratified gradient's second QR pass by its field (ST_INEXACT): q and p are saved
+// before the replay, and where a force set the flag they are restored and the trajectory runs eagerly, which chooses force
+// by force. A trajectory whose starting field makes that likely runs eagerly at once: both give the same result.
+namespace {
+
+struct Retake {
+    int *flags = nullptr;  // null: no stratified gradient, nothing to take back
+    double2 *q0 = nullptr, *p0 = nullptr;
+    bool eager = false;
+};
+
+// max over the time slices of max Im phi - min Im phi (an ordered bit pattern; NaN compares large), one block per slice
+__global__ void k_im_spread(const double2 *__restrict__ phi, int Nx, unsigned long long *__restrict__ out) {
+    __shared__ double hi_sh[4], lo_sh[4];
+    phi += (int64_t)blockIdx.x * Nx;
+    double hi = -INFINITY, lo = INFINITY;
+    for (int x = threadIdx.x; x < Nx; x += 128) {
+        hi = fmax(hi, phi[x].y);
+        lo = fmin(lo, phi[x].y);
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    }
+    if (threadIdx.x % 32 == 0) {
+        hi_sh[threadIdx.x / 32] = hi;
+        lo_sh[threadIdx.x / 32] = lo;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < 4; ++w) {
+        hi = fmax(hi, hi_sh[w]);
+        lo = fmin(lo, lo_sh[w]);
+    }
+    atomicMax(out, (unsigned long long)__double_as_longlong(hi - lo));
+}
+
+// The buffers (before any graph key is formed: they may move the workspace generation).
+int retake_buffers(nslg_fm *fm, int terms, int64_t nconf, Retake &R) {
+    if (!(terms & 2) || !use_stratified_grad(fm)) return NSLG_OK;
+    const int64_t n = nconf * fm->Nt * fm->Nx;
+    unsigned long long *d;
+    NSLG_TRY(ws_get(fm, "lf_spread", 1, &d));
+    NSLG_TRY(ws_get(fm, "lf_q0", (size_t)n, &R.q0));
+    NSLG_TRY(ws_get(fm, "lf_p0", (size_t)n, &R.p0));
+    NSLG_TRY(ws_get(fm, "st_flags", 1, &R.flags));
+    return NSLG_OK;
+}
+
+// Whether q makes ST_INEXACT likely: a chunk's condition may exceed 1e4 (1e3 is about where the flag is set; real fields
+// stay below 200).
+int retake_likely(nslg_fm *fm, const double2 *q, int64_t nconf, Retake &R) {
+    if (!R.flags) return NSLG_OK;
+    cudaStream_t st = fm->ctx->stream;
+    unsigned long long *d, h = 0;
+    NSLG_TRY(ws_get(fm, "lf_spread", 1, &d));
+    NSLG_CUDA(cudaMemsetAsync(d, 0, sizeof h, st));
+    k_im_spread<<<(unsigned)(nconf * fm->Nt), 128, 0, st>>>(q, (int)fm->Nx, d);
+    note_launch(st);
+    NSLG_CUDA(cudaGetLastError());
+    NSLG_CUDA(cudaMemcpyAsync(&h, d, sizeof h, cudaMemcpyDeviceToHost, st));
+    NSLG_CUDA(cudaStreamSynchronize(st));
+    double spread;
+    std::memcpy(&spread, &h, sizeof h);
+    R.eager = !(strat_log_condition(fm, spread) <= std::log(1e4)) && strat_log_condition(fm, 0.0) <= std::log(200.0);
+    return NSLG_OK;
+}
+
+int retake_save(nslg_fm *fm, const double2 *q, const double2 *p, int64_t nconf, const Retake &R) {
+    if (!R.flags) return NSLG_OK;
+    cudaStream_t st = fm->ctx->stream;
+    const size_t bytes = (size_t)(nconf * fm->Nt * fm->Nx) * sizeof(double2);
+    NSLG_CUDA(cudaMemcpyAsync(R.q0, q, bytes, cudaMemcpyDeviceToDevice, st));
+    NSLG_CUDA(cudaMemcpyAsync(R.p0, p, bytes, cudaMemcpyDeviceToDevice, st));
+    NSLG_CUDA(cudaMemsetAsync(R.flags, 0, sizeof(int), st));
+    return NSLG_OK;
+}
+
+int retake_restore(nslg_fm *fm, double2 *q, double2 *p, int64_t nconf, const Retake &R) {
+    cudaStream_t st = fm->ctx->stream;
+    const size_t bytes = (size_t)(nconf * fm->Nt * fm->Nx) * sizeof(double2);
+    NSLG_CUDA(cudaMemcpyAsync(q, R.q0, bytes, cudaMemcpyDeviceToDevice, st));
+    NSLG_CUDA(cudaMemcpyAsync(p, R.p0, bytes, cudaMemcpyDeviceToDevice, st));
+    return NSLG_OK;
+}
+
+}  // namespace
+
 // A trajectory on the workspace buffers q, p. The first call for a given (Nmd, length, direction, terms, U~) runs
 // eagerly, which builds every workspace and exp(delta K) entry; the second captures the same launches into a CUDA
 // graph (thousands of small kernels on small lattices, so launch latency would dominate) and later calls replay it.
@@ -453,6 +542,8 @@ void after_trajectory(nslg_fm *fm, int terms, int64_t nconf) {
 int leapfrog_dev(nslg_fm *fm, double2 *q, double2 *p, double2 Ut, double traj, int64_t nmd, int backward,
                  int real_force, int terms, int64_t nconf, const double2 *uin_cfg) {
     cudaStream_t st = fm->ctx->stream;
+    Retake R;
+    NSLG_TRY(retake_buffers(fm, terms, nconf, R));
     auto make_key = [&]() { return lf_key(fm, q, p, Ut, uin_cfg, traj, nmd, backward, real_force, terms, nconf); };
     std::string key = make_key();
     auto it = fm->graphs.find(key);
@@ -461,6 +552,8 @@ int leapfrog_dev(nslg_fm *fm, double2 *q, double2 *p, double2 Ut, double traj, i
         fm->lf_seen[make_key()] = 1;  // the key after the eager run's allocations
         return NSLG_OK;
     }
+    NSLG_TRY(retake_likely(fm, q, nconf, R));
+    if (R.eager) return leapfrog_steps(fm, q, p, Ut, uin_cfg, traj, nmd, backward, real_force, terms, nconf);
     int *sing = nullptr;
     if (terms & 2) NSLG_TRY(ws_get(fm, "lu_singular", 1, &sing));
     if (it == fm->graphs.end()) {
@@ -490,13 +583,19 @@ int leapfrog_dev(nslg_fm *fm, double2 *q, double2 *p, double2 Ut, double traj, i
         fm->graph_defs[key] = g;
     }
     if (sing) NSLG_CUDA(cudaMemsetAsync(sing, 0, sizeof(int), st));
+    NSLG_TRY(retake_save(fm, q, p, nconf, R));
     NSLG_CUDA(cudaGraphLaunch(it->second, st));
     note_launch(st, fm->graph_kernels[key]);
     after_trajectory(fm, terms, nconf);
     if (sing) {
-        int h = 0;
+        int h = 0, flags = 0;
         NSLG_CUDA(cudaMemcpyAsync(&h, sing, sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (R.flags) NSLG_CUDA(cudaMemcpyAsync(&flags, R.flags, sizeof(int), cudaMemcpyDeviceToHost, st));
         NSLG_CUDA(cudaStreamSynchronize(st));
+        if (flags & ST_INEXACT) {
+            NSLG_TRY(retake_restore(fm, q, p, nconf, R));
+            return leapfrog_steps(fm, q, p, Ut, uin_cfg, traj, nmd, backward, real_force, terms, nconf);
+        }
         NSLG_REQUIRE(!h, NSLG_ERR_ARG, "gradLogDetM: 1 + A^{-1} is singular");
     }
     return NSLG_OK;
@@ -512,10 +611,16 @@ int leapfrog_group_dev(int ng, nslg_fm *const *fms, const int64_t *nconf, double
     nslg_fm *f0 = fms[0];
     cudaStream_t st = f0->ctx->stream;
     std::vector<std::string> keys(ng);
+    std::vector<Retake> R(ng);
     bool ready = true;
     for (int g = 0; g < ng; ++g) {
+        NSLG_TRY(retake_buffers(fms[g], terms, nconf[g], R[g]));
         keys[g] = lf_key(fms[g], q[g], p[g], Ut[g], uin_cfg[g], traj, nmd, backward, real_force, terms, nconf[g]);
         ready &= fms[g]->graph_defs.count(keys[g]) > 0;
+    }
+    for (int g = 0; g < ng && ready && ng > 1; ++g) {
+        NSLG_TRY(retake_likely(fms[g], q[g], nconf[g], R[g]));
+        ready &= !R[g].eager;
     }
     if (!ready || ng == 1) {
         for (int g = 0; g < ng; ++g)
@@ -550,14 +655,22 @@ int leapfrog_group_dev(int ng, nslg_fm *const *fms, const int64_t *nconf, double
             NSLG_TRY(ws_get(fms[g], "lu_singular", 1, &sing[g]));
             NSLG_CUDA(cudaMemsetAsync(sing[g], 0, sizeof(int), st));
         }
+    for (int g = 0; g < ng; ++g) NSLG_TRY(retake_save(fms[g], q[g], p[g], nconf[g], R[g]));
     NSLG_CUDA(cudaGraphLaunch(it->second, st));
     note_launch(st, f0->graph_kernels[pk]);
-    std::vector<int> h(ng, 0);
+    std::vector<int> h(ng, 0), flags(ng, 0);
     for (int g = 0; g < ng; ++g) {
         after_trajectory(fms[g], terms, nconf[g]);
         if (sing[g]) NSLG_CUDA(cudaMemcpyAsync(&h[g], sing[g], sizeof(int), cudaMemcpyDeviceToHost, st));
+        if (R[g].flags) NSLG_CUDA(cudaMemcpyAsync(&flags[g], R[g].flags, sizeof(int), cudaMemcpyDeviceToHost, st));
     }
     NSLG_CUDA(cudaStreamSynchronize(st));
+    for (int g = 0; g < ng; ++g) {
+        if (!(flags[g] & ST_INEXACT)) continue;
+        h[g] = 0;
+        NSLG_TRY(retake_restore(fms[g], q[g], p[g], nconf[g], R[g]));
+        NSLG_TRY(leapfrog_steps(fms[g], q[g], p[g], Ut[g], uin_cfg[g], traj, nmd, backward, real_force, terms, nconf[g]));
+    }
     for (int g = 0; g < ng; ++g) NSLG_REQUIRE(!h[g], NSLG_ERR_ARG, "gradLogDetM: 1 + A^{-1} is singular");
     return NSLG_OK;
 }

@@ -1438,7 +1438,7 @@ int fm_grad_logdet(nslg_fm *fm, double2 *out) {
     if (use_stratified_grad(fm)) {
         const ExpEntry *Ed;
         NSLG_TRY(get_exp(fm, make_double2(fm->sgn * fm->delta.x, fm->sgn * fm->delta.y), &Ed));
-        NSLG_TRY(grad_logdet_strat(fm, 1, &E, &Ed, fm->phase, fm->phase_inv, out));
+        return grad_logdet_strat(fm, 1, &E, &Ed, fm->phase, fm->phase_inv, out);
     } else if (fm->force_precision == NSLG_PREC_BF16_SPLIT && fm->kind == NSLG_FM_EXP && E->is_real && n <= 2048) {
         NSLG_TRY(grad_logdet_tc(fm, E, out));
     } else {

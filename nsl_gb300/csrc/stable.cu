@@ -217,14 +217,20 @@ __global__ void __launch_bounds__(CQ_NB *CQ_NB) k_cholqr_panel(const double2 *__
 }
 
 // Second pass to first order. Q1 from one pass is orthogonal up to E = Q1^H Q1 - 1, |E| ~ cond(Z)^2 eps (1e-11 and less for
-// the chunk products here); its Cholesky factor is R2 = 1 + T + O(E^2), T the strict upper triangle of E plus half its
-// diagonal, so Q = Q1 (1 - T) and R = (1 + T) R1 to O(E^2) ~ 1e-22. E itself is evaluated in FP64; the corrections
-// Q1 T and T R1, of relative size |E|, are formed in FP32 (an error of 6e-8 |E| < 1e-18) and added in FP64.
+// real fields); its Cholesky factor is R2 = 1 + T + O(E^2), T the strict upper triangle of E plus half its diagonal, so
+// Q = Q1 (1 - T) and R = (1 + T) R1 to O(E^2) ~ 1e-22. E itself is evaluated in FP64; the corrections Q1 T and T R1, of
+// relative size |E|, are formed in FP32 (an error of 6e-8 |E| < 1e-17) and added in FP64. How large E is depends on the
+// field: phases of a complex one have moduli exp(+-Im phi), and an exp(delta K) set by the caller may have any condition. So
+// the kernel measures it: an entry above FIRST_ORDER_E, or a diagonal of R1 that FP32 cannot hold, sets ST_INEXACT in flags,
+// and the stacks are built again with a full second pass (strat_stacks; a captured trajectory is taken back and run eagerly).
+// Measured, ring 32, Nt = 32, beta = 8, Im phi of standard deviation 1.75: gradient error 7.6e-3 with the first order alone,
+// 2e-7 with the full pass.
 // out = C + sign A B (A, B rounded to FP32) for the matrices of a batch; Eu: the upper triangle of Q1^H Q1, which stands
 // for T as B (t_left = false: A = C = Q1, sign -1) or as A (t_left: B = C = R1, sign +1).
+constexpr float FIRST_ORDER_E = 1e-10f;
 constexpr int RF = 32;
 __global__ void __launch_bounds__(256) k_refine(const double2 *__restrict__ Eu, const double2 *__restrict__ X,
-                                                double2 *__restrict__ out, int n, bool t_left) {
+                                                double2 *__restrict__ out, int n, bool t_left, int *flags) {
     __shared__ float2 As[RF][RF + 1], Bs[RF][RF + 1];
     const int64_t nn = (int64_t)n * n;
     Eu += blockIdx.z * nn;
@@ -245,12 +251,18 @@ __global__ void __launch_bounds__(256) k_refine(const double2 *__restrict__ Eu, 
     float2 acc[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) acc[i] = make_float2(0.f, 0.f);
+    bool inexact = false;
     // T[k][c] is zero for k > c; T[r][k] for k < r, and R1[k][c] for k > c
     const int kend = min(n, c0 + RF);
     for (int k0 = t_left ? r0 : 0; k0 < kend; k0 += RF) {
         for (int r = ty; r < RF; r += 8) {
             As[r][tx] = t_left ? tval(r0 + r, k0 + tx) : xval(r0 + r, k0 + tx);
-            Bs[r][tx] = t_left ? xval(k0 + r, c0 + tx) : tval(k0 + r, c0 + tx);
+            const float2 b = t_left ? xval(k0 + r, c0 + tx) : tval(k0 + r, c0 + tx);
+            Bs[r][tx] = b;
+            if (blockIdx.y == 0) {  // these CTAs see all of E, or the diagonal of R1 (negated tests: NaN is inexact)
+                if (!t_left) inexact |= !(fabsf(b.x) <= FIRST_ORDER_E && fabsf(b.y) <= FIRST_ORDER_E);
+                else if (k0 + r == c0 + tx && c0 + tx < n) inexact |= !(b.x > 1e-25f && b.x < 1e25f);
+            }
         }
         __syncthreads();
 #pragma unroll 8
@@ -265,6 +277,7 @@ __global__ void __launch_bounds__(256) k_refine(const double2 *__restrict__ Eu, 
         }
         __syncthreads();
     }
+    if (inexact) atomicOr(flags, ST_INEXACT);
     const int c = c0 + tx;
     const double sg = t_left ? 1.0 : -1.0;
 #pragma unroll
@@ -465,6 +478,7 @@ struct Strat {
     double2 *Ep = nullptr, *E = nullptr;        // E' = exp(-sgn delta K), E = exp(sgn delta K) per matrix
     double2 *C = nullptr;                       // chunk products (nmat, J, n, n)
     bool first_order = true;                    // second QR pass to first order (chunks of bounded condition)
+    int *flags = nullptr;                       // ST_* of this evaluation
     double2 *SU = nullptr, *ST = nullptr;       // suffix stack (nmat, J + 1, n, n)
     double2 *PU = nullptr, *PT = nullptr;       // prefix stack (adjoint) (nmat, J + 1, n, n)
     double *Sd = nullptr, *Pd = nullptr;        // (nmat, J + 1, n)
@@ -489,7 +503,7 @@ int chunk_len(const nslg_fm *fm) {
 }
 
 int strat_setup(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, bool need_prefix,
-                Strat &S) {
+                bool full_pass, Strat &S) {
     cudaStream_t st = fm->ctx->stream;
     S.n = (int)fm->Nx;
     S.Nt = (int)fm->Nt;
@@ -528,10 +542,12 @@ int strat_setup(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry
     NSLG_TRY(ws_get(fm, "st_Tn", qn, &S.Tn));
     NSLG_TRY(ws_get(fm, "st_dn", (size_t)side * nmat * S.n, &S.dn));
     NSLG_TRY(ws_get(fm, "st_rank", (size_t)side * nmat * S.n, &S.rank));
-    // condition of a chunk product: at most exp(2 k |delta| rho). Up to 200 (the automatic chunk length keeps 81) the
-    // first QR pass leaves |E| < 1e-10 and its second order below rounding; one slice of a very large delta exceeds it.
-    const double kd = (double)(S.q + (S.r > 0)) * std::hypot(fm->delta.x, fm->delta.y) * fm->hops_norm1;
-    S.first_order = kd <= 0.5 * std::log(200.0);
+    NSLG_TRY(ws_get(fm, "st_flags", 1, &S.flags));
+    if (!fm->defer_checks) NSLG_CUDA(cudaMemsetAsync(S.flags, 0, sizeof(int), st));
+    // condition of a chunk product of a real field: at most exp(2 k |delta| rho). Up to 200 (the automatic chunk length keeps
+    // 81) the first QR pass leaves |E| < 1e-10 and its second order below rounding; one slice of a very large delta
+    // exceeds it. What a complex field adds is measured (k_refine).
+    S.first_order = !full_pass && strat_log_condition(fm, 0.0) <= std::log(200.0);
     return NSLG_OK;
 }
 
@@ -607,8 +623,8 @@ int cholqr2(nslg_fm *fm, Strat &S, int cnt) {
         gram.upper = true;
         NSLG_TRY(zprod(st, gram, cnt));
         const dim3 grid((unsigned)ceil_div(n, RF), (unsigned)ceil_div(n, RF), (unsigned)cnt);
-        k_refine<<<grid, 256, 0, st>>>(S.Gm, S.Z, S.Q, n, false);
-        k_refine<<<grid, 256, 0, st>>>(S.Gm, S.R1, S.R, n, true);
+        k_refine<<<grid, 256, 0, st>>>(S.Gm, S.Z, S.Q, n, false, S.flags);
+        k_refine<<<grid, 256, 0, st>>>(S.Gm, S.R1, S.R, n, true, S.flags);
         note_launch(st, 2);
     } else {
         NSLG_TRY(cholqr_pass(fm, S, S.R2, cnt));
@@ -648,6 +664,7 @@ int udt_fold(nslg_fm *fm, Strat &S, int z0, const double *d_prev, const double2 
 }
 
 // Both stacks (the prefix one only when S.PU is set), one batched step per chunk.
+constexpr int EARLY_LOOK = 128;
 int strat_stacks(nslg_fm *fm, Strat &S) {
     cudaStream_t st = fm->ctx->stream;
     const int n = S.n, J = S.J, nmat = S.nmat;
@@ -680,6 +697,18 @@ int strat_stacks(nslg_fm *fm, Strat &S) {
         if (prefix)
             NSLG_TRY(udt_fold(fm, S, nmat, S.Pd + (int64_t)i * n, S.PT + i * nn, S.PU + (i + 1) * nn,
                               S.PT + (i + 1) * nn, S.Pd + (int64_t)(i + 1) * n, ms, ds));
+        // the first step shows most fields that need a full second pass; on large lattices looking there saves most of an
+        // evaluation that would be repeated (a look costs 0.9 % of a gradient at 72 sites, less than 0.1 % at 288)
+        if (i == 0 && n >= EARLY_LOOK && S.first_order && !fm->defer_checks) {
+            int h = 0;
+            NSLG_CUDA(cudaMemcpyAsync(&h, S.flags, sizeof(int), cudaMemcpyDeviceToHost, st));
+            NSLG_CUDA(cudaStreamSynchronize(st));
+            if (h & ST_INEXACT) {
+                S.first_order = false;
+                NSLG_CUDA(cudaMemsetAsync(S.flags, 0, sizeof(int), st));
+                return strat_stacks(fm, S);
+            }
+        }
     }
     return NSLG_OK;
 }
@@ -697,6 +726,11 @@ bool use_stratified(const nslg_fm *fm) {
     return beta_rho > 14.0;
 }
 
+double strat_log_condition(const nslg_fm *fm, double spread) {
+    const int64_t J = ceil_div(fm->Nt, chunk_len(fm));
+    return (double)ceil_div(fm->Nt, J) * (2.0 * std::hypot(fm->delta.x, fm->delta.y) * fm->hops_norm1 + spread);
+}
+
 // The gradient (the HMC force) follows use_stratified, except that the split-BF16 force setting
 // (nslg_fm_set_force_precision(NSLG_PREC_BF16_SPLIT): a fast force whose error is stated, not the FP64 one) keeps the
 // direct product under AUTO while beta rho <= 28: there the split-BF16 direct-product gradient is within ~2e-7 of the
@@ -709,13 +743,13 @@ bool use_stratified_grad(const nslg_fm *fm) {
     return !(fm->force_precision == NSLG_PREC_BF16_SPLIT && fm->stabilisation == NSLG_STAB_AUTO && beta_rho <= 28.0);
 }
 
-// d log det M / d phi for nmat matrices (matrix g: factors E'[g] = exp(-sgn_g delta K) and E[g] = exp(sgn_g delta K),
-// phase rows ph[g] = phiExp and pinv[g] = phiExpInv (Nt, Nx)); out (nmat, Nt, Nx) on the device.
-int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, const double2 *ph,
-                      const double2 *pinv, double2 *out) {
+namespace {
+
+int grad_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, const double2 *ph,
+               const double2 *pinv, double2 *out, bool full_pass) {
     cudaStream_t st = fm->ctx->stream;
     Strat S;
-    NSLG_TRY(strat_setup(fm, nmat, Ep, E, true, S));
+    NSLG_TRY(strat_setup(fm, nmat, Ep, E, true, full_pass, S));
     NSLG_TRY(strat_chunks(fm, S, pinv));
     NSLG_TRY(strat_stacks(fm, S));
     const int n = S.n, J = S.J, Nt = S.Nt;
@@ -790,16 +824,40 @@ int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const Ex
     return NSLG_OK;
 }
 
+}  // namespace
+
+// d log det M / d phi for nmat matrices (matrix g: factors E'[g] = exp(-sgn_g delta K) and E[g] = exp(sgn_g delta K),
+// phase rows ph[g] = phiExp and pinv[g] = phiExpInv (Nt, Nx)); out (nmat, Nt, Nx) on the device. Waits for the result and
+// evaluates again with a full second QR pass where the first order was not exact enough, except inside a captured
+// trajectory, whose flags are read after its replay.
+int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, const double2 *ph,
+                      const double2 *pinv, double2 *out) {
+    if (fm->defer_checks) return grad_strat(fm, nmat, Ep, E, ph, pinv, out, false);
+    cudaStream_t st = fm->ctx->stream;
+    int *sing, *flags, h[2] = {0, 0};
+    for (int full = 0; full < 2; ++full) {
+        NSLG_TRY(grad_strat(fm, nmat, Ep, E, ph, pinv, out, full != 0));
+        NSLG_TRY(ws_get(fm, "lu_singular", 1, &sing));
+        NSLG_TRY(ws_get(fm, "st_flags", 1, &flags));
+        NSLG_CUDA(cudaMemcpyAsync(&h[0], sing, sizeof(int), cudaMemcpyDeviceToHost, st));
+        NSLG_CUDA(cudaMemcpyAsync(&h[1], flags, sizeof(int), cudaMemcpyDeviceToHost, st));
+        NSLG_CUDA(cudaStreamSynchronize(st));
+        if (!(h[1] & ST_INEXACT)) break;
+    }
+    NSLG_REQUIRE(!h[0], NSLG_ERR_ARG, "gradLogDetM: 1 + A^{-1} is singular");
+    return NSLG_OK;
+}
+
 // log det M for nmat matrices (as above; ph[g] = phiExp rows, sgn_g the species sign of matrix g): the suffix stack
 // to s = 0, then log det(1 + C(0)) = log det U_L + sum log D_Lb + log det X with X = D_Lb^{-1} U_L^H + D_Ls T_L,
 // plus log det of the slices' inverses, Nt sgn delta tr K + sum Log phiExp. The LUs of X and of U_L (unitary: its phase)
 // are one batch: their panels are chains of dependent steps on one SM per matrix. out[g] on the host, imaginary part on
 // the principal branch; -inf for a singular X.
 int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntry *const *E, const int *sgn,
-                 const double2 *ph, const double2 *pinv, double2 *out) {
+                 const double2 *ph, const double2 *pinv, double2 *out, bool full_pass) {
     cudaStream_t st = fm->ctx->stream;
     Strat S;
-    NSLG_TRY(strat_setup(fm, nmat, Ep, E, false, S));
+    NSLG_TRY(strat_setup(fm, nmat, Ep, E, false, full_pass, S));
     NSLG_TRY(strat_chunks(fm, S, pinv));
     NSLG_TRY(strat_stacks(fm, S));
     const int n = S.n, J = S.J;
@@ -829,12 +887,15 @@ int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntr
     NSLG_CUDA(cudaGetLastError());
     std::vector<double2> ls((size_t)2 * nmat), tm((size_t)nmat * LT_BLOCKS);
     std::vector<int> sw((size_t)2 * nmat);
-    int sing = 0;
+    int sing = 0, flags = 0;
+    NSLG_CUDA(cudaMemcpyAsync(&flags, S.flags, sizeof(int), cudaMemcpyDeviceToHost, st));
     NSLG_CUDA(cudaMemcpyAsync(ls.data(), lx.logsum, ls.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
     NSLG_CUDA(cudaMemcpyAsync(sw.data(), lx.swaps, sw.size() * sizeof(int), cudaMemcpyDeviceToHost, st));
     NSLG_CUDA(cudaMemcpyAsync(&sing, lx.singular, sizeof(int), cudaMemcpyDeviceToHost, st));
     NSLG_CUDA(cudaMemcpyAsync(tm.data(), terms, tm.size() * sizeof(double2), cudaMemcpyDeviceToHost, st));
     NSLG_CUDA(cudaStreamSynchronize(st));
+    if (flags & ST_INEXACT)  // the second QR pass to first order was not exact enough (a full pass never sets it)
+        return logdet_strat(fm, nmat, Ep, E, sgn, ph, pinv, out, true);
     for (int g = 0; g < nmat; ++g) {
         if (sing) {
             out[g] = make_double2(-INFINITY, 0.0);

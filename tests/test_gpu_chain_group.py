@@ -154,3 +154,31 @@ def test_group_argument_checks():
     assert call([a, b], u) == _lib.ERR_ARG
     assert call([a, a], u) == _lib.ERR_ARG
     assert call([a], uz) == _lib.ERR_ARG
+
+
+def test_group_trajectory_that_needs_the_full_second_pass():
+    """A group of which one member's chunks (an installed exp(delta K) of 2.2 times the hopping) are too ill-conditioned for the
+    first-order second QR pass: its captured trajectory is taken back, alone and as a branch of the group's launch, and gives
+    the eager one's bits; the other member's is kept."""
+    from nsl_gb300.hmc import ChainEnsemble
+    from nsl_gb300.lattice import Honeycomb, Ring
+
+    Nt, beta = 16, 8.0
+    ring = Ring(6)
+    w, V = np.linalg.eigh(np.array(ring.hopping_matrix()).real)
+    for s in (1, -1):
+        ring.set_exp_hopping_matrix(s * beta / Nt, (V * np.exp(2.2 * s * beta / Nt * w)) @ V.T + 0j)
+    groups = [{"lattice": ring, "Nt": Nt, "beta": beta, "U": [1.0, 2.0]},
+              {"lattice": Honeycomb((2, 2)), "Nt": Nt, "beta": beta, "U": [1.5]}]
+    ens = ChainEnsemble(groups, 0.5, 3, seed=1, real_force=True)
+    rng = np.random.default_rng(9)
+    qs, ps = [], []
+    for g, Nx in zip(groups, (6, 8)):
+        n = len(g["U"])
+        qs.append(rng.standard_normal((n, Nt, Nx)) * np.sqrt(beta / Nt * np.asarray(g["U"]))[:, None, None] + 0j)
+        ps.append(rng.standard_normal((n, Nt, Nx)) + 0j)
+    runs = [ens.leapfrog(qs, ps) for _ in range(4)]  # eager, captured per group, one graph launch, replay
+    for k in range(1, 4):
+        for g in range(2):
+            assert np.isfinite(runs[k][0][g]).all()
+            assert np.array_equal(runs[k][0][g], runs[0][0][g]) and np.array_equal(runs[k][1][g], runs[0][1][g]), (k, g)

@@ -243,3 +243,46 @@ def test_nan_field_stays_inside_the_matrices(Nx, mode):
         pass
     (ld, g), (ld0, g0) = evaluate(h, phi), evaluate(fresh, phi)
     assert ld == ld0 and np.array_equal(g, g0)
+
+
+@pytest.mark.parametrize("kind,a", [("im", 0.5), ("im", 2.0), ("im", 4.0), ("scale", 45.0), ("scale", -45.0),
+                                    ("installed", 2.0), ("installed", 8.0), ("installed", 16.0)])
+def test_stratified_beyond_the_first_order_second_pass(monkeypatch, kind, a):
+    """Chunk products whose condition the lattice does not bound, one slice each (so that no wrap inside a chunk amplifies
+    anything): Im phi of +-a per site (a condition of exp(2 a) and more), a common Im phi of a (entries of exp(+-a), out of
+    FP32's range after the correction), and an installed exp(delta K) of a times the hopping (a condition of exp(a)). Gradient and
+    log det of both species against the dense inverse of M, within the bar of test_stratified_panel_edges."""
+    import nsl_gb300 as N
+
+    monkeypatch.setenv("NSLG_STRAT_CHUNK", "1")
+    eps = 256 * 2.0 ** -53
+    Nx, Nt, beta = 24, 12, 3.0
+    lat = N.Ring(Nx)
+    rng = np.random.default_rng(31)
+    phi = rng.standard_normal((Nt, Nx)) * np.sqrt(beta / Nt) + 0j
+    if kind == "im":
+        phi = phi + 1j * a * rng.choice((-1.0, 1.0), (Nt, Nx))
+    elif kind == "scale":
+        phi = phi + 1j * a * np.where(np.arange(Nt) % 2 == 0, 1.0, -1.0)[:, None]
+    else:
+        w, V = np.linalg.eigh(np.array(lat.hopping_matrix()).real)
+        for s in (1, -1):
+            lat.set_exp_hopping_matrix(s * beta / Nt, (V * np.exp(a * s * beta / Nt * w)) @ V.T + 0j)
+    for species in (0, 1):
+        h = N.HubbardExp(lat, Nt, beta, 0.0, N.Species(species))
+        h.set_stabilisation("stratified")
+        h.populate(phi)
+        ho = O.HubbardExp(lat.hopping_matrix(), Nt, beta, 0.0, species)
+        for s in (1, -1):
+            ho.set_expK(s * beta / Nt, h.exp_hopping_matrix(s * beta / Nt))
+        ho.populate(phi)
+        n = Nt * Nx
+        Md = ho.M_dense().reshape(n, n)
+        inv = np.linalg.inv(Md)
+        nM, nI = np.linalg.norm(Md, 2), np.linalg.norm(inv, 2)
+        want = 1j * np.diag(inv).reshape(Nt, Nx)
+        err = np.abs(np.asarray(h.gradLogDetM()) - want).max()
+        assert err <= max(1e-13 * np.abs(want).max(), eps * nI ** 2 * nM), (species, err)
+        s, l = np.linalg.slogdet(Md)  # (tr K = 0: an installed exp(delta K) has determinant 1 too)
+        ref = complex(l, np.angle(s))
+        assert abs(mod2pi(h.logDetM() - ref)) <= max(1e-13 * abs(ref), n * eps * nI * nM)
