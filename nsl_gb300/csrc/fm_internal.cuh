@@ -240,6 +240,8 @@ int fm_apply_ddtc(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *xh, c
 bool use_stratified(const nslg_fm *fm);
 // Bits of the workspace word "st_flags" (cleared by an evaluation, or before the replay of a captured trajectory):
 constexpr int ST_INEXACT = 1;  // the second QR pass to first order is not exact enough for this field
+constexpr int ST_BREAKDOWN = 2;  // a pivot of a chunk's Gram matrix is not positive: the result means nothing
+int strat_breakdown(int flags);  // the error for ST_BREAKDOWN
 // log of the bound exp(2 k |delta| rho + k spread) on a chunk's condition; spread: max - min of Im phi over a slice's sites
 double strat_log_condition(const nslg_fm *fm, double spread);
 bool use_stratified_grad(const nslg_fm *fm);

@@ -596,6 +596,7 @@ int leapfrog_dev(nslg_fm *fm, double2 *q, double2 *p, double2 Ut, double traj, i
             NSLG_TRY(retake_restore(fm, q, p, nconf, R));
             return leapfrog_steps(fm, q, p, Ut, uin_cfg, traj, nmd, backward, real_force, terms, nconf);
         }
+        NSLG_TRY(strat_breakdown(flags));
         NSLG_REQUIRE(!h, NSLG_ERR_ARG, "gradLogDetM: 1 + A^{-1} is singular");
     }
     return NSLG_OK;
@@ -666,7 +667,10 @@ int leapfrog_group_dev(int ng, nslg_fm *const *fms, const int64_t *nconf, double
     }
     NSLG_CUDA(cudaStreamSynchronize(st));
     for (int g = 0; g < ng; ++g) {
-        if (!(flags[g] & ST_INEXACT)) continue;
+        if (!(flags[g] & ST_INEXACT)) {
+            NSLG_TRY(strat_breakdown(flags[g]));
+            continue;
+        }
         h[g] = 0;
         NSLG_TRY(retake_restore(fms[g], q[g], p[g], nconf[g], R[g]));
         NSLG_TRY(leapfrog_steps(fms[g], q[g], p[g], Ut[g], uin_cfg[g], traj, nmd, backward, real_force, terms, nconf[g]));

@@ -110,7 +110,7 @@ constexpr int CQ_NB = 16;
 
 __global__ void __launch_bounds__(CQ_NB *CQ_NB) k_cholqr_panel(const double2 *__restrict__ G, double2 *__restrict__ R,
                                                                double2 *__restrict__ Z, int n, int k0, int nb,
-                                                               int ngb, bool refine, int *singular) {
+                                                               int ngb, bool refine, int *flags) {
     constexpr int NB = CQ_NB;
     __shared__ double2 D[NB][NB + 1], L[NB][NB + 1], T[NB][NB + 1];
     __shared__ double rd[NB], sd[NB], dd[NB];  // 1 / d, 1 / sqrt(d), d
@@ -167,7 +167,8 @@ __global__ void __launch_bounds__(CQ_NB *CQ_NB) k_cholqr_panel(const double2 *__
             R[(int64_t)(k0 + i) * n + k0 + j] =
                 j == i ? make_double2(sqrt(fmax(dd[i], 0.0)), 0.0) : make_double2(D[i][j].x * s, D[i][j].y * s);
         }
-        if (threadIdx.x < nb && dd[threadIdx.x] == 0.0) *singular = 1;
+        // (a NaN passes: it shows in the result)
+        if (threadIdx.x < nb && dd[threadIdx.x] <= 0.0) atomicOr(flags, ST_BREAKDOWN);
     }
     // gpart: y = L^{-1} t per column (T[q][column]), R_{k0 + i, o0 + j} = y_i / sqrt(d_i).
     // else: y = L^{-1} conj t per row (T[row][q]), Q_{o0 + i, k0 + j} = conj(y_j) / sqrt(d_j).
@@ -582,8 +583,6 @@ int cholqr_pass(nslg_fm *fm, Strat &S, double2 *R, int cnt) {
     cudaStream_t st = fm->ctx->stream;
     const int n = S.n;
     const int64_t nn = (int64_t)n * n;
-    int *singular;
-    NSLG_TRY(ws_get(fm, "lu_singular", 1, &singular));
     ZProd gram(n, n, n, S.Z, n, nn, S.Z, n, nn, S.Gm, n, nn);
     gram.a_adjoint = true;
     gram.upper = true;
@@ -593,7 +592,7 @@ int cholqr_pass(nslg_fm *fm, Strat &S, double2 *R, int cnt) {
         const int nb = std::min(CQ_NB, n - k0), rest = n - k0 - nb;
         const int ngb = (int)ceil_div(rest, CQ_NB), nzb = (int)ceil_div(n, CQ_NB);
         k_cholqr_panel<<<dim3((unsigned)(ngb + nzb), (unsigned)cnt), CQ_NB * CQ_NB, 0, st>>>(S.Gm, R, S.Z, n, k0, nb, ngb,
-                                                                                          !S.first_order, singular);
+                                                                                          !S.first_order, S.flags);
         note_launch(st);
         if (rest == 0) break;
         const double2 *Rk = R + (int64_t)k0 * n + k0 + nb;
@@ -726,6 +725,13 @@ bool use_stratified(const nslg_fm *fm) {
     return beta_rho > 14.0;
 }
 
+int strat_breakdown(int flags) {
+    NSLG_REQUIRE(!(flags & ST_BREAKDOWN), NSLG_ERR_ARG,
+                 "stratified log det / gradient: a chunk of time slices is too ill-conditioned to be factored (condition beyond "
+                 "~1e8)");
+    return NSLG_OK;
+}
+
 double strat_log_condition(const nslg_fm *fm, double spread) {
     const int64_t J = ceil_div(fm->Nt, chunk_len(fm));
     return (double)ceil_div(fm->Nt, J) * (2.0 * std::hypot(fm->delta.x, fm->delta.y) * fm->hops_norm1 + spread);
@@ -844,6 +850,7 @@ int grad_logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const Ex
         NSLG_CUDA(cudaStreamSynchronize(st));
         if (!(h[1] & ST_INEXACT)) break;
     }
+    NSLG_TRY(strat_breakdown(h[1]));
     NSLG_REQUIRE(!h[0], NSLG_ERR_ARG, "gradLogDetM: 1 + A^{-1} is singular");
     return NSLG_OK;
 }
@@ -896,6 +903,7 @@ int logdet_strat(nslg_fm *fm, int nmat, const ExpEntry *const *Ep, const ExpEntr
     NSLG_CUDA(cudaStreamSynchronize(st));
     if (flags & ST_INEXACT)  // the second QR pass to first order was not exact enough (a full pass never sets it)
         return logdet_strat(fm, nmat, Ep, E, sgn, ph, pinv, out, true);
+    NSLG_TRY(strat_breakdown(flags));
     for (int g = 0; g < nmat; ++g) {
         if (sing) {
             out[g] = make_double2(-INFINITY, 0.0);

@@ -286,3 +286,41 @@ def test_stratified_beyond_the_first_order_second_pass(monkeypatch, kind, a):
         s, l = np.linalg.slogdet(Md)  # (tr K = 0: an installed exp(delta K) has determinant 1 too)
         ref = complex(l, np.angle(s))
         assert abs(mod2pi(h.logDetM() - ref)) <= max(1e-13 * abs(ref), n * eps * nI * nM)
+
+
+@pytest.mark.parametrize("chunk,a", [("1", 30.0), ("2", 20.0)])
+def test_stratified_breakdown_is_an_error(monkeypatch, chunk, a):
+    """Chunk products of condition exp(a k) > 1e8 leave their Gram matrix without a Cholesky factor: log det, gradient and a
+    trajectory (eager and captured) report that instead of returning NaN, and the handle goes on with another matrix."""
+    import nsl_gb300 as N
+    from nsl_gb300.action import HubbardFermionAction, HubbardGaugeAction
+    from nsl_gb300.integrator import Leapfrog
+
+    monkeypatch.setenv("NSLG_STRAT_CHUNK", chunk)
+    Nx, Nt, beta = 24, 12, 3.0
+    lat = N.Ring(Nx)
+    w, V = np.linalg.eigh(np.array(lat.hopping_matrix()).real)
+    good = {s * beta / Nt: (V * np.exp(s * beta / Nt * w)) @ V.T + 0j for s in (1, -1)}
+    bad = {s * beta / Nt: (V * np.exp(a * s * beta / Nt * w)) @ V.T + 0j for s in (1, -1)}
+    phi = _field(Nx, Nt, beta, 4)
+    params = {"Nt": Nt, "beta": beta, "U": 1.0}
+    S = HubbardGaugeAction(params) + HubbardFermionAction(lat, params, stabilisation="stratified")
+    h = S._mask_and_fm()[1]
+    lf = Leapfrog(S, 0.2, 2)
+    run = lambda: lf({"phi": phi}, {"phi": 0.1 * phi})
+    for d, E in good.items():
+        h.set_exp_hopping_matrix(d, E)
+    h.populate(phi, N.Species.Particle)
+    ld, g = h.logDetM(), np.asarray(h.gradLogDetM())
+    q = [np.asarray(run()[0]["phi"]) for _ in range(3)]
+    for d, E in bad.items():
+        h.set_exp_hopping_matrix(d, E)
+    h.populate(phi, N.Species.Particle)
+    for f in (h.logDetM, h.gradLogDetM, lambda: S.eval(phi), lambda: S.force(phi), run, run, run):
+        with pytest.raises(RuntimeError, match="ill-conditioned"):
+            f()
+    for d, E in good.items():
+        h.set_exp_hopping_matrix(d, E)
+    h.populate(phi, N.Species.Particle)
+    assert h.logDetM() == ld and np.array_equal(np.asarray(h.gradLogDetM()), g)
+    assert all(np.array_equal(np.asarray(run()[0]["phi"]), v) for v in q)
