@@ -143,8 +143,9 @@ NSLG_API int nslg_fm_populate(nslg_fm *fm, const nslg_c128 *phi, int species);
 NSLG_API int nslg_fm_get_phases(nslg_fm *fm, nslg_c128 *out);
 /* Replaces HubbardExp::M / Mdagger / MMdagger / MdaggerM (hubbardExp.tpp:39-125). psi and out are
  * (nbatch, Nt, Nx) and must not overlap. With device buffers the call is asynchronous on the context's stream; a
- * timeout inside a tensor-core kernel (NSLG_PREC_TF32X3, NSLG_PREC_BF16_SPLIT) is then reported as NSLG_ERR_CUDA by
- * the next call on this handle that synchronises (host buffers, nslg_cg_solve). */
+ * timeout inside a tensor-core kernel (NSLG_PREC_TF32X3, NSLG_PREC_BF16_SPLIT, nslg_fm_apply_dd) is then reported as
+ * NSLG_ERR_CUDA by the next call on this handle that synchronises (host buffers; a solve with one of these precisions or
+ * under NSLG_STOP_TRUE_RESIDUAL_DD). */
 NSLG_API int nslg_fm_apply(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch,
                            int precision);
 

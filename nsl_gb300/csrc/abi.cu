@@ -843,6 +843,12 @@ NSLG_API int nslg_accept_batch(nslg_fm *fm, int64_t nconf, const int32_t *accept
 namespace {
 int cg_solve_abi(nslg_fm *fm, int op, const nslg_c128 *b, const nslg_c128 *x0, nslg_c128 *x, nslg_c128 *x_lo,
                  int64_t nbatch, double eps, int64_t max_iter, int mode, int precision, int stop, nslg_cg_stats *stats);
+
+// Whether a solve may run a tensor-core kernel, whose error word is then read: its operator's, or under the double-double rule
+// that of the residuals, whatever the operator's precision.
+bool uses_tensor_cores(int precision, int stop) {
+    return precision >= NSLG_PREC_TF32X3 || stop == NSLG_STOP_TRUE_RESIDUAL_DD;
+}
 }
 
 NSLG_API int nslg_cg_solve(nslg_fm *fm, int op, const nslg_c128 *b, const nslg_c128 *x0, nslg_c128 *x,
@@ -906,7 +912,7 @@ int cg_solve_abi(nslg_fm *fm, int op, const nslg_c128 *b, const nslg_c128 *x0, n
     if (dlo && dlo != reinterpret_cast<double2 *>(x_lo))
         NSLG_CUDA(cudaMemcpyAsync(x_lo, dlo, bytes, cudaMemcpyDefault, st));
     NSLG_CUDA(cudaStreamSynchronize(st));
-    if (precision >= NSLG_PREC_TF32X3) NSLG_TRY(check_tc_error(fm));
+    if (uses_tensor_cores(precision, stop)) NSLG_TRY(check_tc_error(fm));
     return rc;
 }
 }  // namespace
@@ -949,7 +955,7 @@ NSLG_API int nslg_cg_solve_group(int nfm, nslg_fm *const *fms, int op, const nsl
                                   reinterpret_cast<double2 *const *>(x_lo), nbatch, eps, max_iter, precision, stop,
                                   sp.data());
     if (rc != NSLG_OK && rc != NSLG_NOT_CONVERGED) return rc;
-    if (precision >= NSLG_PREC_TF32X3)
+    if (uses_tensor_cores(precision, stop))
         for (int i = 0; i < nfm; ++i) NSLG_TRY(check_tc_error(fms[i]));
     return rc;
 }

@@ -182,3 +182,33 @@ def test_apply_dd_reports_non_finite_rows():
     want = np.zeros((R, Nt), dtype=bool)
     want[2, 5] = want[2, 6] = want[9, 15] = want[9, 0] = True
     assert np.array_equal(bad, want)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("group", [False, True])
+def test_certified_solve_reports_a_tensor_core_error(precision, group):
+    """Residuals under the double-double rule run on the tensor cores whatever the operator's precision, so such a solve reads
+    their error word. Here it is set by an earlier asynchronous call (an exp(delta K) the split-BF16 operator refuses)."""
+    import nsl_gb300 as N
+    import torch
+
+    Nx, Nt = 320, 16
+    lat = N.Ring(Nx)
+    E = np.eye(Nx) + np.random.default_rng(3).uniform(-1, 1, (Nx, Nx)) / Nx  # beyond the digit-sum bound, well conditioned
+    lat.set_exp_hopping_matrix(0.125, E + 0j)
+    fm = N.HubbardExp(lat, Nt, 0.125 * Nt)
+    fm.populate(np.zeros((Nt, Nx)) + 0j)
+    b = torch.zeros((1, Nt, Nx), dtype=torch.complex128, device="cuda")
+    b[0, 0, 0] = 1.0
+
+    def solve():
+        if group:
+            return N.cg_group([(fm, b)], eps=1e-10, maxIter=5000, precision=precision, stop="true_residual_dd")
+        return N.CG(fm, N.MatrixCombination.MMdagger, 1e-10, 5000, mode="per_rhs", precision=precision,
+                    stop="true_residual_dd")(b)
+
+    solve()
+    fm.M(b, precision="bf16split")  # asynchronous: nothing is reported yet
+    with pytest.raises(RuntimeError, match="delocalised"):
+        solve()
+    solve()  # the report cleared it
