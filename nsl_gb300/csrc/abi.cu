@@ -6,6 +6,7 @@
 #include <type_traits>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -454,8 +455,13 @@ NSLG_API int nslg_fm_get_phases(nslg_fm *fm, nslg_c128 *out) {
     return NSLG_OK;
 }
 
-NSLG_API int nslg_fm_apply(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch,
-                           int precision) {
+namespace {
+
+// nslg_fm_apply, with `other` between the work queued on that stream so far and later. Everything that can be refused is
+// refused first. A handle's two events serve calls from any thread: a wait takes the event's state of that moment, so record
+// and wait are one step under the handle's lock.
+int apply_abi(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch, int precision, bool ordered,
+              cudaStream_t other) {
     NSLG_TRY(check_fm(fm));
     NSLG_REQUIRE(psi && out, NSLG_ERR_ARG, "nslg_fm_apply: null buffer");
     NSLG_REQUIRE(op >= NSLG_OP_M && op <= NSLG_OP_MDAGGERM, NSLG_ERR_ARG, "nslg_fm_apply: unknown operator");
@@ -467,44 +473,62 @@ NSLG_API int nslg_fm_apply(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 
     const size_t bytes = n * sizeof(double2);
     NSLG_REQUIRE(!overlaps(psi, bytes, out, bytes), NSLG_ERR_ARG, "nslg_fm_apply: psi and out overlap");
     if (n == 0) return NSLG_OK;
-    cudaStream_t st = fm->ctx->stream;
-    NSLG_TRY(prepare_apply(fm, op, nbatch, precision));
-    const void *din;
-    NSLG_TRY(stage_in(fm, "io_in", psi, bytes, &din));
     bool out_dev, in_dev;
-    NSLG_TRY(device_ptr(fm, out, &out_dev));
     NSLG_TRY(device_ptr(fm, psi, &in_dev));
-    double2 *dout;
-    if (out_dev) dout = reinterpret_cast<double2 *>(out);
-    else NSLG_TRY(ws_get(fm, "io_out", n, &dout));
-    const double2 *pin = static_cast<const double2 *>(din);
-    if (precision == NSLG_PREC_FP64) NSLG_TRY(fm_apply_dev<double>(fm, op, pin, dout, nbatch));
-    else if (precision == NSLG_PREC_FP32) NSLG_TRY(fm_apply_dev<float>(fm, op, pin, dout, nbatch));
-    else if (precision == NSLG_PREC_TF32X3) NSLG_TRY(fm_apply_dev<TF32x3>(fm, op, pin, dout, nbatch));
-    else NSLG_TRY(fm_apply_dev<BF16Split>(fm, op, pin, dout, nbatch));
-    if (!out_dev) NSLG_CUDA(cudaMemcpyAsync(out, dout, bytes, cudaMemcpyDeviceToHost, st));
-    if (!out_dev || !in_dev) {
-        NSLG_CUDA(cudaStreamSynchronize(st));
-        NSLG_TRY(check_tc_error(fm));
+    NSLG_TRY(device_ptr(fm, out, &out_dev));
+    cudaStream_t st = fm->ctx->stream;
+    ordered = ordered && other != st;
+    if (ordered) {
+        std::lock_guard<std::mutex> lock(fm->order_mu);
+        if (!fm->ev_in) NSLG_CUDA(cudaEventCreateWithFlags(&fm->ev_in, cudaEventDisableTiming));
+        if (!fm->ev_out) NSLG_CUDA(cudaEventCreateWithFlags(&fm->ev_out, cudaEventDisableTiming));
+        NSLG_CUDA(cudaEventRecord(fm->ev_in, other));
+        NSLG_CUDA(cudaStreamWaitEvent(st, fm->ev_in, 0));
     }
-    // device-buffer calls stay asynchronous: a tensor-core pipeline timeout is reported by the next call on this
-    // handle that synchronises
-    return NSLG_OK;
+    auto queue = [&]() -> int {
+        NSLG_TRY(prepare_apply(fm, op, nbatch, precision));
+        const double2 *pin = reinterpret_cast<const double2 *>(psi);
+        if (!in_dev) {
+            double2 *w;
+            NSLG_TRY(ws_get(fm, "io_in", n, &w));
+            NSLG_CUDA(cudaMemcpyAsync(w, psi, bytes, cudaMemcpyHostToDevice, st));
+            pin = w;
+        }
+        double2 *dout;
+        if (out_dev) dout = reinterpret_cast<double2 *>(out);
+        else NSLG_TRY(ws_get(fm, "io_out", n, &dout));
+        if (precision == NSLG_PREC_FP64) NSLG_TRY(fm_apply_dev<double>(fm, op, pin, dout, nbatch));
+        else if (precision == NSLG_PREC_FP32) NSLG_TRY(fm_apply_dev<float>(fm, op, pin, dout, nbatch));
+        else if (precision == NSLG_PREC_TF32X3) NSLG_TRY(fm_apply_dev<TF32x3>(fm, op, pin, dout, nbatch));
+        else NSLG_TRY(fm_apply_dev<BF16Split>(fm, op, pin, dout, nbatch));
+        if (!out_dev) NSLG_CUDA(cudaMemcpyAsync(out, dout, bytes, cudaMemcpyDeviceToHost, st));
+        if (!out_dev || !in_dev) {
+            NSLG_CUDA(cudaStreamSynchronize(st));
+            NSLG_TRY(check_tc_error(fm));
+        }
+        // device-buffer calls stay asynchronous: a tensor-core pipeline timeout is reported by the next call on this
+        // handle that synchronises
+        return NSLG_OK;
+    };
+    const int rc = queue();
+    if (ordered) {  // also after an error: work may have been queued
+        std::lock_guard<std::mutex> lock(fm->order_mu);
+        NSLG_CUDA(cudaEventRecord(fm->ev_out, st));
+        NSLG_CUDA(cudaStreamWaitEvent(other, fm->ev_out, 0));
+    }
+    return rc;
+}
+
+}  // namespace
+
+NSLG_API int nslg_fm_apply(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch,
+                           int precision) {
+    return apply_abi(fm, op, psi, out, nbatch, precision, false, nullptr);
 }
 
 NSLG_API int nslg_fm_apply_on(nslg_fm *fm, int op, const nslg_c128 *psi, nslg_c128 *out, int64_t nbatch,
                               int precision, void *stream) {
-    NSLG_TRY(check_fm(fm));
-    cudaStream_t other = static_cast<cudaStream_t>(stream), st = fm->ctx->stream;
-    if (other == st) return nslg_fm_apply(fm, op, psi, out, nbatch, precision);
-    if (!fm->ev_in) NSLG_CUDA(cudaEventCreateWithFlags(&fm->ev_in, cudaEventDisableTiming));
-    if (!fm->ev_out) NSLG_CUDA(cudaEventCreateWithFlags(&fm->ev_out, cudaEventDisableTiming));
-    NSLG_CUDA(cudaEventRecord(fm->ev_in, other));
-    NSLG_CUDA(cudaStreamWaitEvent(st, fm->ev_in, 0));
-    const int rc = nslg_fm_apply(fm, op, psi, out, nbatch, precision);
-    NSLG_CUDA(cudaEventRecord(fm->ev_out, st));  // also after an error: work may have been queued
-    NSLG_CUDA(cudaStreamWaitEvent(other, fm->ev_out, 0));
-    return rc;
+    return apply_abi(fm, op, psi, out, nbatch, precision, true, static_cast<cudaStream_t>(stream));
 }
 
 NSLG_API int nslg_fm_apply_dd(nslg_fm *fm, int op, const nslg_c128 *psi_hi, const nslg_c128 *psi_lo,

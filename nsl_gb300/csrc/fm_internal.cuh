@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <map>
+#include <mutex>
 #include <string>
 #include <tuple>
 #include <utility>
@@ -108,6 +109,7 @@ struct nslg_fm {
     cudaStream_t side = nullptr;
     cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaEvent_t ev_in = nullptr, ev_out = nullptr;  // orders ctx->stream after and before a caller's stream
+    std::mutex order_mu;                            // one record and its wait at a time
     std::map<std::string, nslg::DevBuf> ws;
     uint64_t ws_generation = 0;  // bumped whenever a workspace buffer moves (invalidates captured graphs)
     std::map<std::string, cudaGraphExec_t> graphs;

@@ -314,3 +314,43 @@ def test_replacing_exp_hopping_replaces_what_was_derived_from_it():
     x, lo = got[10], got[11]
     ho = _same_operator(fm, phi)
     assert max(np.linalg.norm(O.residual_dd(ho, "MMdagger", b[r], x[r], lo[r])) for r in range(R)) <= 1.01 * eps
+
+
+def test_operator_calls_from_several_threads_and_streams():
+    """One handle, three threads, each with its own stream: an application reads its operand after the work queued on its caller's
+    stream (here a copy behind a delay), and that stream's later work reads the result, whichever calls come between."""
+    import threading
+
+    import nsl_gb300 as N
+    import torch
+
+    fm = N.HubbardExp(N.Honeycomb((3, 3)), 16, 4.0)
+    rng = np.random.default_rng(0)
+    fm.populate(rng.standard_normal((16, 18)) + 0j)
+    src = [torch.from_numpy(rng.standard_normal((40, 2, 16, 18)) + 1j * rng.standard_normal((40, 2, 16, 18))).cuda()
+           for _ in range(3)]
+    want = [torch.stack([fm.M(v) for v in s]).cpu() for s in src]
+    got, errors = [None] * 3, []
+
+    def work(k):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                out = torch.zeros_like(src[k])
+                psi = torch.zeros_like(src[k][0])
+                for i in range(len(src[k])):
+                    torch.cuda._sleep(20000)
+                    psi.copy_(src[k][i])
+                    out[i].copy_(fm.M(psi))
+                torch.cuda.current_stream().synchronize()
+                got[k] = out.cpu()
+        except Exception as e:  # pragma: no cover
+            errors.append(e)
+
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    assert all(torch.equal(g, w) for g, w in zip(got, want))
