@@ -240,6 +240,7 @@ int fm_apply_ddtc(nslg_fm *fm, int mode, const ExpEntry *e, const double2 *xh, c
 // matrices with factors Ep[g] = exp(-sgn_g delta K), E[g] = exp(sgn_g delta K) and phase rows ph / pinv
 // (nmat, Nt, Nx).
 bool use_stratified(const nslg_fm *fm);
+bool strat_pair_fits(const nslg_fm *fm);  // whether the log dets of both species may be one batch
 // Bits of the workspace word "st_flags" (cleared by an evaluation, or before the replay of a captured trajectory):
 constexpr int ST_INEXACT = 1;  // the second QR pass to first order is not exact enough for this field
 constexpr int ST_BREAKDOWN = 2;  // a pivot of a chunk's Gram matrix is not positive: the result means nothing

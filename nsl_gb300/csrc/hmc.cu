@@ -302,8 +302,9 @@ int hubbard_eval_batch_dev(nslg_fm *fm, const double2 *phi, int64_t nconf, doubl
                            const double2 *Ut_cfg);
 
 int hubbard_eval_dev(nslg_fm *fm, const double2 *phi, double2 Ut, int terms, double2 *S) {
-    // the stratified log dets of both species as one batch (their launches are the same, and each fills half the GPU)
-    if ((terms & 2) && use_stratified(fm)) {
+    // the stratified log dets of both species as one batch (their launches are the same, and each fills half the GPU), where
+    // two fit; else one after the other
+    if ((terms & 2) && use_stratified(fm) && strat_pair_fits(fm)) {
         NSLG_TRY(hubbard_eval_batch_dev(fm, phi, 1, Ut, terms, S, nullptr));
         return populate_dev(fm, phi, NSLG_HOLE);
     }

@@ -725,6 +725,13 @@ bool use_stratified(const nslg_fm *fm) {
     return beta_rho > 14.0;
 }
 
+// A batch's products are one launch of at most 65535, and a pair needs twice the stacks and chunk products of one matrix (four
+// n x n matrices per chunk): beyond a quarter of the memory the species are evaluated in turn, each filling the GPU.
+bool strat_pair_fits(const nslg_fm *fm) {
+    const int64_t J = ceil_div(fm->Nt, chunk_len(fm));
+    return 2 * J <= 65535 && (double)(2 * 4 * (J + 1) * fm->Nx * fm->Nx) * sizeof(double2) <= 64.0 * (1ull << 30);
+}
+
 int strat_breakdown(int flags) {
     NSLG_REQUIRE(!(flags & ST_BREAKDOWN), NSLG_ERR_ARG,
                  "stratified log det / gradient: a chunk of time slices is too ill-conditioned to be factored (condition beyond "

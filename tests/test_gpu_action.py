@@ -364,3 +364,25 @@ def test_inverse_on_clusters_has_the_single_ctas_bits(Nx):
     for b in (0, 17, 39):
         qb, pb = Leapfrog(S, 0.1, 2)({"phi": phi[b]}, {"phi": p[b]})
         assert np.array_equal(q1["phi"][b], qb["phi"]) and np.array_equal(p1["phi"][b], pb["phi"])
+
+
+def test_action_where_a_pair_of_species_is_more_than_a_launch_takes(monkeypatch):
+    """The action of one configuration evaluates both species' stratified log dets as one batch while its chunks fit a launch
+    (65535 products); 32768 chunks of two slices per species do not, and are evaluated in turn. Against the log dets of the
+    handle."""
+    import nsl_gb300 as N
+    from nsl_gb300.action import HubbardFermionAction
+
+    monkeypatch.setenv("NSLG_STRAT_CHUNK", "2")
+    Nt, beta = 65536, 20.0
+    lat = N.Ring(2)
+    params = {"Nt": Nt, "beta": beta, "U": 1.0}
+    phi = np.random.default_rng(6).standard_normal((Nt, 2)) * np.sqrt(beta / Nt) + 0j
+    got = HubbardFermionAction(lat, params, stabilisation="stratified").eval(phi)
+    h = N.HubbardExp(lat, Nt, beta)
+    h.set_stabilisation("stratified")
+    want = 0
+    for species in (N.Species.Particle, N.Species.Hole):
+        h.populate(phi, species)
+        want -= h.logDetM()
+    assert got == want
