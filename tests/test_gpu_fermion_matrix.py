@@ -354,3 +354,42 @@ def test_operator_calls_from_several_threads_and_streams():
         t.join()
     assert not errors, errors
     assert all(torch.equal(g, w) for g, w in zip(got, want))
+
+
+@pytest.mark.parametrize("Nx,Nt,R", [(18, 16, 5), (72, 7, 9), (97, 5, 13), (288, 3, 11)])
+def test_tf32_operator_row_sizes_and_non_finite_values(Nx, Nt, R):
+    """The 3xTF32 operator on rows of sizes 2^-60 to 2^90, rows of zeros, values outside FP32's range, infinities and NaN. Scaling
+    a row by a power of two scales its result exactly (the splits work on bit patterns); ordinary rows agree with FP64 to
+    8 Nx 2^-21 of the sum of moduli. Where a row holds a value FP32 cannot (or an infinity, or a NaN), what it reaches is not
+    finite, and nothing else changes."""
+    import nsl_gb300 as N
+
+    rng = np.random.default_rng(Nx)
+    fm = N.HubbardExp(N.Ring(Nx), Nt, 0.1 * Nt)
+    fm.populate(rng.standard_normal((Nt, Nx)) + 0j)
+    E = np.abs(fm.exp_hopping_matrix(0.1))
+    base = rng.standard_normal((R, Nt, Nx)) + 1j * rng.standard_normal((R, Nt, Nx))
+    base[0] = 0.0
+    base[1, Nt // 2] = 0.0
+    # (r, t) reaches (r, t +- 1) and itself: one scale per right-hand side
+    scale = 2.0 ** rng.integers(-60, 91, (R, 1, 1))
+    psi, clean = base * scale, {}
+    for op, shift in (("M", 1), ("Mdagger", -1)):
+        one = getattr(fm, op)(base, precision="tf32x3")
+        terms = np.roll(np.abs(base) @ E.T, shift, 1)
+        assert (np.abs(one - getattr(fm, op)(base)) <= 8 * Nx * 2.0 ** -21 * terms).all(), op
+        clean[op] = getattr(fm, op)(psi, precision="tf32x3")
+        assert np.array_equal(clean[op], one * scale), op
+    for bad in (1e40, np.inf, -np.inf, np.nan):
+        for part in (1.0, 1j):
+            x = psi.copy()
+            t, r = Nt - 1, R - 1
+            x[r, t, Nx // 2] = bad * part if np.isfinite(bad) or part == 1.0 else complex(0.0, bad)
+            for op, to in (("M", (t + 1) % Nt), ("Mdagger", t - 1)):
+                got = getattr(fm, op)(x, precision="tf32x3")
+                same = np.ones((R, Nt), bool)
+                same[r, to] = same[r, t] = False
+                assert np.array_equal(got[same], clean[op][same]), (bad, part, op)
+                assert not np.isfinite(got[r, to]).any(), (bad, part, op)
+                elsewhere = np.arange(Nx) != Nx // 2  # psi itself enters its own slice at that site alone
+                assert np.array_equal(got[r, t, elsewhere], clean[op][r, t, elsewhere]), (bad, part, op)
