@@ -355,7 +355,8 @@ __global__ void __launch_bounds__(DT_THREADS, 1)
             for (int i = 1; i <= nk; ++i) {
                 if (!(kl[i] >> 30 & 1)) continue;  // one pass per segment
                 const int buf = seg & 1, use = seg >> 1;
-                if (*abort_flag || !tc::mbar_wait(&bar_tfull[buf], use & 1, err, 46)) {
+                // (a vote: a warp leaves whole, or its shuffles and TMEM reads would wait for lanes that have gone)
+                if (!__all_sync(0xffffffffu, *abort_flag == 0 && tc::mbar_wait(&bar_tfull[buf], use & 1, err, 46))) {
                     ok = false;
                     break;
                 }

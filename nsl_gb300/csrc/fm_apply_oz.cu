@@ -342,7 +342,8 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
         int tc_n = 0;
         for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
             if (!live(t)) continue;
-            if (*abort_flag) break;
+            // (votes: a warp leaves whole, or its shuffles and TMEM reads would wait for lanes that have gone)
+            if (__any_sync(0xffffffffu, *abort_flag != 0)) break;
             const int buf = tc_n & 1, use = tc_n >> 1;
             const int mt = t / ntn, nt = t % ntn;
             const int64_t grow = (int64_t)mt * (OZ_BM / 2) + j;
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
                                                                     : make_double2(0.0, 0.0);
             }
             const int escale = (row_ok ? row_exp[(int64_t)mt * OZ_BM + m] : 0) - OZ_ZSHIFT;
-            if (!tc::mbar_wait(&bar_tfull[buf], use & 1, err, 26)) {
+            if (!__all_sync(0xffffffffu, tc::mbar_wait(&bar_tfull[buf], use & 1, err, 26))) {
                 *abort_flag = 1;
                 break;
             }
