@@ -938,7 +938,9 @@ template <typename Top> int run_chunk(CgRun &R) {
 // run on clusters (k_cg_cluster) while RC_CTAS SMs do an iteration's products faster than five launches take: up to
 // RC_WORK = elements x sites, the systems together on the SMs there are. Measured per iteration at Nt = 16: honeycomb
 // 3x3 (5184) 21.4 us in launches, 7.7 us on a cluster; honeycomb 6x6 (82944) 44 and 22 us, ring 128,
-// Nt = 8 (131072) 51 and 25 us; beyond, the cluster loses its lead (two FP64 FMAs per clock and SM) and its shared memory.
+// Nt = 8 (131072) 51 and 25 us. With as many systems as there are clusters (19): 24.9 and 11.5, 62.6 and 31.8, 53.0 and
+// 48.9 us; other shapes (Nt 12 to 128, 8 to 100 sites) 0.4 to 0.8 of the launches' time. Beyond, the cluster loses its lead
+// (two FP64 FMAs per clock and SM) and soon its shared memory (144 sites, Nt = 6, do not fit).
 constexpr int64_t RC_WORK = 131072;
 constexpr size_t RC_MAX_SMEM = 200 * 1024;
 constexpr int64_t RES_MAX_LEN = 2048;

@@ -11,8 +11,7 @@
 // pairs, columns the output sites, the reduction runs over the input sites with the phase multiply in the operand
 // load and the time shift, boundary sign, conj(phase) (M^dagger) and "psi -" in the epilogue. A row mask skips the
 // right-hand sides that do not need a residual (the CG evaluates it only for systems due an update). Vectors of 4096
-// elements and more with a real exp(delta K) take the tensor-core form (fm_apply_ddtc.cu): 0.06 against 0.36 ms already at
-// honeycomb 3x3 with 15 right-hand sides.
+// elements and more with a real exp(delta K) take the tensor-core form (fm_apply_ddtc.cu, with the figures of both).
 
 #include "dd_math.cuh"
 #include "fm_internal.cuh"

@@ -16,7 +16,8 @@
 // double-double.
 //
 // One persistent CTA per SM as in fm_apply_oz.cu: warp 0 streams k-blocks (one bulk copy per operand), warp 1 issues one
-// MMA per operand digit (N = 16 sites x the digits that meet it), four epilogue warps finish 128 x 16 tiles from one of two
+// MMA per operand digit (N = 16 sites x the digits that meet it; as there, MMAs of different N on overlapping accumulators,
+// executed in issue order), four epilogue warps finish 128 x 16 tiles from one of two
 // accumulator sets while the next segment runs in the other.
 // Measured, M on 64 right-hand sides at honeycomb 12x12, Nt = 64: 23.8 ms on the CUDA cores, 0.49 ms here; on 2 at 24x24,
 // Nt = 128: 23.8 and 0.32 ms.
@@ -150,8 +151,8 @@ __global__ void k_ddtc_klist(const int *__restrict__ sums, const int *__restrict
     kl[0] = n;
 }
 
-// One warp per row (r, t) of rows [row0, row0 + rows) (digits, scales, vh and vl are indexed from row0): the operand (phase o x for M, stored to vh, vl; x itself for M^dagger), its scales (real and
-// imaginary parts) and its digits.
+// One warp per row (r, t) of rows [row0, row0 + rows) (digits, scales, vh and vl are indexed from row0): the operand (phase o x
+// for M, stored to vh, vl; x itself for M^dagger), its scales (real and imaginary parts) and its digits.
 template <int MODE>
 __global__ void __launch_bounds__(256) k_ddtc_digits(const double2 *__restrict__ xh, const double2 *__restrict__ xl,
                                                      const double2 *__restrict__ phase, double2 *__restrict__ vh,
@@ -473,6 +474,9 @@ int planes_of(nslg_fm *fm, const ExpEntry *e, DdPlanes **out) {
 
 }  // namespace
 
+// Measured, one M of a few vectors, CUDA cores and tensor cores: 4608 elements on 18 sites 349 and 44 us, 4096 on 64 sites 681
+// and 51 us, 4608 on 72 sites 846 and 54 us. Below the line the tensor cores are ahead too (128 elements on 8 sites 172 and
+// 35 us, 1024 on 64 sites 660 and 47 us): it is where they were first tried, not where the two forms meet.
 bool ddtc_applies(const ExpEntry *e, int Nx, int64_t rows) {
     return e->is_real && Nx <= 2048 && rows * Nx >= 4096;
 }

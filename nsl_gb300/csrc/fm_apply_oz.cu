@@ -124,8 +124,8 @@ __device__ __forceinline__ void operand_pair(const double2 *__restrict__ psi, co
     }
 }
 
-// One warp per complex row (r, t): scales e (max |Y| < 2^e, real and imaginary GEMM rows separately) and the digit
-// planes A[l][2 row + c][y] (ld sites, zero padded). Lanes take site pairs (4-byte BF16 stores).
+// One warp per complex row (r, t): scales e (max |Y| < 2^e, real and imaginary GEMM rows separately) and the digits of GEMM
+// rows 2 row + c at digit_offset<OZ_TILE_A> (ld sites, zero padded). Lanes take site pairs (4-byte BF16 stores).
 // NP: site pairs a lane keeps in registers (rows of <= 64 NP sites); short rows take the small variant, whose registers
 // let twice the warps in (their loads' latency is what bounds it: 20 -> 9 us at 4608 rows of 72 sites).
 template <int MODE, int NP>
@@ -300,8 +300,11 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
                     // after the other in shared memory (32 rows each), and so do their accumulators d = a + b in
                     // TMEM, so they are one B operand of N = 32 x (number of digits) and the operand slice is read
                     // once. The tile's first k-block has every digit, so its a = 0 product (N = 192, accumulate =
-                    // 0) starts all accumulators. Descriptors are the stage's base descriptor plus an offset (the
-                    // address field is bits 0-13, in 16-byte units).
+                    // 0) starts all accumulators. MMAs of different N then add to overlapping, not equal, ranges of
+                    // TMEM columns: the kernel relies on the tensor core executing one thread's MMAs in issue order
+                    // also where their shapes differ (PTX states it for equal accumulator and shape). The sums of orders
+                    // d <= 3 are exact integers, so a lost update would show; no test sees one. Descriptors are
+                    // the stage's base descriptor plus an offset (the address field is bits 0-13, in 16-byte units).
                     const uint64_t dst = dsm0 + (uint64_t)((s * STAGE) >> 4);
                     const int b0 = __ffs(mask) - 1, b1 = 31 - __clz(mask);
                     const uint64_t db = dst + (uint64_t)((OZ_S * OZ_A_SLICE + b0 * OZ_B_SLICE) >> 4);
@@ -469,10 +472,10 @@ __global__ void __launch_bounds__(OZP_THREADS, 1)
     }
 }
 
-// Digit planes of the real part of exp(d K): plane l holds digit l of every row x (scale 2^{e_x} per row), rows of
-// ld BF16 (zero padded), the planes stacked along the row axis (S * Nx rows) for one 2-D tensor map. One block of
-// 256 threads per row x; it also evaluates the row's digit-sum bounds (256 sum_{l<=d} B_l(x), B_l(x) = sum_y |b_l|)
-// and sets col_exp[Nx] (zeroed before the launch) when an order d < OZ_EXACT reaches 2^24 or any order 2^30.
+// Digits of the real part of exp(d K), row x scaled by 2^{e_x}: digit l of (x, y) at digit_offset<OZ_BN> (tiles of 32 rows and
+// 16 sites in stage order, rows padded with zeros to ld sites and whole tiles). One block of 256 threads per row x; it
+// notes the digits present per k-block (klist) and evaluates the row's digit-sum bounds (256 sum_{l<=d} B_l(x),
+// B_l(x) = sum_y |b_l|) and sets col_exp[Nx] (zeroed before the launch) when an order d < OZ_EXACT reaches 2^24 or any order 2^30.
 __global__ void __launch_bounds__(256) k_oz_planes(const double2 *__restrict__ E, char *planes, int *col_exp,
                                                    int *klist, int Nx, int ld) {
     const int x = blockIdx.x, nkb = ld / OZ_BK;
@@ -629,7 +632,7 @@ int oz_planes(nslg_fm *fm, const ExpEntry *e, OzPlanes **out) {
     return NSLG_OK;
 }
 
-// digits: workspace of S * 2 * rows * ld BF16; rexp: 2 * rows ints.
+// Operand digits fill oz_digit_bytes(rows, Nx), whole tiles of 128 GEMM rows; rexp: 2 * rows ints.
 namespace {
 
 template <int MODE>

@@ -2,18 +2,20 @@
 // hubbardExp.tpp:129-211; HubbardDiag::logDetM / gradLogDetM, hubbardDiag.tpp:169-250, with the time-slice matrix
 // 1 - sgn delta K in place of exp(+-sgn delta K), the product taken in increasing t and i sgn sum(phi) added).
 //
-// logDetM: the time-slice matrices B_t = exp(sgn delta K) diag(phiExp[(t+1) % Nt]) (hubbardExp.tpp:142) are built by
-// one kernel, multiplied as a balanced product tree of batched complex GEMMs (log2(Nt) levels instead of Nt
-// sequential products; the product is the same B_{Nt-1} ... B_0), then 1 + prod is LU-factorised with partial
-// pivoting (right-looking, panels of 32 columns: one panel kernel, the row swaps, a triangular solve for the block
-// row of U and one GEMM update of the trailing matrix per panel) and log det = sum log(u_kk) + i pi (#row swaps),
-// folded onto the principal branch like log(det(.))
+// logDetM (one matrix; batches go through logdet_many below): the time-slice matrices
+// B_t = exp(sgn delta K) diag(phiExp[(t+1) % Nt]) (hubbardExp.tpp:142) are built by one kernel, multiplied as a balanced
+// product tree of batched complex GEMMs (log2(Nt) levels instead of Nt sequential products; the product is the same
+// B_{Nt-1} ... B_0), then 1 + prod is LU-factorised with partial pivoting (right-looking, panels of 32 columns: one panel
+// kernel, the row swaps, a triangular solve for the block row of U and one GEMM update of the trailing matrix per panel)
+// and log det = sum log(u_kk) + i pi (#row swaps), folded onto the principal branch like log(det(.))
 // (src/NSL/LinAlg/det.tpp:15-20). Summing logs instead of forming det() avoids the overflow that makes the
 // reference's value NaN at low temperature.
 //
 // gradLogDetM: Fk(t) = diag(phiExpInv[(t-1) % Nt]) exp(-sgn delta K); suffix products S(t) = Fk(t) ... Fk(Nt-1)
-// and prefix products P(t) = (1 + S(0))^{-1} Fk(0) ... Fk(t) (hubbardExp.tpp:165-208) are each evaluated as a
-// sequence of Nt-1 batched GEMM steps; the diagonal of S(t+1) P(t) needs only O(Nx^2) per slice (a row-column dot
+// and prefix products P(t) = (1 + S(0))^{-1} Fk(0) ... Fk(t) (hubbardExp.tpp:165-208). By size: scans of log2(Nt) levels
+// (up to 32 sites and 8 matrices), a whole chain per launch (k_chain, a real exp(delta K) up to 144 sites), else Nt-1
+// batched products. The inverse is a Gauss-Jordan elimination in shared memory (up to 64 sites; on clusters while few
+// matrices leave SMs free) or the blocked LU. The diagonal of S(t+1) P(t) needs only O(Nx^2) per slice (a row-column dot
 // per site) instead of the reference's full GEMM per slice.
 
 #include <cooperative_groups.h>
@@ -852,7 +854,8 @@ int gj_inverse_plus_one(nslg_fm *fm, const double2 *A, int64_t astride, double2 
             done.insert(fm->ctx->device);
         }
     }
-    // clusters from 24 sites on (equal below: the look-ahead bounds a step either way) while two CTAs per SM hold all matrices.
+    // clusters from 24 sites on while two CTAs per SM hold all matrices. One gradient (ring, Nt = 8), one CTA and clusters:
+    // 14 sites 90 and 92 us, 16 97 and 97, 18 108 and 102, 22 118 and 111, 24 122 and 115, 28 136 and 126, 32 160 and 139.
     // Trajectories of 5 forces, one CTA per matrix against clusters: n = 32, 2 matrices 904 and 803 us; n = 50 2.15 and
     // 1.51 ms, 48 matrices 5.33 and 4.90 ms, 76 6.64 and 6.50 ms; n = 64, 2 matrices 3.05 and 1.54 ms, 48 5.94 and 4.94 ms.
     if (n >= GC_MIN && (int64_t)nmat * GC <= 2 * std::max(1, num_sms())) {
@@ -870,7 +873,7 @@ int gj_inverse_plus_one(nslg_fm *fm, const double2 *A, int64_t astride, double2 
         note_launch(fm->ctx->stream);
         return NSLG_OK;
     }
-    k_gj_inverse<<<(unsigned)nmat, n <= 18 ? 384 : GJ_T, gj_smem(n), fm->ctx->stream>>>(A, astride, G, n, singular);
+    k_gj_inverse<<<(unsigned)nmat, GJ_T, gj_smem(n), fm->ctx->stream>>>(A, astride, G, n, singular);
     note_launch(fm->ctx->stream);
     NSLG_CUDA(cudaGetLastError());
     return NSLG_OK;

@@ -734,8 +734,8 @@ bool strat_pair_fits(const nslg_fm *fm) {
 
 int strat_breakdown(int flags) {
     NSLG_REQUIRE(!(flags & ST_BREAKDOWN), NSLG_ERR_ARG,
-                 "stratified log det / gradient: a chunk of time slices is too ill-conditioned to be factored (condition beyond "
-                 "~1e8)");
+                 "stratified log det / gradient: a chunk of time slices is too ill-conditioned to be factored (condition "
+                 "beyond ~1e8)");
     return NSLG_OK;
 }
 
