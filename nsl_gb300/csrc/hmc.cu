@@ -10,9 +10,8 @@
 // total force and applies the momentum kick and the following drift.
 
 #include <cmath>
-#include <cstring>
-
 #include <cstdio>
+#include <cstring>
 #include <string>
 #include <vector>
 
